@@ -10,11 +10,11 @@
 // device-to-host copy of the offsets; here the experts are routed on the device by the tile
 // map, no synchronisation).
 //
-// Both operands are brought to fp16 with their block scale applied (one rounding of 2^-11
-// per operand, as on the GGUF tensor-core path) and multiplied by the fp16 tcgen05 kernel of
-// tc_gemm.cu with fp32 accumulation.  A native kind::f8f6f4 pipeline with the scales applied
-// on a per-128-K accumulator drain would halve the operand traffic; this version is the
-// correct baseline for it.
+// The single problem runs on kind::f8f6f4 with the scales applied on a per-K-block accumulator
+// drain (fp8_mma.cu), up to four rows on a streaming mat-vec.  The grouped problem, and operands
+// off a 16-byte boundary, are brought to fp16 with their block scale applied (one rounding of
+// 2^-11 per operand, as on the GGUF tensor-core path) and multiplied by the fp16 tcgen05 kernel
+// of tc_gemm.cu with fp32 accumulation.
 //
 // weight_fp8_quant replaces launch_weight_fp8_quant (csrc/smxx/quant/weight_fp8_quant.cu:51-138):
 // one scale per 128 x 128 tile (tile amax / 448, 1 for an all-zero tile), values
@@ -288,6 +288,9 @@ extern "C" int lsg_fp8_gemm(const lsg_fp8_gemm_params* p, void* workspace, size_
         return fail(LSG_ERR_ALIGNMENT, "fp8_gemm: workspace must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int M = p->M, N = p->N, K = p->K;
+    if (fp8_mma_usable(p->A, p->B, K))
+        return fp8_mma(p->A, p->B, static_cast<const float*>(p->scale_A), static_cast<const float*>(p->scale_B), p->D,
+                       p->output_dtype, M, N, K, s);
     uint8_t* base = static_cast<uint8_t*>(workspace);
     __half* a16 = reinterpret_cast<__half*>(base);
     __half* b16 = reinterpret_cast<__half*>(base + a256(static_cast<size_t>(M) * K * 2));

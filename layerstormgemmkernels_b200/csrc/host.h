@@ -57,6 +57,11 @@ int tc_gemm_f16(const void* A16, long long a_rows, const void* B16, long long b_
                 const int* tile_mstart, int t_max, const int32_t* expert_offsets, cudaStream_t s,
                 float alpha_host = 1.0f);
 
+// Block-scaled FP8 GEMM on tcgen05.mma.kind::f8f6f4 (fp8_mma.cu).
+bool fp8_mma_usable(const void* A, const void* B, int K);
+int fp8_mma(const void* A, const void* B, const float* sA, const float* sB, void* D, int out_dtype, int M, int N, int K,
+            cudaStream_t s);
+
 // NVFP4 GEMM on tcgen05.mma.kind::mxf4nvf4.block_scale (nvfp4_mma.cu).
 bool nvfp4_mma_usable(const void* A, const void* B, const void* sfa, const void* sfb, int K);
 int nvfp4_mma(const void* A, long long a_rows, const void* B, long long b_rows, const void* sfa, const void* sfb,

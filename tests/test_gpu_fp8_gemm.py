@@ -56,6 +56,29 @@ def test_fp8_gemm_quantizer_pairing(ops, M, N, K):
     assert (full * got).sum() / np.sqrt((full * full).sum() * (got * got).sum()) > 0.99
 
 
+@pytest.mark.parametrize("dt", ["bf16", "fp16"])
+@pytest.mark.parametrize("M,N,K", [
+    (5, 8, 16),          # less than one K block, one 16-byte row piece
+    (127, 100, 144),     # ragged in every direction, rows of the result off 16-byte boundaries
+    (129, 264, 1040),    # one row and one column piece into the next tile
+    (700, 2056, 512),    # several tiles per CTA's column range
+    (2048, 4096, 640),   # 256-column tiles, more than one per CTA
+])
+def test_fp8_gemm_native_edges(ops, M, N, K, dt):
+    """Exact products, fp32 sums: against float64 within half a unit of the 16-bit result plus
+    1e-5 of the largest one (2^-24 a step over the K values, scaled per block)."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a8, sa = ops.dynamic_fp8_quant(torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16), True)
+    b8, sb = ops.weight_fp8_quant((torch.randn(N, K, generator=g, device="cuda") * 0.05).to(torch.bfloat16))
+    x = a8.double() * sa.double().t().repeat_interleave(128, 1)[:, :K]
+    w = b8.double() * sb.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)[:, :K]
+    ref = x @ w.t()
+    out = ops.fp8_gemm(a8, b8, sa, sb, M, N, K, dt)
+    half_unit = 2.0 ** -8 if dt == "bf16" else 2.0 ** -11
+    assert ((out.double() - ref).abs() <= half_unit * ref.abs() + 1e-5 * ref.abs().max()).all()
+    assert torch.equal(out, ops.fp8_gemm(a8, b8, sa, sb, M, N, K, dt))
+
+
 def test_fp8_grouped_gemm_ragged_experts(ops):
     N, K = 256, 512
     offs = [0, 40, 40, 170, 173]
