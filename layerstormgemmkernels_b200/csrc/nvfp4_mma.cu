@@ -31,6 +31,13 @@
 // tokens on the 128-lane side a thread's accumulator row is one output row and stores are
 // contiguous.  Work items are (token tile, weight tile) pairs; token tiles come from a dense
 // problem or from the device-built tile map of the grouped one.  Every wait is time-limited.
+//
+// A dense call with few tokens has fewer output tiles than the chip has SMs (77 x 4096: 16
+// pairs).  Its K range is then split over the CTAs of a cluster (split_plan below): every CTA
+// parks its fp32 accumulators in its own shared memory, which the finished main loop has left
+// free, and after a cluster barrier the CTAs add the partial tiles in rank order, each its share
+// of the elements, reading the peers' through distributed shared memory.  No workspace, no
+// counters, the same bits on every run.
 #include "common.cuh"
 #include "host.h"
 #include "tcgen05.cuh"
@@ -73,7 +80,29 @@ struct F4Args {
     const int32_t* expert_offsets;
     const int32_t* sf_offsets;
     unsigned int* status;
+    int tile_cols;            // 128-column output tiles per work item: 2, or 1
+    int ksplit;               // CTAs of a cluster sharing one work item's K range (1: no cluster)
+    int kt_per_split;         // K tiles of each
 };
+
+constexpr int kFPartRow = 2 * FN * 4 + 16;   // bytes of a parked accumulator row; 16 more so that
+                                             // eight lanes' 16-byte pieces hit different banks
+static_assert(FM * kFPartRow <= kFStages * kFStageBytes, "the parked tile takes the ring's place");
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
+    uint32_t addr;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
 
 // Shared-memory matrix descriptor of one scale atom for tcgen05.cp: 32 rows of 16 bytes, no
 // swizzle, 8-row core matrices 128 bytes apart.
@@ -144,11 +173,14 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
     pdl_wait_prior();
 
-    const int ktiles = (a.K + 255) / 256;
+    const int rank = static_cast<int>(blockIdx.x) % a.ksplit;    // of this CTA in its cluster
+    const int w0 = static_cast<int>(blockIdx.x) / a.ksplit, w_step = static_cast<int>(gridDim.x) / a.ksplit;
+    const int kt0 = rank * a.kt_per_split;
+    const int kt1 = min((a.K + 255) / 256, kt0 + a.kt_per_split);
     const int gpr = a.K >> 4;                        // scale groups per row (a multiple of 4)
     const long long sf_tile_bytes = 128ll * gpr;     // one 128-row tile of scale atoms
-    const int n_pairs = (a.n_tiles + 1) >> 1;
-    const int total = a.m_tiles * n_pairs;
+    const int n_items = (a.n_tiles + a.tile_cols - 1) / a.tile_cols;
+    const int total = a.m_tiles * n_items;
 
     if (warp == 4) {
         // ------------------------------ producer ------------------------------
@@ -157,9 +189,9 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         int s = 0;
         uint32_t lap = 0;
         bool ok = true;
-        for (int w = blockIdx.x; w < total && ok && !*abort_flag; w += gridDim.x) {
-            const int t = w % a.m_tiles, j = 2 * (w / a.m_tiles);
-            const bool two = j + 1 < a.n_tiles;
+        for (int w = w0; w < total && ok && !*abort_flag; w += w_step) {
+            const int t = w % a.m_tiles, j = a.tile_cols * (w / a.m_tiles);
+            const bool two = a.tile_cols == 2 && j + 1 < a.n_tiles;
             int mstart = t * FM;
             long long brow0 = static_cast<long long>(j) * FN;
             const uint8_t* sfa_tile = a.sfa + static_cast<long long>(t) * sf_tile_bytes;
@@ -173,7 +205,7 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 sfa_tile = a.sfa + (static_cast<long long>(a.sf_offsets[e]) + 128ll * local_tile) * gpr;
                 sfb_tile += static_cast<long long>(e) * a.sfb_expert_bytes;
             }
-            for (int kt = 0; kt < ktiles; ++kt) {
+            for (int kt = kt0; kt < kt1; ++kt) {
                 if (lap > 0)
                     ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], (lap - 1) & 1, a.status, kDevWaitEmpty));
                 if (!ok) break;
@@ -213,17 +245,17 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         int s = 0, tile_i = 0;
         uint32_t lap = 0;
         bool ok = true;
-        for (int w = blockIdx.x; w < total && ok && !*abort_flag; w += gridDim.x) {
-            const int t = w % a.m_tiles, j = 2 * (w / a.m_tiles);
+        for (int w = w0; w < total && ok && !*abort_flag; w += w_step) {
+            const int t = w % a.m_tiles, j = a.tile_cols * (w / a.m_tiles);
             if (a.tile_expert && a.tile_expert[t] < 0) continue;
-            const bool two = j + 1 < a.n_tiles;
+            const bool two = a.tile_cols == 2 && j + 1 < a.n_tiles;
             // one accumulator pair: the epilogue releases it as soon as it has read it out
             if (tile_i >= 1)
                 ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_empty[0], (tile_i - 1) & 1, a.status, kDevWaitTmem));
             if (!ok) break;
             tc_fence_after();
             const uint32_t d_tmem = tmem_base;
-            for (int kt = 0; kt < ktiles; ++kt) {
+            for (int kt = kt0; kt < kt1; ++kt) {
                 ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], lap & 1, a.status, kDevWaitFull));
                 if (!ok) break;
                 tc_fence_after();
@@ -241,7 +273,7 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     }
                     for (int k = 0; k < atoms; ++k) {
                         // 64 values = 32 bytes further along K inside the swizzle atom
-                        const uint32_t acc = (kt | k) != 0 ? 1u : 0u;
+                        const uint32_t acc = (kt != kt0 || k != 0) ? 1u : 0u;
                         tc_mma_nvf4(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, tmem_base + kFSfaCol + 4 * k,
                                     tmem_base + kFSfbCol + 4 * k, acc);
                         if (two)
@@ -265,8 +297,8 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     } else {
         // ------------------------------ epilogue (warps 0-3) ------------------------------
         int tile_i = 0;
-        for (int w = blockIdx.x; w < total && !*abort_flag; w += gridDim.x) {
-            const int t = w % a.m_tiles, j = 2 * (w / a.m_tiles);
+        for (int w = w0; w < total && !*abort_flag; w += w_step) {
+            const int t = w % a.m_tiles, j = a.tile_cols * (w / a.m_tiles);
             int mstart = t * FM, mend = a.M;
             float alpha = a.alpha_host;
             if (a.tile_expert) {
@@ -288,13 +320,27 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const int row = mstart + warp * 32 + lane;
             const bool row_ok = row < mend;
             const int n0 = j * FN;
-            const int ncols_all = min(2 * FN, a.N - n0);           // live columns of the pair
+            const int ncols_all = min(a.tile_cols * FN, a.N - n0);   // live columns of the item
             const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
             auto release = [&]() {
                 tc_fence_before();
                 __syncwarp();
                 if (elect_one()) mbar_arrive(&acc_empty[0]);
             };
+            if (a.ksplit > 1) {
+                // split K: park the tile in the ring's place, the sum follows after the cluster barrier
+                const uint32_t mine = smem_u32(smem) + static_cast<uint32_t>((warp * 32 + lane) * kFPartRow);
+                for (int c = 0; c < ncols_all; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(t_lane + c, r);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(mine + (c + 4 * q) * 4),
+                                     "r"(r[4 * q]), "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3])
+                                     : "memory");
+                }
+                break;   // one work item per cluster
+            }
             const bool vec_ok = (a.ldd & 7) == 0 && (reinterpret_cast<uintptr_t>(a.D) & 15) == 0 && (a.N & 31) == 0;
             if (a.out_dtype != LSG_DTYPE_F32 && vec_ok) {
                 // 16-bit outputs: the whole pair is read out of tensor memory into packed registers
@@ -335,8 +381,7 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
             } else {
 #pragma unroll 1
-                for (int c = 0; c < 2 * FN; c += 32) {
-                    if (c >= ncols_all) break;
+                for (int c = 0; c < ncols_all; c += 32) {
                     uint32_t r[32];
                     tmem_ld32(t_lane + c, r);
                     if (row_ok) {
@@ -367,6 +412,66 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tc_fence_after();
         tmem_dealloc(tmem_base, kFTmemCols);
     }
+    if (a.ksplit > 1) {
+        // Every thread of every CTA of the cluster comes here, after a time-out too.
+        cluster_sync();
+        const int mstart = (w0 % a.m_tiles) * FM, n0 = a.tile_cols * (w0 / a.m_tiles) * FN;
+        const int live = min(FM, a.M - mstart);
+        const int vecs = min(a.tile_cols * FN, a.N - n0) >> 2;   // 4-column pieces per row (N % 8 == 0)
+        const float alpha = a.alpha_host;
+        const uint32_t base = smem_u32(smem);
+        for (int i = rank * kFThreads + threadIdx.x; i < live * vecs; i += a.ksplit * kFThreads) {
+            const int r = i / vecs, c = (i - r * vecs) * 4;
+            const uint32_t at = base + static_cast<uint32_t>(r * kFPartRow + c * 4);
+            float4 v = ld_cluster_f4(at, 0);
+            for (int sp = 1; sp < a.ksplit; ++sp) {
+                const float4 p = ld_cluster_f4(at, sp);
+                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            }
+            v.x *= alpha; v.y *= alpha; v.z *= alpha; v.w *= alpha;
+            const size_t o = static_cast<size_t>(mstart + r) * a.ldd + n0 + c;
+            if (a.out_dtype == LSG_DTYPE_F32) {
+                *reinterpret_cast<float4*>(static_cast<float*>(a.D) + o) = v;
+            } else if (a.out_dtype == LSG_DTYPE_F16) {
+                const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.D) + o) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            } else {
+                const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.D) + o) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            }
+        }
+        __syncwarp();
+        cluster_sync();   // no CTA leaves while a peer still reads its shared memory
+    }
+}
+
+// How a dense call is cut: output tiles per work item (2 or 1) and CTAs per item along K.  An
+// unsplit CTA takes 0.78 us per K tile of a pair and about 0.52 us per K tile of a single output
+// tile (the bytes it pulls out of L2); splitting adds the parked tile, two cluster barriers and
+// the sum, 2 us.  The cheapest of the combinations whose CTAs are all resident at once wins; a
+// call that fills the chip without splitting keeps pairs and no cluster.
+struct SplitPlan {
+    int tile_cols, ksplit, kt_per_split;
+};
+SplitPlan split_plan(int m_tiles, int n_tiles, int ktiles, int sms) {
+    SplitPlan best = {2, 1, ktiles};
+    double best_us = 1e30;
+    for (int cols = 2; cols >= 1; --cols) {
+        const long long items = static_cast<long long>(m_tiles) * ((n_tiles + cols - 1) / cols);
+        const double us_kt = cols == 2 ? 0.78 : 0.52;
+        for (int ks = 1; ks <= 8; ks *= 2) {
+            const int kps = (ktiles + ks - 1) / ks;
+            if (ks > 1 && (items * ks > sms - sms / 8 || (ks - 1) * kps >= ktiles)) continue;
+            const double us = static_cast<double>((items * ks + sms - 1) / sms) * kps * us_kt + (ks > 1 ? 2.0 : 0.0);
+            if (us < best_us) {
+                best_us = us;
+                best = {cols, ks, kps};
+            }
+        }
+    }
+    return best;
 }
 
 // Packed e2m1 matrix [rows, K/2 bytes] -> tensor map with a (128 bytes x 128 rows) box.
@@ -418,6 +523,16 @@ int nvfp4_mma(const void* A, long long a_rows, const void* B, long long b_rows, 
     a.M = M; a.tile_expert = tile_expert; a.tile_mstart = tile_mstart; a.expert_offsets = expert_offsets;
     a.sf_offsets = sf_offsets;
     a.status = device_status_word();
+    a.tile_cols = 2;
+    a.ksplit = 1;
+    a.kt_per_split = (K + 255) / 256;
+    // the sum of split tiles stores 4-column pieces; grouped calls have their tiles on the device
+    if (!tile_expert && N % 8 == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0) {
+        const SplitPlan sp = split_plan(a.m_tiles, a.n_tiles, a.kt_per_split, sm_count());
+        a.tile_cols = sp.tile_cols;
+        a.ksplit = sp.ksplit;
+        a.kt_per_split = sp.kt_per_split;
+    }
     static bool configured[64] = {};
     int dev = 0;
     LSG_CUDA_TRY(cudaGetDevice(&dev));
@@ -425,7 +540,25 @@ int nvfp4_mma(const void* A, long long a_rows, const void* B, long long b_rows, 
         LSG_CUDA_TRY(cudaFuncSetAttribute(nvfp4_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    const long long items = static_cast<long long>(a.m_tiles) * ((a.n_tiles + 1) / 2);
+    const long long items = static_cast<long long>(a.m_tiles) * ((a.n_tiles + a.tile_cols - 1) / a.tile_cols);
+    if (a.ksplit > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(items * a.ksplit));
+        cfg.blockDim = dim3(kFThreads);
+        cfg.dynamicSmemBytes = kFSmem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = static_cast<unsigned>(a.ksplit);
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, nvfp4_mma_kernel, tmA, tmB, a));
+        return LSG_OK;
+    }
     int grid = sm_count();
     if (grid > items) grid = static_cast<int>(items);
     if (grid < 1) grid = 1;

@@ -147,6 +147,38 @@ def test_single_gemm_from_bf16(ops, M, N, K):
     assert cos > 0.99
 
 
+@pytest.mark.parametrize("dt", ["bf16", "fp16"])
+@pytest.mark.parametrize("M,N,K", [
+    (1, 32, 2112),        # one ragged output tile, K ends inside a 256-value tile
+    (77, 4096, 3584),     # ragged rows
+    (128, 264, 2048),     # last output tile of a pair is eight columns wide
+    (129, 1024, 4096),    # a second row tile with one live row
+    (300, 136, 1088),
+    (40, 100, 2048),      # N not a multiple of 8: never split
+])
+def test_single_gemm_few_rows_split_k(ops, M, N, K, dt):
+    """Sizes whose K range is shared by a cluster of CTAs: every output against the exact product.
+    The fp32 sum of K exact products is off by at most about sqrt(K) * 2^-24 of the row norms, far
+    below the rounding of the 16-bit result, so the bound is half a unit of that plus 1e-5."""
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
+    c, sc, s2 = Q.quantize_nvfp4(torch.randn(N, K, generator=g).numpy())
+    wdeq = torch.from_numpy(Q.dequantize_nvfp4(c, sc, 1.0).astype(np.float64)).cuda()
+    sfb = ops.nvfp4_gemm_preprocess(torch.from_numpy(sc).cuda(), N, K)
+    codes, sfa = ops.bf16_to_nvfp4(x)
+    lut = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, -0., -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64, device="cuda")
+    vals = lut[torch.stack([codes & 15, codes >> 4], -1).reshape(M, K).long()]
+    r, q = torch.arange(M, device="cuda")[:, None], torch.arange(K // 16, device="cuda")[None]
+    at = ((r // 128) * ((K // 16 + 3) // 4) + q // 4) * 512 + (r % 32) * 16 + ((r % 128) // 32) * 4 + q % 4
+    scale = sfa.view(torch.float8_e4m3fn).double()[at]
+    ref = float(np.float32(s2)) * ((vals.reshape(M, -1, 16) * scale[..., None]).reshape(M, K) @ wdeq.T)
+    wc = torch.from_numpy(c).cuda()
+    out = ops.nvfp4_gemm(codes, wc, sfa, sfb, M, N, K, float(s2), dt)
+    half_unit = 2.0 ** -8 if dt == "bf16" else 2.0 ** -11
+    assert ((out.double() - ref).abs() <= half_unit * ref.abs() + 1e-5 * ref.abs().max()).all()
+    assert torch.equal(out, ops.nvfp4_gemm(codes, wc, sfa, sfb, M, N, K, float(s2), dt))
+
+
 @pytest.mark.parametrize("N,K,s2", [(64, 256, 1.0), (130, 512, 0.0371), (1, 16, 3.5)])
 def test_nvfp4_dequant_bf16_bit_exact(ops, N, K, s2):
     """(e2m1 * e4m3 scale) * weight_scale_2 in fp32, rounded to bf16: same bits as the formula of
