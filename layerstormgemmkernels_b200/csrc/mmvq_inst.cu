@@ -2,7 +2,10 @@
 // eight decoders build in parallel.  Picks the kernel variant and the pipeline
 // geometry for a shape and launches it.
 #include "mmvq_grouped.cuh"
+#include "mmvq_mma.cuh"
 
+#include <atomic>
+#include <stdlib.h>
 
 #ifndef LSG_MMVQ_TYPE
 #error "compile with -DLSG_MMVQ_TYPE=<lsg_gguf_type id>"
@@ -48,6 +51,157 @@ int launch_rows(int rw, int lanes, const MmvqArgs& a, int grid, size_t smem, cud
     return launch_lanes<MT, 2>(lanes, a, grid, smem, stream, pdl);
 }
 
+// CTAs (clusters of CTAs) of a joined launch in proportion to the matrices' rows; what rounding
+// leaves over goes, one at a time, to the matrix with the most rows per CTA.  Returns the rows of
+// the fullest CTA.
+int share_ctas(int grid, int n_prob, const int* n_rows, int n_total, int* ctas_of) {
+    int used = 0;
+    for (int j = 0; j < n_prob; ++j) {
+        int g = static_cast<int>(static_cast<long long>(grid) * n_rows[j] / n_total);
+        ctas_of[j] = g < 1 ? 1 : g;
+        used += ctas_of[j];
+    }
+    while (used != grid) {
+        int pick = 0;
+        double worst = used < grid ? -1.0 : 1e30;
+        for (int j = 0; j < n_prob; ++j) {
+            const double load = static_cast<double>(n_rows[j]) / ctas_of[j];
+            if (used < grid ? load > worst : (ctas_of[j] > 1 && load < worst)) {
+                worst = load;
+                pick = j;
+            }
+        }
+        ctas_of[pick] += used < grid ? 1 : -1;
+        used += used < grid ? 1 : -1;
+    }
+    int rows_per_cta = 0;
+    for (int j = 0; j < n_prob; ++j) {
+        const int r = (n_rows[j] + ctas_of[j] - 1) / ctas_of[j];
+        rows_per_cta = r > rows_per_cta ? r : rows_per_cta;
+    }
+    return rows_per_cta;
+}
+
+// Row ranges of a joined launch: the first CTA of every matrix and its rows per CTA.
+void place_matrices(MmvqArgs& a, const int* n_rows, const int* ctas_of) {
+    a.rows_q = n_rows[0] / ctas_of[0];
+    a.rows_r = n_rows[0] % ctas_of[0];
+    int first = ctas_of[0];
+    for (int j = 0; j < a.n_extra; ++j) {
+        a.cta0x[j] = first;
+        a.rows_qx[j] = n_rows[1 + j] / ctas_of[1 + j];
+        a.rows_rx[j] = n_rows[1 + j] % ctas_of[1 + j];
+        first += ctas_of[1 + j];
+    }
+}
+
+// Batch rows from which the tensor-core mat-vec takes a call (LSG_MMVQ_MMA_ROWS=9: never).
+int mma_min_rows() {
+    static const int m = [] {
+        const char* e = getenv("LSG_MMVQ_MMA_ROWS");
+        return e ? atoi(e) : 2;
+    }();
+    return m;
+}
+
+// How the tensor-core mat-vec cuts K: by K and the type alone.
+bool mma_cut_k(MmaCut& g, int K) {
+    if (K % 256 != 0) return false;
+    g.sb_bytes = 256 / Fmt<T>::VALS * Fmt<T>::BYTES;
+    g.nsb = K / 256;
+    g.ksplit = 1;
+    while (g.ksplit < 8 && g.nsb > g.ksplit * kMmaSliceBlocks) g.ksplit *= 2;
+    g.slice = (g.nsb + g.ksplit - 1) / g.ksplit;
+    if (g.slice > kMmaSliceBlocks || (g.ksplit - 1) * g.slice >= g.nsb) return false;
+    g.wpg = g.slice > 4 ? 8 : (g.slice > 2 ? 4 : 2);   // short rows: fewer warps per row group, more groups
+    g.nc = (g.slice + g.wpg - 1) / g.wpg;
+    g.chunk = (g.slice + g.nc - 1) / g.nc;
+    return true;
+}
+
+// Shared memory: the deepest ring that fits (`sum_rows` rows of cluster sums).  Returns the bytes,
+// 0 when not even two stages per row group fit.
+template <class D>
+int mma_place(MmaCut& g, int sum_rows) {
+    const int nsets = kMmaWarps / g.wpg;
+    g.pitch = g.chunk * g.sb_bytes + (g.sb_bytes % 16 ? 32 : 0);
+    while (g.pitch % D::kPitchMod != D::kPitchRem) g.pitch = (g.pitch + 16) & ~15;
+    g.img_bytes = g.slice * 8 * (256 + (D::kSums ? 64 : 32));
+    const long long sum_bytes = static_cast<long long>(sum_rows + 15) / 16 * 16 * kMmaCols * 4;
+    const int bar_bytes = 2 * nsets * kMmaMaxRing * 8 + 16;
+    const int part_bytes = kMmaWarps * 2 * 128 * 4;
+    const long long avail = kSmemCap - g.img_bytes - part_bytes - sum_bytes - bar_bytes;
+    const long long ring = avail / (nsets * 16 * g.pitch);
+    if (avail < 0 || ring < 2) return 0;
+    g.ring = ring > kMmaMaxRing ? kMmaMaxRing : static_cast<int>(ring);
+    g.part_off = g.img_bytes + nsets * g.ring * 16 * g.pitch;
+    g.sum_off = g.part_off + part_bytes;
+    g.bar_off = g.sum_off + static_cast<int>(sum_bytes);
+    return g.bar_off + bar_bytes;
+}
+
+// The tensor-core mat-vec (mmvq_mma.cuh), or kMmaNotTaken.
+constexpr int kMmaNotTaken = 1;
+template <int TT>
+int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
+    if constexpr (MmaDec<TT>::kHas) {
+        MmaArgs g = {};
+        g.v = v;
+        if (v.M > kMmaCols || v.drop_slab >= 0 || !mma_cut_k(g.c, v.K)) return kMmaNotTaken;
+        auto kernel = mmvq_mma_kernel<TT>;
+        static std::atomic<int> clusters[64][4];   // resident clusters of 1, 2, 4, 8 CTAs, per device
+        int dev = 0;
+        LSG_CUDA_TRY(cudaGetDevice(&dev));
+        const int log_split = g.c.ksplit == 1 ? 0 : (g.c.ksplit == 2 ? 1 : (g.c.ksplit == 4 ? 2 : 3));
+        cudaLaunchConfig_t cfg = {};
+        cfg.blockDim = dim3(kMmaThreads);
+        cfg.dynamicSmemBytes = kSmemCap;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(g.c.ksplit);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int slots = dev >= 0 && dev < 64 ? clusters[dev][log_split].load(std::memory_order_relaxed) : 0;
+        if (slots == 0) {
+            LSG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
+            slots = sm_count();
+            if (g.c.ksplit > 1) {
+                cfg.gridDim = dim3(static_cast<unsigned>(g.c.ksplit));
+                LSG_CUDA_TRY(cudaOccupancyMaxActiveClusters(&slots, kernel, &cfg));
+                if (slots < 1) return kMmaNotTaken;
+            }
+            if (dev >= 0 && dev < 64) clusters[dev][log_split].store(slots, std::memory_order_relaxed);
+        }
+        MmvqArgs& a = g.v;
+        a.row_bytes = g.c.nsb * g.c.sb_bytes;
+        const int n_prob = 1 + a.n_extra;
+        int n_rows[1 + kMmvqMaxExtra] = {a.N}, ctas_of[1 + kMmvqMaxExtra] = {};
+        int n_total = a.N;
+        for (int j = 0; j < a.n_extra; ++j) {
+            n_rows[1 + j] = a.Nx[j];
+            n_total += a.Nx[j];
+        }
+        const int grid = n_total < slots ? n_total : slots;
+        if (grid < n_prob) return kMmaNotTaken;
+        const int rows = share_ctas(grid, n_prob, n_rows, n_total, ctas_of);
+        place_matrices(a, n_rows, ctas_of);
+        const int smem = mma_place<MmaDec<TT>>(g.c, g.c.ksplit > 1 ? rows : 0);
+        if (smem == 0) return kMmaNotTaken;
+        cfg.gridDim = dim3(static_cast<unsigned>(grid * g.c.ksplit));
+        cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+        if (g.c.ksplit == 1) cfg.attrs = attr + 1;   // no cluster
+        cfg.numAttrs = (g.c.ksplit > 1 ? 1 : 0) + (pdl ? 1 : 0);
+        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, g));
+        return LSG_OK;
+    }
+    return kMmaNotTaken;
+}
+
 }  // namespace
 
 // Largest number of batch rows one launch can hold in shared memory.
@@ -63,6 +217,10 @@ int MMVQ_FN(max_rows)(int K) {
 int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool pdl) {
     using F = Fmt<T>;
     a.row_bytes = (a.K / F::VALS) * F::BYTES;
+    if (a.M >= mma_min_rows() && !tn_in.skip_math) {
+        const int rc = launch_mma<T>(a, stream, pdl);
+        if (rc != kMmaNotTaken) return rc;
+    }
     // Small matrices (a CTA's share of the weights is at most 40 KB, e.g. a 1024 x 4096 Q4_K
     // k or v projection launched alone): eleven
     // consumer warps and half the shared memory, so that two consecutive launches of a
@@ -126,32 +284,7 @@ int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool
         grid = n_total < slots ? n_total : slots;
         int rows_per_cta = (n_total + grid - 1) / grid;
         if (n_prob > 1) {
-            // CTAs in proportion to the rows; what rounding leaves over goes, one at a
-            // time, to the matrix with the most rows per CTA.
-            int used = 0;
-            for (int j = 0; j < n_prob; ++j) {
-                int g = static_cast<int>(static_cast<long long>(grid) * n_rows[j] / n_total);
-                ctas_of[j] = g < 1 ? 1 : g;
-                used += ctas_of[j];
-            }
-            while (used != grid) {
-                int pick = 0;
-                double worst = used < grid ? -1.0 : 1e30;
-                for (int j = 0; j < n_prob; ++j) {
-                    const double load = static_cast<double>(n_rows[j]) / ctas_of[j];
-                    if (used < grid ? load > worst : (ctas_of[j] > 1 && load < worst)) {
-                        worst = load;
-                        pick = j;
-                    }
-                }
-                ctas_of[pick] += used < grid ? 1 : -1;
-                used += used < grid ? 1 : -1;
-            }
-            rows_per_cta = 0;
-            for (int j = 0; j < n_prob; ++j) {
-                const int r = (n_rows[j] + ctas_of[j] - 1) / ctas_of[j];
-                rows_per_cta = r > rows_per_cta ? r : rows_per_cta;
-            }
+            rows_per_cta = share_ctas(grid, n_prob, n_rows, n_total, ctas_of);
         }
         // Long rows: one row per lane group, so that the rows resident in the ring
         // are enough to occupy every consumer warp.
@@ -191,17 +324,7 @@ int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool
         break;
     }
 
-    if (n_prob > 1) {
-        a.rows_q = n_rows[0] / ctas_of[0];
-        a.rows_r = n_rows[0] % ctas_of[0];
-        int first = ctas_of[0];
-        for (int j = 0; j < a.n_extra; ++j) {
-            a.cta0x[j] = first;
-            a.rows_qx[j] = n_rows[1 + j] / ctas_of[1 + j];
-            a.rows_rx[j] = n_rows[1 + j] % ctas_of[1 + j];
-            first += ctas_of[1 + j];
-        }
-    }
+    if (n_prob > 1) place_matrices(a, n_rows, ctas_of);
     finish_args(a, grid, (32 / lanes) * rw);
     if (a.M == 1) return launch_rows<1>(rw, lanes, a, grid, smem, stream, pdl);
     if (a.M == 2) return launch_rows<2>(rw, lanes, a, grid, smem, stream, pdl);
@@ -229,10 +352,42 @@ int launch_grouped_variant(const GroupedArgs& a, int grid, size_t smem, cudaStre
 constexpr int kGroupedCtlBytes = 2 * kMmvqMaxStages * 8 + 16 + kMmvqMaxStages * 4 + 3 * kGroupedMaxSlabs * 4;
 constexpr int kGroupedImageBudget = 64 * 1024;  // activation image of one segment
 
+// Whether grouped calls of this type and K take the tensor-core mat-vec, whose segments hold up
+// to eight rows; its cut and shared memory when they do.
+template <int TT>
+bool grouped_mma(int K, MmaCut& c, int& smem) {
+    if constexpr (MmaDec<TT>::kHas) {
+        if (mma_min_rows() > kMmaCols || !mma_cut_k(c, K) || c.ksplit > 1) return false;
+        smem = mma_place<MmaDec<TT>>(c, 0);
+        return smem > 0;
+    }
+    return false;
+}
+
+template <int TT>
+int launch_grouped_mma(const GroupedArgs& v, const MmaCut& c, int smem, cudaStream_t stream, bool pdl) {
+    if constexpr (MmaDec<TT>::kHas) {
+        MmaGroupedArgs g = {v, c};
+        g.v.row_bytes = c.nsb * c.sb_bytes;
+        static std::atomic<bool> configured[64];
+        int dev = 0;
+        LSG_CUDA_TRY(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_relaxed)) {
+            LSG_CUDA_TRY(cudaFuncSetAttribute(mmvq_mma_grouped_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
+            if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_relaxed);
+        }
+        LSG_CUDA_TRY(launch_kernel(mmvq_mma_grouped_kernel<TT>, dim3(sm_count()), dim3(kMmaThreads), smem, stream, pdl, g));
+    }
+    return LSG_OK;
+}
+
 }  // namespace
 
 // Rows of one segment: as many batch rows as fit the image budget (at least 1, at most 64).
 int MMVQ_FN(grouped_max_rows)(int K, const MmvqTune&) {
+    MmaCut c = {};
+    int smem = 0;
+    if (grouped_mma<T>(K, c, smem)) return kMmaCols;
     int rows = kGroupedImageBudget / x_row_bytes<T>(K);
     if (rows > 64) rows = 64;
     if (rows >= 8) rows &= ~7;
@@ -242,6 +397,9 @@ int MMVQ_FN(grouped_max_rows)(int K, const MmvqTune&) {
 int MMVQ_FN(grouped_launch)(GroupedArgs a, const MmvqTune& tn, int max_segments, cudaStream_t stream,
                             bool pdl) {
     using F = Fmt<T>;
+    MmaCut c = {};
+    int mma_smem = 0;
+    if (grouped_mma<T>(a.K, c, mma_smem)) return launch_grouped_mma<T>(a, c, mma_smem, stream, pdl);
     a.row_bytes = (a.K / F::VALS) * F::BYTES;
     a.cons_warps = tn.warps;
     const int U = a.K / Mmvq<T>::UV;

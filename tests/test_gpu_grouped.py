@@ -115,6 +115,17 @@ def test_grouped_single_expert_and_determinism(ops, name, m):
     check(single.cpu().numpy(), ref, TOL_F32)
 
 
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "Q4_0"])
+@pytest.mark.parametrize("N,K", [(768, 2048), (2056, 768), (17, 256), (300, 1280), (40, 4096)])
+def test_grouped_matvec_edges(ops, name, N, K):
+    """Row groups and segments at their edges: experts with 0, 1, 8, 9 and 17 rows, ragged N, one
+    to sixteen blocks per row."""
+    A, off, ptrs, dev_w, host_w, offs = build_group(name, [1, 0, 8, 9, 17, 3], N, K, seed=N)
+    ref = oracle_grouped(name, A, host_w, offs, K)
+    out = ops.gguf_grouped_gemm(A, off, ptrs, T[name], S_INT, N, K, F_MMVQ, out_dtype=torch.float32)
+    check(out.cpu().numpy(), ref, TOL_F32)
+
+
 @pytest.mark.parametrize("name", ["Q8_0", "Q4_K", "Q6_K"])
 def test_grouped_topk_like_counts(ops, name):
     """Uneven counts as top-k routing produces (tests/test_gguf_grouped_gemm.py:202-221)."""

@@ -133,6 +133,34 @@ def test_mmvq_q4k_golden_fixture(ops, golden_dir):
     assert rel_err(got, ref) <= TOL_F32
 
 
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "Q4_0"])
+@pytest.mark.parametrize("M,N,K", [
+    (2, 1, 256),        # one block, one row
+    (3, 17, 768),       # three blocks, a row group with one live row
+    (8, 2400, 1280),    # several row groups per CTA, the last one ragged
+    (5, 300, 4096),     # the longest row one CTA takes
+    (8, 33, 4352),      # K shared by two CTAs, odd number of blocks
+    (4, 161, 8448),     # by four
+    (7, 700, 14336),    # activations quantized by a kernel of their own
+    (2, 40, 16640),     # by eight, the last one with fewer blocks
+])
+def test_mmvq_tensor_core_edges(ops, name, M, N, K):
+    """Two to eight batch rows, at the edges of the row groups and of the cuts of K: same integers
+    as the oracle, so only the order of the fp32 sums differs (TOL_F32); and independent of what
+    shares the launch."""
+    t = T[name]
+    A = torch.randn(M, K, generator=torch.Generator().manual_seed(N)).to(torch.bfloat16).cuda()
+    W = Q.random_gguf_weight(name, N, K, seed=K)
+    Wd = torch.from_numpy(W).cuda()
+    ref = oracle.mmvq(t, oracle.quantize_q8_1(bf16_bits(A)), W, K)
+    got = ops.gguf_mmvq(A, Wd, t, N, K, out_dtype=torch.float32)
+    assert rel_err(got.cpu().numpy(), ref) <= TOL_F32
+    W2 = torch.from_numpy(Q.random_gguf_weight(name, 50, K, seed=K + 1)).cuda()
+    both = ops.gguf_mmvq_batch(A, [(W2, 50), (Wd, N)], t, out_dtype=torch.float32)
+    assert torch.equal(both[1], got)
+    assert torch.equal(both[0], ops.gguf_mmvq(A, W2, t, 50, K, out_dtype=torch.float32))
+
+
 def test_mmvq_bit_deterministic(ops):
     """tests/test_gguf_mmvq.py:91-103."""
     N, K = 640, 1024
