@@ -77,11 +77,12 @@ int check_common(const lsg_gguf_grouped_gemm_params* p) {
 
 // The grouped mat-vec over a device-built segment list: activations quantized into the
 // workspace (skipped when `xq_ready`: the caller, or the call in front with the same A_base, K
-// and workspace, left them there) and segments built from the offsets (skipped when
-// `seg_ready`: the call in front had the same offsets and K and skipped the same experts - the
-// caller guarantees that an expert has a weight here when it had one there), then one launch.
+// and workspace, left them there) and segments built from the offsets (`seg_ready` is the list of
+// a call in front with the same offsets and the same rows per segment that skipped the same
+// experts - the caller guarantees that an expert has a weight here when it had one there), then
+// one launch.
 int grouped_matvec_tail(const lsg_gguf_grouped_gemm_params* p, int T, uint8_t* base, const WsLayout& w,
-                        cudaStream_t s, bool xq_ready, bool seg_ready) {
+                        cudaStream_t s, bool xq_ready, const int* seg_ready) {
     int rc = LSG_OK;
     if (!xq_ready) {
         rc = quantize_q8_1(p->A_base, base, T, p->K, s, true);
@@ -98,7 +99,7 @@ int grouped_matvec_tail(const lsg_gguf_grouped_gemm_params* p, int T, uint8_t* b
     GroupedArgs a = {};
     a.xq = base;
     a.B_ptrs = p->B_ptrs;
-    a.seg = seg;
+    a.seg = seg_ready ? seg_ready : seg;
     a.D = p->D_base;
     a.status = device_status_word();
     a.N = p->N;
@@ -160,7 +161,7 @@ int grouped_int(const lsg_gguf_grouped_gemm_params* p, int T, void* ws, size_t w
                            p->out_dtype == LSG_DTYPE_F32, tile_expert, tile_mstart, t_max,
                            base + w.total, ws_bytes - w.total, s);
     }
-    return grouped_matvec_tail(p, T, base, w, s, false, false);
+    return grouped_matvec_tail(p, T, base, w, s, false, nullptr);
 }
 
 // Host per-expert loop: the golden of both strategies and the Dequant implementation.
@@ -212,10 +213,12 @@ int grouped_hostloop(const lsg_gguf_grouped_gemm_params* p, void* ws, size_t ws_
 // The mat-vec route of lsg_gguf_grouped_gemm for a caller inside the library that runs several
 // projections of the same rows through the same workspace (gate and up of an expert block):
 // `xq_ready` skips the activation quantizer (the Q8_1 blocks of all T rows are at the start of
-// the workspace already) and `seg_ready` the segment list (every expert with rows has all its
-// weights: lsg_gguf_moe_ffn's contract).  A_base may be null with `xq_ready`.
+// the workspace already).  `seg_k` is the K of an earlier call of the block whose segment list is
+// still in the workspace, 0 when there is none (every expert with rows has all its weights:
+// lsg_gguf_moe_ffn's contract); the list serves when it was cut into segments of the same rows and
+// this call's Q8_1 blocks end in front of it.  A_base may be null with `xq_ready`.
 int grouped_gemm_matvec(const lsg_gguf_grouped_gemm_params* p, int T, void* ws, size_t ws_bytes, cudaStream_t s,
-                        bool xq_ready, bool seg_ready) {
+                        bool xq_ready, int seg_k) {
     int rc = check_common(p);
     if (rc != LSG_OK) return rc;
     if (p->num_experts <= 0 || T <= 0) return LSG_OK;
@@ -227,7 +230,14 @@ int grouped_gemm_matvec(const lsg_gguf_grouped_gemm_params* p, int T, void* ws, 
     const WsLayout w = ws_layout(T, p->K, p->num_experts);
     if (ws_bytes < w.total)
         return fail(LSG_ERR_WORKSPACE, "GGUF grouped int: workspace too small (have %zu, need %zu)", ws_bytes, w.total);
-    return grouped_matvec_tail(p, T, static_cast<uint8_t*>(ws), w, s, xq_ready, seg_ready);
+    const int* seg = nullptr;
+    if (seg_k > 0) {
+        const WsLayout first = ws_layout(T, seg_k, p->num_experts);
+        const MmvqTune tn = mmvq_tuning();
+        if (w.q8_bytes <= first.seg_off && grouped_max_rows(p->type, seg_k, tn) == grouped_max_rows(p->type, p->K, tn))
+            seg = reinterpret_cast<const int*>(static_cast<uint8_t*>(ws) + first.seg_off);
+    }
+    return grouped_matvec_tail(p, T, static_cast<uint8_t*>(ws), w, s, xq_ready, seg);
 }
 
 }  // namespace lsg

@@ -10,13 +10,40 @@
 //   * segment list        - (expert, first row, rows) pieces of at most `max_rows` rows,
 //     the work list of the grouped mat-vec kernel (no counterpart in the reference).
 //
-// One warp does each scan with ballots / prefix sums; expert counts are a few hundred.
+// One CTA does each scan, an expert per thread (expert counts are a few hundred): with one warp
+// the dependent loads of every 32 experts came one after the other, 5-7 us a list of 128.
 #include "common.cuh"
 #include "host.h"
 
 namespace lsg {
 
 namespace {
+
+constexpr int kScanThreads = 256;
+
+// Sum of v over the threads in front of this one; `all` becomes the sum over the CTA.
+__device__ __forceinline__ int scan_exclusive(int v, int& all) {
+    __shared__ int warp_sum[kScanThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    __syncthreads();   // the sums of an earlier call have been read
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    all = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+        const int x = warp_sum[w];
+        before += w < warp ? x : 0;
+        all += x;
+    }
+    return before + incl - v;
+}
 
 __global__ void active_expert_list_kernel(const int32_t* __restrict__ offs, int E, int cap,
                                           int* __restrict__ active) {
@@ -45,10 +72,9 @@ __global__ void mmq_tile_map_kernel(const int32_t* __restrict__ offs, int E, int
                                     int balanced, int* __restrict__ tile_expert, int* __restrict__ tile_mstart) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    const int lane = threadIdx.x & 31;
-    int t0 = 0;  // tiles emitted so far (warp-uniform)
-    for (int base = 0; base < E; base += 32) {
-        const int e = base + lane;
+    int t0 = 0;  // tiles emitted so far (the same in every thread)
+    for (int base = 0; base < E; base += kScanThreads) {
+        const int e = base + threadIdx.x;
         int off = 0, nt = 0, height = tile_m;
         if (e < E) {
             off = min(offs[e], rows);
@@ -56,14 +82,8 @@ __global__ void mmq_tile_map_kernel(const int32_t* __restrict__ offs, int E, int
             nt = m > 0 ? (m + tile_m - 1) / tile_m : 0;
             if (balanced && nt > 0) height = balanced_tile_rows(m, tile_m);
         }
-        // exclusive prefix sum of nt over the warp
-        int incl = nt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int first = t0 + incl - nt;
+        int all;
+        const int first = t0 + scan_exclusive(nt, all);
         for (int i = 0; i < nt; ++i) {
             const int t = first + i;
             if (t < T_max) {
@@ -71,9 +91,9 @@ __global__ void mmq_tile_map_kernel(const int32_t* __restrict__ offs, int E, int
                 tile_mstart[t] = off + i * height;
             }
         }
-        t0 += __shfl_sync(0xffffffffu, incl, 31);
+        t0 += all;
     }
-    for (int t = t0 + lane; t < T_max; t += 32) {
+    for (int t = t0 + threadIdx.x; t < T_max; t += kScanThreads) {
         tile_expert[t] = -1;
         tile_mstart[t] = 0;
     }
@@ -86,10 +106,9 @@ __global__ void segment_list_kernel(const int32_t* __restrict__ offs, const void
                                     int E, int max_rows, int max_segments, int rows, int* __restrict__ seg) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    const int lane = threadIdx.x & 31;
     int s0 = 0;
-    for (int base = 0; base < E; base += 32) {
-        const int e = base + lane;
+    for (int base = 0; base < E; base += kScanThreads) {
+        const int e = base + threadIdx.x;
         int off = 0, m = 0, ns = 0;
         if (e < E) {
             off = min(offs[e], rows);
@@ -97,13 +116,8 @@ __global__ void segment_list_kernel(const int32_t* __restrict__ offs, const void
             if (m < 0 || B_ptrs[e] == nullptr) m = 0;
             ns = (m + max_rows - 1) / max_rows;
         }
-        int incl = ns;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int first = s0 + incl - ns;
+        int all;
+        const int first = s0 + scan_exclusive(ns, all);
         for (int i = 0; i < ns; ++i) {
             const int s = first + i;
             if (s < max_segments) {
@@ -112,9 +126,9 @@ __global__ void segment_list_kernel(const int32_t* __restrict__ offs, const void
                 seg[3 + 3 * s] = min(max_rows, m - i * max_rows);
             }
         }
-        s0 += __shfl_sync(0xffffffffu, incl, 31);
+        s0 += all;
     }
-    if (lane == 0) seg[0] = min(s0, max_segments);
+    if (threadIdx.x == 0) seg[0] = min(s0, max_segments);
 }
 
 }  // namespace
@@ -129,14 +143,14 @@ int build_active_expert_list(const int32_t* offs, int E, int cap, int* active, c
 int build_mmq_tile_map(const int32_t* offs, int E, int tile_m, int T_max, int* tile_expert,
                        int* tile_mstart, cudaStream_t s, int rows, bool balanced) {
     if (T_max <= 0) return LSG_OK;
-    LSG_CUDA_TRY(launch_kernel(mmq_tile_map_kernel, dim3(1), dim3(32), 0, s, true, offs, E, tile_m,
+    LSG_CUDA_TRY(launch_kernel(mmq_tile_map_kernel, dim3(1), dim3(kScanThreads), 0, s, true, offs, E, tile_m,
                                T_max, rows, balanced ? 1 : 0, tile_expert, tile_mstart));
     return LSG_OK;
 }
 
 int build_segment_list(const int32_t* offs, const void* const* B_ptrs, int E, int max_rows,
                        int max_segments, int* seg, cudaStream_t s, int rows) {
-    LSG_CUDA_TRY(launch_kernel(segment_list_kernel, dim3(1), dim3(32), 0, s, true, offs, B_ptrs, E,
+    LSG_CUDA_TRY(launch_kernel(segment_list_kernel, dim3(1), dim3(kScanThreads), 0, s, true, offs, B_ptrs, E,
                                max_rows, max_segments, rows, seg));
     return LSG_OK;
 }
