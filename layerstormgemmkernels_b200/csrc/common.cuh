@@ -151,6 +151,28 @@ __device__ __forceinline__ void q8_round8(const float* x, float d, float rcp, ui
     w1 = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
 }
 
+// The Q8_1 round trip of eight values of one block, dh * rn(fl(x / d)) as floats, on the arithmetic
+// of q8_round8 (the rounded quotient is read back by subtracting the magic number instead of being
+// taken off the mantissa; a quotient that rounds to -0 comes out as +0).
+__device__ __forceinline__ void q8_roundtrip8(const float* x, float d, float rcp, float dh, float* out) {
+    const float magic = 12582912.0f;
+    float km[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float t = x[i] * rcp;
+        km[i] = fmaf(fmaf(-t, d, x[i]), rcp, t) + magic;
+    }
+    const float m = max_nan(max_nan(max_nan(km[0], km[1]), max_nan(km[2], km[3])),
+                            max_nan(max_nan(km[4], km[5]), max_nan(km[6], km[7])));
+    if (!(d >= 1e-28f && d <= 1e30f) || m != m) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[i] = dh * q8_round_f(x[i], d, rcp);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = dh * (km[i] - magic);
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
                  : "memory");

@@ -889,18 +889,9 @@ x_prep_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ out, int
         const float d = amax / 127.0f;
         const float rcp = (amax == 0.0f) ? 0.0f : 1.0f / d;
         const float dh = __half2float(__float2half(d));
-        uint32_t pk[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float r2[2];
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                // same integer as rn(fl(x / d)): the product with the reciprocal only differs
-                // next to a half-integer, and there the true quotient decides
-                r2[hh] = dh * q8_round_f(val[2 * i + hh], d, rcp);
-            }
-            pk[i] = pack_h2(r2[0], r2[1]);
-        }
+        float q[8];
+        q8_roundtrip8(val, d, rcp, dh, q);
+        const uint32_t pk[4] = {pack_h2(q[0], q[1]), pack_h2(q[2], q[3]), pack_h2(q[4], q[5]), pack_h2(q[6], q[7])};
         if (ok[j]) {
             const int r = rbase + j * blockDim.y;
             reinterpret_cast<uint4*>(out)[static_cast<size_t>(r) * vpr + v] = make_uint4(pk[0], pk[1], pk[2], pk[3]);

@@ -395,6 +395,140 @@ __global__ void weights_to_f16_kernel(const uint8_t* __restrict__ W, const void*
     }
 }
 
+// The same for the types in use, 32 x 256 values per CTA.  With a thread per 32 values fetching its
+// bytes one by one the pass was bound by instruction issue (4096 x 14336 of Q6_K: 63.8 us for
+// 165 MB, 31.5 us now); here the packed bytes come in as 16-byte pieces through shared memory, a thread turns
+// eight of them at a time into floats with one permute and one subtraction each, and neighbouring
+// lanes store neighbouring 16-byte pieces.  Same fp32 products as dequant_chunk32.
+//
+// pack8(): values 8g .. 8g + 7 of the 256 at shared address b, as four fp16 pairs.
+template <int T> struct W8 { static constexpr bool kHas = false; };
+
+// byte k of w as 2^23 + byte, less `bias`: exact
+__device__ __forceinline__ float biased_byte(uint32_t w, int k, float bias) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7550u | k)) - bias;
+}
+__device__ __forceinline__ void pack8_scaled(const uint32_t (&q)[2], float bias, float s, uint32_t (&p)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 h = __floats2half2_rn(s * biased_byte(q[i >> 1], 2 * (i & 1), bias), s * biased_byte(q[i >> 1], 2 * (i & 1) + 1, bias));
+        p[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+}
+template <bool FIVE> struct W8K45 {
+    static constexpr bool kHas = true;
+    __device__ static __forceinline__ void pack8(uint32_t b, int g, uint32_t (&p)[4]) {
+        const int c = g >> 2, l0 = (g & 3) * 8;
+        uint32_t h[4], q[2];
+        lds_words_unaligned<4>(b, h);
+        // 6-bit scale and minimum c of the 12 bytes behind (d, dmin)
+        const int k = 8 * (c & 3);
+        uint32_t sc, mn;
+        if (c < 4) {
+            sc = (h[1] >> k) & 63u;
+            mn = (h[2] >> k) & 63u;
+        } else {
+            sc = ((h[3] >> k) & 15u) | (((h[1] >> k) & 0xC0u) >> 2);
+            mn = ((h[3] >> (k + 4)) & 15u) | (((h[2] >> k) & 0xC0u) >> 2);
+        }
+        const float ds = fp16_bits_to_float(h[0]) * static_cast<float>(sc), ms = fp16_bits_to_float(h[0] >> 16) * static_cast<float>(mn);
+        lds_words_unaligned<2>(b + (FIVE ? 48 : 16) + 32 * (c >> 1) + l0, q);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) q[i] = (q[i] >> (4 * (c & 1))) & 0x0F0F0F0Fu;
+        if (FIVE) {
+            uint32_t f[2];
+            lds_words_unaligned<2>(b + 16 + l0, f);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) q[i] |= ((f[i] >> c) & 0x01010101u) << 4;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __half2 v = __floats2half2_rn(fmaf(ds, biased_byte(q[i >> 1], 2 * (i & 1), 8388608.0f), -ms),
+                                                fmaf(ds, biased_byte(q[i >> 1], 2 * (i & 1) + 1, 8388608.0f), -ms));
+            p[i] = *reinterpret_cast<const uint32_t*>(&v);
+        }
+    }
+};
+template <> struct W8<LSG_GGUF_Q4_K> : W8K45<false> {};
+template <> struct W8<LSG_GGUF_Q5_K> : W8K45<true> {};
+template <> struct W8<LSG_GGUF_Q6_K> {
+    static constexpr bool kHas = true;
+    __device__ static __forceinline__ void pack8(uint32_t b, int g, uint32_t (&p)[4]) {
+        const int ip = g >> 4, quad = (g >> 2) & 3, l0 = (g & 3) * 8;
+        uint32_t q[2], h[2];
+        lds_words_unaligned<2>(b + 64 * ip + 32 * (quad & 1) + l0, q);
+        lds_words_unaligned<2>(b + 128 + 32 * ip + l0, h);
+        const uint32_t at = b + 192 + 8 * ip + 2 * quad + (l0 >> 4);
+        const int sc = static_cast<int>(static_cast<int8_t>(lds8(at)));
+        const float s = fp16_bits_to_float(lds16(b + 208)) * static_cast<float>(sc);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            q[i] = ((q[i] >> (4 * (quad >> 1))) & 0x0F0F0F0Fu) | (((h[i] >> (2 * quad)) & 0x03030303u) << 4);
+        pack8_scaled(q, 8388608.0f + 32.0f, s, p);
+    }
+};
+template <> struct W8<LSG_GGUF_Q8_0> {
+    static constexpr bool kHas = true;
+    __device__ static __forceinline__ void pack8(uint32_t b, int g, uint32_t (&p)[4]) {
+        b += 34 * (g >> 2);
+        uint32_t q[2];
+        lds_words_unaligned<2>(b + 2 + 8 * (g & 3), q);
+        q[0] ^= 0x80808080u;
+        q[1] ^= 0x80808080u;
+        pack8_scaled(q, 8388608.0f + 128.0f, fp16_bits_to_float(lds16(b)), p);
+    }
+};
+template <> struct W8<LSG_GGUF_Q4_0> {
+    static constexpr bool kHas = true;
+    __device__ static __forceinline__ void pack8(uint32_t b, int g, uint32_t (&p)[4]) {
+        b += 18 * (g >> 2);
+        uint32_t q[2];
+        lds_words_unaligned<2>(b + 2 + 8 * (g & 1), q);   // low nibbles: values 0-15, high nibbles: 16-31
+#pragma unroll
+        for (int i = 0; i < 2; ++i) q[i] = (q[i] >> (2 * (g & 2))) & 0x0F0F0F0Fu;
+        pack8_scaled(q, 8388608.0f + 8.0f, fp16_bits_to_float(lds16(b)), p);
+    }
+};
+
+constexpr int kW8Blocks = 32;   // 256-value blocks per CTA: 32 of any type are whole 16-byte pieces
+template <int T>
+__global__ void __launch_bounds__(256)
+weights_to_f16_staged_kernel(const uint8_t* __restrict__ W, const void* const* __restrict__ B_ptrs,
+                             const int32_t* __restrict__ expert_offsets, __half* __restrict__ out, int N, int K) {
+    constexpr int kBytes = 256 / Fmt<T>::VALS * Fmt<T>::BYTES;
+    __shared__ __align__(16) uint8_t stage[kW8Blocks * kBytes + 16];   // the word behind the last one is read too
+    pdl_launch_dependents();
+    pdl_wait_prior();
+    const int e = blockIdx.y;
+    const uint8_t* base = W;
+    if (B_ptrs) {
+        if (expert_offsets[e + 1] - expert_offsets[e] <= 0) return;
+        base = static_cast<const uint8_t*>(B_ptrs[e]);
+        if (!base) return;
+    }
+    const long long values = static_cast<long long>(N) * K;
+    const long long v0 = static_cast<long long>(blockIdx.x) * (kW8Blocks * 256);
+    const int live = static_cast<int>(min(values - v0, static_cast<long long>(kW8Blocks * 256)));   // whole 32-value groups
+    const uint8_t* src = base + v0 / 256 * kBytes;
+    const int bytes = live / Fmt<T>::VALS * Fmt<T>::BYTES;
+    const int whole = (reinterpret_cast<uintptr_t>(base) & 15) == 0 ? bytes & ~15 : 0;   // a matrix off a 16-byte boundary: bytes
+    for (int i = threadIdx.x * 16; i < whole; i += 256 * 16)
+        *reinterpret_cast<uint4*>(stage + i) = __ldg(reinterpret_cast<const uint4*>(src + i));
+    for (int i = whole + threadIdx.x; i < bytes; i += 256) stage[i] = __ldg(src + i);
+    __syncthreads();
+    const uint32_t sb = smem_u32(stage);
+    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<long long>(e) * values + v0);
+#pragma unroll
+    for (int it = 0; it < kW8Blocks * 32 / 256; ++it) {
+        const int i = it * 256 + threadIdx.x;
+        if (i * 8 < live) {
+            uint32_t p[4];
+            W8<T>::pack8(sb + (i >> 5) * kBytes, i & 31, p);
+            dst[i] = make_uint4(p[0], p[1], p[2], p[3]);
+        }
+    }
+}
+
 // bf16 x[M,K] -> fp16 of the Q8_1 round trip: d_h * rn(x / d) with d = amax/127 per 32
 // values and d_h its fp16 rounding (what the integer paths multiply by).  Four lanes per
 // block, eight values per lane.
@@ -422,15 +556,12 @@ x_q8_1_roundtrip_f16_kernel(const __nv_bfloat16* __restrict__ x, __half* __restr
     const float d = amax / 127.0f;
     const float rcp = (amax == 0.0f) ? 0.0f : 1.0f / d;
     const float dh = __half2float(__float2half(d));
+    float r[8];
+    q8_roundtrip8(v, d, rcp, dh, r);
     uint32_t p[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        float r[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            r[h] = dh * q8_round_f(v[2 * i + h], d, rcp);   // same integer as rn(fl(x / d))
-        }
-        const __half2 hv = __floats2half2_rn(r[0], r[1]);
+        const __half2 hv = __floats2half2_rn(r[2 * i], r[2 * i + 1]);
         p[i] = *reinterpret_cast<const uint32_t*>(&hv);
     }
     reinterpret_cast<uint4*>(out)[tk] = make_uint4(p[0], p[1], p[2], p[3]);
@@ -457,6 +588,13 @@ int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const TcArgs& a, i
 template <int T>
 int launch_w16(const void* W, const void* const* B_ptrs, const int32_t* offs, __half* out, int E, int N,
                int K, cudaStream_t s) {
+    if constexpr (W8<T>::kHas) {
+        const long long values = static_cast<long long>(N) * K;
+        dim3 grid8(static_cast<unsigned>((values + kW8Blocks * 256 - 1) / (kW8Blocks * 256)), E);
+        LSG_CUDA_TRY(launch_kernel(weights_to_f16_staged_kernel<T>, grid8, dim3(256), 0, s, true,
+                                   static_cast<const uint8_t*>(W), B_ptrs, offs, out, N, K));
+        return LSG_OK;
+    }
     const long long nb = static_cast<long long>(N) * (K / Fmt<T>::VALS);
     const long long chunks = nb * (Fmt<T>::VALS / 32);
     dim3 grid(static_cast<unsigned>((chunks + 255) / 256), E);
