@@ -95,49 +95,47 @@ void place_matrices(MmvqArgs& a, const int* n_rows, const int* ctas_of) {
     }
 }
 
-// Batch rows from which the tensor-core mat-vec takes a call (LSG_MMVQ_MMA_ROWS=9: never).
+// Batch rows from which the tensor-core mat-vec takes a call (LSG_MMVQ_MMA_ROWS=9: never).  Its
+// time hardly depends on the rows, that of the dp4a kernel does.  28672 x 4096 of Q4_K, us:
+// 4 rows 21.8 on dp4a and 25 here, 8 rows 40.0 and 25.2 (Q6_K 27.4 and 36, 54.3 and 36.4;
+// 4096 x 14336 of Q4_K 20.1 and 17.5, 38.4 and 18.1); five to seven rows cost dp4a what eight do.
 int mma_min_rows() {
     static const int m = [] {
         const char* e = getenv("LSG_MMVQ_MMA_ROWS");
-        return e ? atoi(e) : 2;
+        return e ? atoi(e) : 5;
     }();
     return m;
 }
 
-// How the tensor-core mat-vec cuts K: by K and the type alone.
-bool mma_cut_k(MmaCut& g, int K) {
+// How the tensor-core mat-vec cuts K: by K and the type alone.  A CTA's share has up to
+// `max_blocks` blocks; two blocks of a row group per warp, so that its part of the barrier and the
+// sum is paid for by two tiles.
+bool mma_cut_k(MmaCut& g, int K, int max_split, int max_blocks) {
     if (K % 256 != 0) return false;
     g.sb_bytes = 256 / Fmt<T>::VALS * Fmt<T>::BYTES;
     g.nsb = K / 256;
     g.ksplit = 1;
-    while (g.ksplit < 8 && g.nsb > g.ksplit * kMmaSliceBlocks) g.ksplit *= 2;
+    while (g.ksplit < max_split && g.nsb > g.ksplit * max_blocks) g.ksplit *= 2;
     g.slice = (g.nsb + g.ksplit - 1) / g.ksplit;
-    if (g.slice > kMmaSliceBlocks || (g.ksplit - 1) * g.slice >= g.nsb) return false;
-    g.wpg = g.slice > 4 ? 8 : (g.slice > 2 ? 4 : 2);   // short rows: fewer warps per row group, more groups
-    g.nc = (g.slice + g.wpg - 1) / g.wpg;
-    g.chunk = (g.slice + g.nc - 1) / g.nc;
+    if (g.slice > max_blocks || (g.ksplit - 1) * g.slice >= g.nsb) return false;
+    g.wpg = g.slice > 8 ? 8 : (g.slice > 4 ? 4 : (g.slice > 2 ? 2 : 1));
     return true;
 }
 
-// Shared memory: the deepest ring that fits (`sum_rows` rows of cluster sums).  Returns the bytes,
-// 0 when not even two stages per row group fit.
+// Shared memory: the deepest rings that fit (`sum_rows` rows of cluster sums).  Returns the bytes,
+// 0 when not even two blocks per warp fit.
 template <class D>
 int mma_place(MmaCut& g, int sum_rows) {
-    const int nsets = kMmaWarps / g.wpg;
-    g.pitch = g.chunk * g.sb_bytes + (g.sb_bytes % 16 ? 32 : 0);
-    while (g.pitch % D::kPitchMod != D::kPitchRem) g.pitch = (g.pitch + 16) & ~15;
-    g.img_bytes = g.slice * 8 * (256 + (D::kSums ? 64 : 32));
     const long long sum_bytes = static_cast<long long>(sum_rows + 15) / 16 * 16 * kMmaCols * 4;
-    const int bar_bytes = 2 * nsets * kMmaMaxRing * 8 + 16;
-    const int part_bytes = kMmaWarps * 2 * 128 * 4;
-    const long long avail = kSmemCap - g.img_bytes - part_bytes - sum_bytes - bar_bytes;
-    const long long ring = avail / (nsets * 16 * g.pitch);
-    if (avail < 0 || ring < 2) return 0;
-    g.ring = ring > kMmaMaxRing ? kMmaMaxRing : static_cast<int>(ring);
-    g.part_off = g.img_bytes + nsets * g.ring * 16 * g.pitch;
+    constexpr int part_bytes = kMmaWarps * 2 * 128 * 4;
+    g.ring_off = mma_image_bytes<D>(g.slice * 8);
+    const long long avail = kSmemCap - g.ring_off - part_bytes - sum_bytes;
+    const long long depth = avail / (kMmaWarps * 16 * D::kPitch);
+    if (avail < 0 || depth < 2) return 0;
+    g.depth = depth > kMmaMaxDepth ? kMmaMaxDepth : static_cast<int>(depth);
+    g.part_off = g.ring_off + kMmaWarps * g.depth * 16 * D::kPitch;
     g.sum_off = g.part_off + part_bytes;
-    g.bar_off = g.sum_off + static_cast<int>(sum_bytes);
-    return g.bar_off + bar_bytes;
+    return g.sum_off + static_cast<int>(sum_bytes);
 }
 
 // The tensor-core mat-vec (mmvq_mma.cuh), or kMmaNotTaken.
@@ -147,7 +145,7 @@ int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
     if constexpr (MmaDec<TT>::kHas) {
         MmaArgs g = {};
         g.v = v;
-        if (v.M > kMmaCols || v.drop_slab >= 0 || !mma_cut_k(g.c, v.K)) return kMmaNotTaken;
+        if (v.M > kMmaCols || v.drop_slab >= 0 || !mma_cut_k(g.c, v.K, 8, kMmaSliceBlocks)) return kMmaNotTaken;
         auto kernel = mmvq_mma_kernel<TT>;
         static std::atomic<int> clusters[64][4];   // resident clusters of 1, 2, 4, 8 CTAs, per device
         int dev = 0;
@@ -357,7 +355,7 @@ constexpr int kGroupedImageBudget = 64 * 1024;  // activation image of one segme
 template <int TT>
 bool grouped_mma(int K, MmaCut& c, int& smem) {
     if constexpr (MmaDec<TT>::kHas) {
-        if (mma_min_rows() > kMmaCols || !mma_cut_k(c, K) || c.ksplit > 1) return false;
+        if (mma_min_rows() > kMmaCols || !mma_cut_k(c, K, 1, kMmaGroupedBlocks)) return false;
         smem = mma_place<MmaDec<TT>>(c, 0);
         return smem > 0;
     }

@@ -1,6 +1,6 @@
-// GGUF mat-vec for 2 to 8 batch rows on the integer tensor-core instruction (mma.sync s8).
+// GGUF mat-vec for 5 to 8 batch rows on the integer tensor-core instruction (mma.sync s8).
 //
-// From two batch rows on the mat-vec of mmvq.cuh is bound by its dp4a arithmetic (eight rows of
+// With more batch rows the mat-vec of mmvq.cuh is bound by its dp4a arithmetic (eight rows of
 // Q6_K: a quarter of the copy bandwidth), so here a warp multiplies 16 weight rows by eight
 // batch rows: one mma.m16n8k32 (k16 for Q6_K, whose scales cover 16 values) replaces 32 dp4a per
 // lane, and with the magic number 1.5 * 2^23 as the initial accumulator its integer result is
@@ -15,12 +15,13 @@
 //     of the warp takes bytes 8t..8t+7 of the packed 32 bytes of rows g and g + 8 (one 8-byte
 //     load, low nibbles = one scale group, high nibbles = the next) and the activation image
 //     keeps a block of eight columns x 32 codes so that the matching operand is one 8-byte load.
-//   * A stage of the ring holds 16 rows x up to eight super-blocks, one bulk copy per row.  The
-//     rows' pitch is chosen so that the eight rows of a fragment load hit different banks; that
-//     is why the rows are copied one by one.
-//   * `wpg` warps share a row group, warp i taking super-block i of every stage; their partial
-//     16 x 8 tiles are added in warp order through shared memory.  16 / wpg groups are in work at
-//     a time, each with a ring of its own, so a warp meets every lap of the ring it waits on.
+//   * Every warp streams the blocks it multiplies itself: cp.async of 16-byte pieces into a ring of
+//     its own, two to four 16-row blocks deep, so nothing is synchronised between warps on the way
+//     in.  The rows' pitch is chosen so that the eight rows of a fragment load hit different banks.
+//     (One bulk copy per row and stage, as first written, took the copy engine 80 to 110 cycles
+//     each: 66 MB of Q4_K in 20 us with the arithmetic left out.)
+//   * `wpg` warps share a row group, warp i taking blocks i, i + wpg, ..; their partial 16 x 8
+//     tiles are added in warp order through shared memory.  16 / wpg groups are in work at a time.
 //   * Long rows are split along K over the CTAs of a cluster (4096 values each): a CTA then
 //     quantizes and holds only its part of the activations, and the cluster has more rows.
 //     The CTAs add their sums in rank order through distributed shared memory.
@@ -32,22 +33,21 @@
 
 namespace lsg {
 
-constexpr int kMmaWarps = 16;                         // consumer warps
-constexpr int kMmaThreads = (kMmaWarps + 1) * 32;
+constexpr int kMmaWarps = 16;
+constexpr int kMmaThreads = kMmaWarps * 32;
 constexpr int kMmaCols = 8;                           // batch rows of one launch
-constexpr int kMmaSliceBlocks = 16;                   // super-blocks of one CTA's share of K, at most
-constexpr int kMmaMaxRing = 8;                        // stages of one row group's ring
+constexpr int kMmaSliceBlocks = 16;                   // 256-value blocks of one CTA's share of K, at most
+constexpr int kMmaGroupedBlocks = 16;                 // .. of a row in a grouped call, which has no clusters
+constexpr int kMmaMaxDepth = 4;
 
 // How a row is cut and where things lie in shared memory.
 struct MmaCut {
     int sb_bytes;        // bytes of 256 packed values
     int nsb;             // 256-value blocks of a row
     int ksplit, slice;   // CTAs of a cluster along K, blocks of each
-    int nc, chunk;       // stages per row group, blocks of a stage
     int wpg;             // warps of a row group
-    int ring;            // stages of a row group's ring
-    int pitch;           // bytes between the rows of a stage
-    int img_bytes, part_off, sum_off, bar_off;   // image, ring, partial tiles, cluster sums, barriers
+    int depth;           // 16-row blocks of a warp's ring
+    int ring_off, part_off, sum_off;   // image (at 0), rings, partial tiles, cluster sums
 };
 
 struct MmaArgs {
@@ -66,30 +66,32 @@ template <int T> struct MmaDec { static constexpr bool kHas = false; };
 
 #if defined(__CUDACC__)
 
-__device__ __forceinline__ void mma_u8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                             uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// d = a * b + c; a start of its own, and not the result's registers, so that none is copied.
+__device__ __forceinline__ void mma_u8s8_k32(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                             uint32_t b0, uint32_t b1, int c) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
 }
-__device__ __forceinline__ void mma_s8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                             uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma_s8s8_k32(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                             uint32_t b0, uint32_t b1, int c) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
 }
-__device__ __forceinline__ void mma_s8s8_k16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-        : "r"(a0), "r"(a1), "r"(b0));
+__device__ __forceinline__ void mma_u8s8_k16(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0, const uint4& c) {
+    asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(b0), "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w));
 }
 
 // An integer of magnitude below 2^22 added to this bit pattern is that integer as a float, offset
 // by kMmaBias; the largest sum here is 32 * 128 * 127.
 constexpr int kMmaBiasBits = 0x4B400000;
 constexpr float kMmaBias = 12582912.0f;
-__device__ __forceinline__ void mma_zero(int (&c)[4]) { c[0] = c[1] = c[2] = c[3] = kMmaBiasBits; }
-__device__ __forceinline__ float mma_val(int c) { return __int_as_float(c) - kMmaBias; }
+// (c - bias) * s with ns = -bias * s: the product of a sum below 2^22 and a scale below 2^8 in
+// magnitude is an integer of at most 24 bits here, so the one rounding of the fma is exact.
+__device__ __forceinline__ float mma_scaled(int c, float s, float ns) { return fmaf(__int_as_float(c), s, ns); }
 // Byte k of w as a float (unsigned; or signed after its sign bit has been flipped).
 __device__ __forceinline__ float byte_f(uint32_t w, int k) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7550u | k)) - 8388608.0f;
@@ -97,24 +99,31 @@ __device__ __forceinline__ float byte_f(uint32_t w, int k) {
 __device__ __forceinline__ float sbyte_f(uint32_t w_flipped, int k) {
     return __uint_as_float(__byte_perm(w_flipped, 0x4B000000u, 0x7550u | k)) - 8388736.0f;
 }
-__device__ __forceinline__ uint32_t lds_word_unaligned(uint32_t addr) {
-    const uint32_t b = addr & ~3u;
-    return __funnelshift_r(lds32(b), lds32(b + 4), (addr & 3u) * 8u);
-}
+// Unaligned words at constant distances (multiples of 4) from one address: the alignment is worked
+// out once.
+struct MmaWords {
+    uint32_t base, sh;
+    __device__ __forceinline__ explicit MmaWords(uint32_t addr) : base(addr & ~3u), sh((addr & 3u) * 8u) {}
+    __device__ __forceinline__ uint32_t at(int off) const { return __funnelshift_r(lds32(base + off), lds32(base + off + 4), sh); }
+};
 
 // tile(): acc[i] += the products of one 256-value block: rows r0 (accumulators 0, 1) and r1 (2, 3)
 // with columns 2t and 2t + 1.
 //   r0, r1  shared addresses of the block in rows g and g + 8
 //   xq      codes of this lane's column g: block j of the 256 values at xq + 256 j, lane offset in
-//   xs      scales (with the block sum where kSums) of columns 2t, 2t + 1: block j at xs + j * 64 or 32
+//   xs      scales of columns 2t, 2t + 1 (and what kKind says): block j at xs + j * kScaleBytes
 // kHalves: the words of a block's two 16-value halves alternate in the image.
+// kKind: 0 scales {d}; 1 {d, d * sum of the codes}; 2 {d} and, behind the scales of all blocks, the
+// accumulator starts of the block's two halves, bias - 32 * sum of the half's codes, for columns
+// 2t, 2t + 1 twice over (Q6_K: the offset of its codes is in the sums before they are scaled).
 template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
     static constexpr bool kHas = true;
-    static constexpr bool kSums = true, kHalves = false;
+    static constexpr int kKind = 1, kScaleBytes = 64;
+    static constexpr bool kHalves = false;
     static constexpr int kBytes = FIVE ? 176 : 144;
-    static constexpr int kPitchMod = 64, kPitchRem = 32;   // 8-byte loads of eight rows: no bank twice
+    static constexpr int kPitch = FIVE ? 176 : 160;   // 8-byte loads of four rows: no bank twice with 160 (224 would not fit)
 
-    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs,
+    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
                                                 float (&acc)[4]) {
         constexpr int QS = FIVE ? 48 : 16;
         const uint4 h0 = lds128(r0), h1 = lds128(r1);
@@ -146,14 +155,14 @@ template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
                 const float dx0 = __uint_as_float(xv.x), sx0 = __uint_as_float(xv.y);
                 const float dx1 = __uint_as_float(xv.z), sx1 = __uint_as_float(xv.w);
                 int c[4];
-                mma_zero(c);
-                mma_u8s8_k32(c, a0, a1, a2, a3, xb.x, xb.y);
+                mma_u8s8_k32(c, a0, a1, a2, a3, xb.x, xb.y, kMmaBiasBits);
                 const float c0 = byte_f(sc0[j >> 2], j & 3), c1 = byte_f(sc1[j >> 2], j & 3);
                 const float m0 = byte_f(mn0[j >> 2], j & 3), m1 = byte_f(mn1[j >> 2], j & 3);
-                s1[0] = fmaf(dx0, mma_val(c[0]) * c0, s1[0]);   // integer products below 2^24: exact
-                s1[1] = fmaf(dx1, mma_val(c[1]) * c0, s1[1]);
-                s1[2] = fmaf(dx0, mma_val(c[2]) * c1, s1[2]);
-                s1[3] = fmaf(dx1, mma_val(c[3]) * c1, s1[3]);
+                const float n0 = -kMmaBias * c0, n1 = -kMmaBias * c1;
+                s1[0] = fmaf(dx0, mma_scaled(c[0], c0, n0), s1[0]);
+                s1[1] = fmaf(dx1, mma_scaled(c[1], c0, n0), s1[1]);
+                s1[2] = fmaf(dx0, mma_scaled(c[2], c1, n1), s1[2]);
+                s1[3] = fmaf(dx1, mma_scaled(c[3], c1, n1), s1[3]);
                 s2[0] = fmaf(m0, sx0, s2[0]);
                 s2[1] = fmaf(m0, sx1, s2[1]);
                 s2[2] = fmaf(m1, sx0, s2[2]);
@@ -173,25 +182,20 @@ template <> struct MmaDec<LSG_GGUF_Q5_K> : MmaDecK45<true> {};
 
 template <> struct MmaDec<LSG_GGUF_Q6_K> {
     static constexpr bool kHas = true;
-    static constexpr bool kSums = false, kHalves = true;
+    static constexpr int kKind = 2, kScaleBytes = 32;
+    static constexpr bool kHalves = true;
     static constexpr int kBytes = 210;
-    static constexpr int kPitchMod = 32, kPitchRem = 16;   // 4-byte loads of eight rows
+    static constexpr int kPitch = 240;   // 4-byte loads of eight rows: no bank twice
 
-    // four 6-bit values 0..63 -> value - 32 as signed bytes
-    __device__ static __forceinline__ uint32_t sext6(uint32_t v) {
-        const uint32_t x = v ^ 0x20202020u;
-        return x | ((x & 0x20202020u) * 6u);
-    }
-    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs,
+    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t xi,
                                                 float (&acc)[4]) {
-        const uint32_t row[2] = {r0, r1};
+        const MmaWords w[2] = {MmaWords(r0), MmaWords(r1)};
         uint32_t scw[2][4];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            lds_words_unaligned<4>(row[r] + 192, scw[r]);
+        for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) scw[r][i] ^= 0x80808080u;
-        }
+            for (int i = 0; i < 4; ++i) scw[r][i] = w[r].at(192 + 4 * i) ^ 0x80808080u;
+        const MmaWords v[2] = {MmaWords(r0 + 4 * t), MmaWords(r1 + 4 * t)};
         float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int ip = 0; ip < 2; ++ip) {
@@ -200,15 +204,16 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
             for (int r = 0; r < 2; ++r)
 #pragma unroll
                 for (int hs = 0; hs < 2; ++hs) {
-                    la[r][hs] = lds_word_unaligned(row[r] + 64 * ip + 16 * hs + 4 * t);
-                    lb[r][hs] = lds_word_unaligned(row[r] + 64 * ip + 32 + 16 * hs + 4 * t);
-                    qh[r][hs] = lds_word_unaligned(row[r] + 128 + 32 * ip + 16 * hs + 4 * t);
+                    la[r][hs] = v[r].at(64 * ip + 16 * hs);
+                    lb[r][hs] = v[r].at(64 * ip + 32 + 16 * hs);
+                    qh[r][hs] = v[r].at(128 + 32 * ip + 16 * hs);
                 }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const uint2 xb = lds64(xq + 256 * (4 * ip + q));
-                const uint2 xv = lds64(xs + 32 * (4 * ip + q));
-                float f[2][4];
+                const int j = 4 * ip + q;
+                const uint2 xb = lds64(xq + 256 * j);
+                const uint2 xv = lds64(xs + 32 * j);
+                int c[2][4];
 #pragma unroll
                 for (int hs = 0; hs < 2; ++hs) {
                     uint32_t a[2];
@@ -216,13 +221,9 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
                     for (int r = 0; r < 2; ++r) {
                         const uint32_t lo = ((q & 1) ? lb[r][hs] : la[r][hs]) >> (4 * (q >> 1));
                         const uint32_t hi = q == 0 ? qh[r][hs] << 4 : (q == 1 ? qh[r][hs] << 2 : (q == 2 ? qh[r][hs] : qh[r][hs] >> 2));
-                        a[r] = sext6((lo & 0x0F0F0F0Fu) | (hi & 0x30303030u));
+                        a[r] = (lo & 0x0F0F0F0Fu) | (hi & 0x30303030u);
                     }
-                    int c[4];
-                    mma_zero(c);
-                    mma_s8s8_k16(c, a[0], a[1], hs ? xb.y : xb.x);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) f[hs][i] = mma_val(c[i]);
+                    mma_u8s8_k16(c[hs], a[0], a[1], hs ? xb.y : xb.x, lds128(xi + 128 * j + 64 * hs));
                 }
                 const int e = 8 * ip + 2 * q;
                 const float dx0 = __uint_as_float(xv.x), dx1 = __uint_as_float(xv.y);
@@ -230,8 +231,9 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const float sa = sbyte_f(scw[r][e >> 2], e & 3), sb = sbyte_f(scw[r][(e + 1) >> 2], (e + 1) & 3);
-                    s[2 * r] = fmaf(dx0, fmaf(f[1][2 * r], sb, f[0][2 * r] * sa), s[2 * r]);
-                    s[2 * r + 1] = fmaf(dx1, fmaf(f[1][2 * r + 1], sb, f[0][2 * r + 1] * sa), s[2 * r + 1]);
+                    const float na = -kMmaBias * sa, nb = -kMmaBias * sb;
+                    s[2 * r] = fmaf(dx0, mma_scaled(c[0][2 * r], sa, na) + mma_scaled(c[1][2 * r], sb, nb), s[2 * r]);
+                    s[2 * r + 1] = fmaf(dx1, mma_scaled(c[0][2 * r + 1], sa, na) + mma_scaled(c[1][2 * r + 1], sb, nb), s[2 * r + 1]);
                 }
             }
         }
@@ -245,68 +247,82 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
 
 template <> struct MmaDec<LSG_GGUF_Q8_0> {   // eight 34-byte blocks
     static constexpr bool kHas = true;
-    static constexpr bool kSums = false, kHalves = false;
+    static constexpr int kKind = 0, kScaleBytes = 32;
+    static constexpr bool kHalves = false;
     static constexpr int kBytes = 272;
-    static constexpr int kPitchMod = 64, kPitchRem = 32;
+    static constexpr int kPitch = 272;
 
-    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs,
+    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
                                                 float (&acc)[4]) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            uint32_t w0[2], w1[2];
-            lds_words_unaligned<2>(r0 + 34 * j + 2 + 8 * t, w0);
-            lds_words_unaligned<2>(r1 + 34 * j + 2 + 8 * t, w1);
+            // rows start on 16-byte boundaries: every second block's codes are a half word off
+            const uint32_t p0 = r0 + 8 * t + ((34 * j + 2) & ~3), p1 = r1 + 8 * t + ((34 * j + 2) & ~3);
+            uint32_t w0[3], w1[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                w0[i] = (i < 2 || j % 2 == 0) ? lds32(p0 + 4 * i) : 0u;
+                w1[i] = (i < 2 || j % 2 == 0) ? lds32(p1 + 4 * i) : 0u;
+            }
+            if (j % 2 == 0) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    w0[i] = __byte_perm(w0[i], w0[i + 1], 0x5432);
+                    w1[i] = __byte_perm(w1[i], w1[i + 1], 0x5432);
+                }
+            }
             const uint2 xb = lds64(xq + 256 * j);
             const uint2 xv = lds64(xs + 32 * j);
             int c[4];
-            mma_zero(c);
-            mma_s8s8_k32(c, w0[0], w1[0], w0[1], w1[1], xb.x, xb.y);
+            mma_s8s8_k32(c, w0[0], w1[0], w0[1], w1[1], xb.x, xb.y, kMmaBiasBits);
             const float d0 = fp16_bits_to_float(lds16(r0 + 34 * j)), d1 = fp16_bits_to_float(lds16(r1 + 34 * j));
             const float dx0 = __uint_as_float(xv.x), dx1 = __uint_as_float(xv.y);
-            acc[0] = fmaf(d0 * dx0, mma_val(c[0]), acc[0]);
-            acc[1] = fmaf(d0 * dx1, mma_val(c[1]), acc[1]);
-            acc[2] = fmaf(d1 * dx0, mma_val(c[2]), acc[2]);
-            acc[3] = fmaf(d1 * dx1, mma_val(c[3]), acc[3]);
+            acc[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, acc[0]);
+            acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
+            acc[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, acc[2]);
+            acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
         }
     }
 };
 
 template <> struct MmaDec<LSG_GGUF_Q4_0> {   // eight 18-byte blocks; byte i: values i and i + 16
     static constexpr bool kHas = true;
-    static constexpr bool kSums = false, kHalves = true;
+    static constexpr int kKind = 0, kScaleBytes = 32;
+    static constexpr bool kHalves = true;
     static constexpr int kBytes = 144;
-    static constexpr int kPitchMod = 32, kPitchRem = 16;
+    static constexpr int kPitch = 144;
 
     // four nibbles 0..15 -> value - 8 as signed bytes
     __device__ static __forceinline__ uint32_t sext4(uint32_t v) {
         const uint32_t x = v ^ 0x08080808u;
         return x | ((x & 0x08080808u) * 30u);
     }
-    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs,
+    __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
                                                 float (&acc)[4]) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const uint32_t w0 = lds_word_unaligned(r0 + 18 * j + 2 + 4 * t);
-            const uint32_t w1 = lds_word_unaligned(r1 + 18 * j + 2 + 4 * t);
+            // rows start on 16-byte boundaries: every second block's codes are a half word off
+            const uint32_t p0 = r0 + 4 * t + ((18 * j + 2) & ~3), p1 = r1 + 4 * t + ((18 * j + 2) & ~3);
+            const uint32_t w0 = j % 2 ? lds32(p0) : __byte_perm(lds32(p0), lds32(p0 + 4), 0x5432);
+            const uint32_t w1 = j % 2 ? lds32(p1) : __byte_perm(lds32(p1), lds32(p1 + 4), 0x5432);
             const uint2 xb = lds64(xq + 256 * j);
             const uint2 xv = lds64(xs + 32 * j);
             int c[4];
-            mma_zero(c);
             mma_s8s8_k32(c, sext4(w0 & 0x0F0F0F0Fu), sext4(w1 & 0x0F0F0F0Fu), sext4((w0 >> 4) & 0x0F0F0F0Fu),
-                         sext4((w1 >> 4) & 0x0F0F0F0Fu), xb.x, xb.y);
+                         sext4((w1 >> 4) & 0x0F0F0F0Fu), xb.x, xb.y, kMmaBiasBits);
             const float d0 = fp16_bits_to_float(lds16(r0 + 18 * j)), d1 = fp16_bits_to_float(lds16(r1 + 18 * j));
             const float dx0 = __uint_as_float(xv.x), dx1 = __uint_as_float(xv.y);
-            acc[0] = fmaf(d0 * dx0, mma_val(c[0]), acc[0]);
-            acc[1] = fmaf(d0 * dx1, mma_val(c[1]), acc[1]);
-            acc[2] = fmaf(d1 * dx0, mma_val(c[2]), acc[2]);
-            acc[3] = fmaf(d1 * dx1, mma_val(c[3]), acc[3]);
+            acc[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, acc[0]);
+            acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
+            acc[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, acc[2]);
+            acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
         }
     }
 };
 
 // ---------------------------------------------------------------------------
 // Activation image of `nblk` 32-value blocks from block b0 on, eight columns (batch rows from M
-// on are zeros):  codes [block][column][32], then scales [block][column]{d} or {d, d * sum}.
+// on are zeros): codes [block][column][32], then the scales and accumulator starts of D::kKind.
 // ---------------------------------------------------------------------------
 template <class D>
 __device__ __forceinline__ void mma_put_half(uint8_t* img, int b, int col, int half, const uint4& q) {
@@ -321,13 +337,21 @@ __device__ __forceinline__ void mma_put_half(uint8_t* img, int b, int col, int h
         *reinterpret_cast<uint4*>(at + 16 * half) = q;
     }
 }
+template <class D> __host__ __device__ constexpr int mma_image_bytes(int nblk) {
+    return nblk * (256 + D::kScaleBytes + (D::kKind == 2 ? 128 : 0));
+}
+// sum: of the 32 codes; with kKind 2 of the 16 of half `half` (called once per half then)
 template <class D>
-__device__ __forceinline__ void mma_put_scale(uint8_t* img, int nblk, int b, int col, float d, int sum) {
+__device__ __forceinline__ void mma_put_scale(uint8_t* img, int nblk, int b, int col, int half, float d, int sum) {
     float* s = reinterpret_cast<float*>(img + nblk * 256);
-    if (D::kSums) {
+    if (D::kKind == 1) {
         *reinterpret_cast<float2*>(s + (b * 8 + col) * 2) = make_float2(d, d * static_cast<float>(sum));
     } else {
-        s[b * 8 + col] = d;
+        if (half == 0) s[b * 8 + col] = d;
+        if (D::kKind == 2) {
+            int* start = reinterpret_cast<int*>(img + nblk * (256 + D::kScaleBytes)) + (b * 2 + half) * 16 + (col >> 1) * 4 + (col & 1);
+            start[0] = start[2] = kMmaBiasBits - 32 * sum;
+        }
     }
 }
 
@@ -342,12 +366,18 @@ __device__ __forceinline__ void mma_image_q8_1(uint8_t* img, const uint8_t* __re
 #pragma unroll
             for (int i = 0; i < 9; ++i) w[i] = __ldg(src + i);
         }
-        int sum = 0;
+        int sum[2] = {0, 0};
 #pragma unroll
-        for (int i = 1; i < 9; ++i) sum = __dp4a(static_cast<int>(w[i]), 0x01010101, sum);
+        for (int i = 1; i < 9; ++i) sum[(i - 1) >> 2] = __dp4a(static_cast<int>(w[i]), 0x01010101, sum[(i - 1) >> 2]);
         mma_put_half<D>(img, b, m, 0, make_uint4(w[1], w[2], w[3], w[4]));
         mma_put_half<D>(img, b, m, 1, make_uint4(w[5], w[6], w[7], w[8]));
-        mma_put_scale<D>(img, nblk, b, m, fp16_bits_to_float(w[0]), sum);
+        const float d = fp16_bits_to_float(w[0]);
+        if (D::kKind == 2) {
+            mma_put_scale<D>(img, nblk, b, m, 0, d, sum[0]);
+            mma_put_scale<D>(img, nblk, b, m, 1, d, sum[1]);
+        } else {
+            mma_put_scale<D>(img, nblk, b, m, 0, d, sum[0] + sum[1]);
+        }
     }
 }
 
@@ -355,16 +385,21 @@ __device__ __forceinline__ void mma_image_q8_1(uint8_t* img, const uint8_t* __re
 template <class D>
 __device__ __forceinline__ void mma_image_bf16(uint8_t* img, const __nv_bfloat16* __restrict__ A, int M, int K, int b0,
                                                int nblk, int tid, int nthreads) {
-    const int total = kMmaCols * nblk * 2;   // a multiple of 32, as nthreads: no warp is split by the loop
-    for (int idx = tid; idx < total; idx += nthreads) {
+    // columns without a batch row: zeros (the quantizer would take its slow path for a scale of 0)
+    for (int idx = tid; idx < (kMmaCols - M) * nblk * 2; idx += nthreads) {
+        const int half = idx & 1, task = idx >> 1;
+        const int c = task / nblk, b = task - c * nblk;
+        mma_put_half<D>(img, b, M + c, half, make_uint4(0, 0, 0, 0));
+        if (D::kKind == 2 || half == 0) mma_put_scale<D>(img, nblk, b, M + c, half, 0.0f, 0);
+    }
+    const int total = M * nblk * 2;
+    for (int base = tid & ~31; base < total; base += nthreads) {   // whole warps: the two lanes of a block exchange values
+        const int idx = min(base + (tid & 31), total - 1);
+        const bool live = base + (tid & 31) < total;
         const int half = idx & 1, task = idx >> 1;
         const int m = task / nblk, b = task - m * nblk;
-        uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
-        if (m < M) {
-            const uint4* src = reinterpret_cast<const uint4*>(A + static_cast<size_t>(m) * K + static_cast<size_t>(b0 + b) * 32 + 16 * half);
-            r0 = __ldg(src);
-            r1 = __ldg(src + 1);
-        }
+        const uint4* src = reinterpret_cast<const uint4*>(A + static_cast<size_t>(m) * K + static_cast<size_t>(b0 + b) * 32 + 16 * half);
+        const uint4 r0 = __ldg(src), r1 = __ldg(src + 1);
         const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
         float x[16];
 #pragma unroll
@@ -385,9 +420,11 @@ __device__ __forceinline__ void mma_image_bf16(uint8_t* img, const __nv_bfloat16
                   __dp4a(static_cast<int>(q.y), 0x01010101,
                   __dp4a(static_cast<int>(q.z), 0x01010101,
                   __dp4a(static_cast<int>(q.w), 0x01010101, 0))));
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        mma_put_half<D>(img, b, m, half, q);
-        if (half == 0) mma_put_scale<D>(img, nblk, b, m, __half2float(__float2half(d)), sum);
+        if (D::kKind != 2) sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        if (live) {
+            mma_put_half<D>(img, b, m, half, q);
+            if (D::kKind == 2 || half == 0) mma_put_scale<D>(img, nblk, b, m, half, __half2float(__float2half(d)), sum);
+        }
     }
 }
 
@@ -403,66 +440,135 @@ __device__ __forceinline__ float mma_ld_cluster(uint32_t local_addr, uint32_t ra
     return v;
 }
 
-// One stage: `nrows` rows of `bytes` packed bytes each, row r at src + r * row_bytes, into the
-// stage at `pitch`.  `shifted`: a row keeps its offset from a 16-byte boundary (the types whose
-// blocks are not whole 16-byte pieces).  Bulk copies take whole 16-byte pieces; what a row holds
-// behind the last whole piece of the matrix (w_end_al), and all of it when the matrix itself is
-// not 16-byte aligned (w_end_al = 0), is moved with byte loads.  Called by a converged warp.
-__device__ __forceinline__ void mma_copy_stage(uint8_t* dst, uintptr_t src, int nrows, long long row_bytes, int bytes,
-                                               int pitch, uintptr_t w_end_al, bool shifted, uint64_t* bar, uint64_t policy) {
-    const int lane = threadIdx.x & 31;
-    const uintptr_t my_b = src + static_cast<uintptr_t>(lane < nrows ? lane : 0) * row_bytes, my_e = my_b + bytes;
-    const uintptr_t at_b = shifted ? my_b & ~uintptr_t(15) : my_b;   // what the row's place in the stage stands for
-    uintptr_t cp_e = (my_e + 15) & ~uintptr_t(15);
-    if (cp_e > w_end_al) cp_e = w_end_al > at_b ? w_end_al : at_b;
-    const uint32_t mine = lane < nrows ? static_cast<uint32_t>(cp_e - at_b) : 0u;
-    const uint32_t all = __reduce_add_sync(0xffffffffu, mine);
-    if (lane < nrows)
-        for (uintptr_t p = mine > 0 ? cp_e : my_b; p < my_e; ++p)
-            dst[lane * pitch + (p - at_b)] = *reinterpret_cast<const uint8_t*>(p);
-    __syncwarp();
-    if (elect_one_lane()) mbar_arrive_expect_tx(bar, all);
-    __syncwarp();
-    if (mine > 0) bulk_g2s_hint(dst + lane * pitch, reinterpret_cast<const void*>(at_b), mine, bar, policy);
-    __syncwarp();
-}
-
-// One warp's part of a row group: block `wi` of each of its stages, the partial tile left in
-// mine[16 rows][8 columns].  lo0: low bits of the address of the group's first row, at this CTA's
-// first block.  s, phase: the warp's position in its set's ring.
+// A warp's weight stream: 16-row blocks through its ring.  A block's rows are copied as 16-byte
+// pieces; where blocks are not whole pieces (kShifted), those that meet the row, which keeps its
+// offset from a 16-byte boundary.  The bytes behind the last whole piece of a matrix, and all of a
+// matrix that is not 16-byte aligned (w_end = 0), are moved one by one.
 template <class D>
-__device__ __forceinline__ void mma_row_group(const MmaCut& g, int lane, int wi, uint32_t lo0, uint32_t row_bytes, int nsb,
-                                              uint32_t xq0, uint32_t xs0, uint32_t ring0, uint64_t* full, uint64_t* empty,
-                                              int& s, uint32_t& phase, volatile int* abort_flag, unsigned int* status,
-                                              long long wait_limit, float* mine) {
-    constexpr int kScaleBytes = D::kSums ? 64 : 32;
-    const int gl = lane >> 2, t = lane & 3;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int c = 0; c < g.nc; ++c) {
-        // After a wait has run out the warps keep walking (the barriers of their set need every
-        // warp) but neither wait nor compute.
-        bool ok = *abort_flag == 0;
-        ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(&full[s], phase, status, kDevWaitFull, 2000u, wait_limit));
-        if (!ok) *abort_flag = 1;
-        const int sb = c * g.chunk + wi;
-        if (ok && wi < g.chunk && sb < nsb) {
-            uint32_t p0 = ring0 + static_cast<uint32_t>(s * 16 + gl) * g.pitch + wi * D::kBytes, p1 = p0 + 8 * g.pitch;
-            if (D::kBytes % 16 != 0) {   // rows may start off a 16-byte boundary
-                const uint32_t lo = lo0 + static_cast<uint32_t>(gl) * row_bytes + static_cast<uint32_t>(c * g.chunk) * D::kBytes;
-                p0 += lo & 15u;
-                p1 += (lo + 8u * row_bytes) & 15u;
+struct MmaStream {
+    static constexpr bool kShifted = D::kBytes % 16 != 0;
+    static constexpr int kPieces = kShifted ? (D::kBytes + 15 + 15) / 16 : D::kBytes / 16;
+    // kShifted: sixteen lanes per row, two rows per issue; otherwise the pieces of all rows in turn
+    static constexpr int kIssues = kShifted ? 8 : (16 * kPieces + 31) / 32;
+    static_assert(kPieces <= 16 || !kShifted, "sixteen lanes cover a row");
+    static_assert(kPieces * 16 <= D::kPitch, "a row's pieces fit its pitch");
+    uint32_t goff[kShifted ? 1 : kIssues], soff[kShifted ? 1 : kIssues];   // this lane's pieces, from the block's first row
+    uint32_t row_bytes;
+    int lane;
+
+    __device__ __forceinline__ MmaStream(uint32_t rb, int l) : row_bytes(rb), lane(l) {
+        if (kShifted) {
+            goff[0] = static_cast<uint32_t>(lane >> 4) * rb;
+            soff[0] = static_cast<uint32_t>((lane >> 4) * D::kPitch + 16 * (lane & 15));
+        } else {
+#pragma unroll
+            for (int i = 0; i < kIssues; ++i) {
+                const int p = lane + 32 * i, row = p / kPieces, k = p - row * kPieces;
+                goff[i] = static_cast<uint32_t>(row) * rb + 16 * k;
+                soff[i] = static_cast<uint32_t>(row * D::kPitch + 16 * k);
             }
-            D::tile(p0, p1, t, xq0 + sb * 2048, xs0 + sb * 8 * kScaleBytes, acc);
-        }
-        __syncwarp();
-        if (elect_one_lane()) mbar_arrive(&empty[s]);
-        if (++s == g.ring) {
-            s = 0;
-            phase ^= 1;
         }
     }
+    __device__ static __forceinline__ void copy16(uint32_t dst, uintptr_t src, uint64_t policy) {
+        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+    }
+    // src: first row of the group at the block, of which nrows rows are left
+    __device__ __forceinline__ void issue(uint32_t slot, uintptr_t src, int nrows, uintptr_t w_end, uint64_t policy) const {
+        nrows = min(nrows, 16);
+        const uintptr_t last = src + static_cast<uintptr_t>(static_cast<uint32_t>(nrows - 1) * row_bytes) + D::kBytes;
+        if (((last + 15) & ~uintptr_t(15)) <= w_end) {
+            if (kShifted) {
+                const uint32_t k16 = 16 * (lane & 15);
+                uintptr_t b = src + goff[0];
+                uint32_t dst = slot + soff[0];
+#pragma unroll
+                for (int i = 0; i < kIssues; ++i) {
+                    const uint32_t off = static_cast<uint32_t>(b) & 15u;
+                    if (2 * i + (lane >> 4) < nrows && k16 < off + D::kBytes) copy16(dst, b - off + k16, policy);
+                    b += 2 * row_bytes;
+                    dst += 2 * D::kPitch;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < kIssues; ++i)
+                    if (lane + 32 * i < nrows * kPieces) copy16(slot + soff[i], src + goff[i], policy);
+            }
+            return;
+        }
+        for (int p = lane; p < nrows * kPieces; p += 32) {
+            const int row = p / kPieces, k = p - row * kPieces;
+            const uintptr_t b = src + static_cast<uintptr_t>(static_cast<uint32_t>(row) * row_bytes);
+            const uintptr_t at = (kShifted ? b & ~uintptr_t(15) : b) + 16 * k;
+            const uint32_t dst = slot + static_cast<uint32_t>(row * D::kPitch + 16 * k);
+            if (at + 16 <= w_end) {
+                copy16(dst, at, policy);
+            } else {
+                for (uintptr_t q = at < b ? b : at; q < at + 16 && q < b + D::kBytes; ++q)
+                    asm volatile("st.shared.u8 [%0], %1;" ::"r"(dst + static_cast<uint32_t>(q - at)),
+                                 "r"(static_cast<uint32_t>(*reinterpret_cast<const uint8_t*>(q)))
+                                 : "memory");
+            }
+        }
+    }
+};
+
+// Waits until all but the youngest depth - 1 blocks of this thread's copies have landed.
+__device__ __forceinline__ void mma_wait_block(int depth) {
+    if (depth == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+    else if (depth == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else asm volatile("cp.async.wait_group 1;" ::: "memory");
+}
+
+// What a warp needs of the image and its ring.
+template <class D>
+struct MmaWarp {
+    uint32_t xq, xs, xi, ring;
+    int lane, wi, set, depth;
+    __device__ __forceinline__ MmaWarp(const MmaCut& g, uint8_t* smem, int nblk) {
+        lane = threadIdx.x & 31;
+        const int warp = threadIdx.x >> 5;
+        set = warp / g.wpg;
+        wi = warp - set * g.wpg;
+        depth = g.depth;
+        const uint32_t img = smem_u32(smem);
+        xq = img + (lane >> 2) * 32 + 8 * (lane & 3);
+        xs = img + nblk * 256 + (lane & 3) * (D::kScaleBytes / 4);
+        xi = img + nblk * (256 + D::kScaleBytes) + (lane & 3) * 16;
+        ring = img + g.ring_off + static_cast<uint32_t>(warp * depth * 16 * D::kPitch);
+    }
+    __device__ __forceinline__ uint32_t slot(int i) const { return ring + static_cast<uint32_t>(i * 16 * D::kPitch); }
+    // The block in slot i times the columns; lo: low bits of the address of its first row.
+    __device__ __forceinline__ void multiply(int i, int sb, uint32_t lo, uint32_t row_bytes, float (&acc)[4]) const {
+        const int gl = lane >> 2;
+        uint32_t p0 = slot(i) + static_cast<uint32_t>(gl * D::kPitch), p1 = p0 + 8 * D::kPitch;
+        if (MmaStream<D>::kShifted) {
+            const uint32_t a = lo + static_cast<uint32_t>(gl) * row_bytes;
+            p0 += a & 15u;
+            p1 += (a + 8u * row_bytes) & 15u;
+        }
+        D::tile(p0, p1, lane & 3, xq + sb * 2048, xs + sb * 8 * D::kScaleBytes, xi + sb * 1024, acc);
+    }
+};
+
+// The partial tiles of a row group's warps, added in warp order.  sink(row, column, value) takes
+// each of the 16 x 8 sums once.  Tiles alternate between two buffers: the one being read is not
+// written before every warp of the group has passed the next barrier.
+template <class Sink>
+__device__ __forceinline__ void mma_add_tiles(const MmaCut& g, float* part, int set, int buf, int wi, int lane, const float (&acc)[4],
+                                              Sink sink) {
+    float* all = part + (set * 2 + buf) * g.wpg * 128;
+    float* mine = all + wi * 128;
+    const int gl = lane >> 2, t = lane & 3;
     *reinterpret_cast<float2*>(mine + gl * 8 + 2 * t) = make_float2(acc[0], acc[1]);
     *reinterpret_cast<float2*>(mine + (gl + 8) * 8 + 2 * t) = make_float2(acc[2], acc[3]);
+    if (g.wpg == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(2 + set), "r"(g.wpg * 32) : "memory");
+    for (int i = wi * 32 + lane; i < 128; i += g.wpg * 32) {
+        const int col = i >> 4, r = i & 15;
+        float v = all[r * 8 + col];
+        for (int w = 1; w < g.wpg; ++w) v += all[w * 128 + r * 8 + col];
+        sink(r, col, v);
+    }
 }
 
 template <int T>
@@ -471,15 +577,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
     const MmvqArgs& a = args.v;
     const MmaCut& g = args.c;
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* ring = smem + g.img_bytes;
     float* part = reinterpret_cast<float*>(smem + g.part_off);     // [set][2][wpg][16 rows][8]
     float* sums = reinterpret_cast<float*>(smem + g.sum_off);      // [row][8], with ksplit > 1
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + g.bar_off);
-    const int nsets = kMmaWarps / g.wpg;
-    uint64_t* empty = full + nsets * g.ring;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + nsets * g.ring);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int rank = static_cast<int>(blockIdx.x) % g.ksplit;
     int bx = static_cast<int>(blockIdx.x) / g.ksplit;
     const uint8_t* Wm = a.W;
@@ -509,97 +610,60 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
     const int groups = (row_end - row_begin + 15) >> 4;
     const int sb0 = rank * g.slice;
     const int nsb = min(g.slice, g.nsb - sb0);   // blocks of this CTA's part of K
-    const int stage_bytes = 16 * g.pitch;
 
-    if (tid < nsets * g.ring) {
-        mbar_init(&full[tid], 1);
-        mbar_init(&empty[tid], g.wpg);
-        mbar_fence_init();
-    }
-    if (tid == 0) *abort_flag = 0;
-    __syncthreads();
+    // dep_mode 1: nothing behind this launch runs before the work in front of the batch is done
     if (a.dep_mode != 1) pdl_launch_dependents();
 
-    const uintptr_t w_base = reinterpret_cast<uintptr_t>(Wm);
-    if (warp == kMmaWarps) {
-        // ------------------------------ producer ------------------------------
-        const uint64_t policy = l2_policy_evict_first();
-        const uintptr_t w_end_al = (w_base + static_cast<uintptr_t>(Nm) * a.row_bytes) & ~uintptr_t(15);
-        bool released = a.dep_mode != 1;
-        bool ok = true;
-        int slot = 0;        // ring position, the same in every set's ring
-        uint32_t lap = 0;
-        for (int g0 = 0; g0 < groups && ok; g0 += nsets) {
-            for (int c = 0; c < g.nc && ok; ++c) {
-                const int cb = min(g.chunk, nsb - c * g.chunk);   // blocks of the stage, may be 0 or less
-                for (int h = 0; h < nsets && g0 + h < groups; ++h) {
-                    const int s = h * g.ring + slot;
-                    if (lap > 0) {
-                        // first launch of a batch whose later launches do not wait: release them once
-                        // the ring is full and the work in front of the batch has completed
-                        if (!released) {
-                            pdl_wait_prior();
-                            pdl_launch_dependents();
-                            released = true;
-                        }
-                        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], (lap - 1) & 1, a.status, kDevWaitEmpty, 2000u, a.wait_limit));
-                        if (!ok) break;
-                    }
-                    const int r0 = row_begin + (g0 + h) * 16;
-                    const int nrows = min(16, row_end - r0);
-                    if (cb > 0)
-                        mma_copy_stage(ring + static_cast<size_t>(s) * stage_bytes,
-                                       w_base + static_cast<uintptr_t>(r0) * a.row_bytes + static_cast<uintptr_t>(sb0 + c * g.chunk) * g.sb_bytes,
-                                       nrows, a.row_bytes, cb * g.sb_bytes, g.pitch, w_end_al, D::kBytes % 16 != 0, &full[s], policy);
-                    else if (elect_one_lane())
-                        mbar_arrive(&full[s]);
-                    __syncwarp();
-                }
-                if (++slot == g.ring) {
-                    slot = 0;
-                    ++lap;
-                }
-            }
-        }
-        if (!ok) *abort_flag = 1;
-        if (!released) {
-            pdl_wait_prior();
-            pdl_launch_dependents();
-        }
-    } else {
-        // ------------------------------ consumers ------------------------------
-        const int n_cons = kMmaWarps * 32;
-        if (a.dep_mode != 2) pdl_wait_prior();
-        if (a.dep_mode == 1) pdl_launch_dependents();
-        const int nblk = nsb * 8;
-        if (Am) mma_image_bf16<D>(smem, Am, a.M, a.K, sb0 * 8, nblk, tid, n_cons);
-        else mma_image_q8_1<D>(smem, xqm, a.M, a.K / 32, sb0 * 8, nblk, tid, n_cons);
-        asm volatile("bar.sync 1, %0;" ::"r"(n_cons) : "memory");
+    const MmaWarp<D> w(g, smem, nsb * 8);
+    const int nsets = kMmaWarps / g.wpg;
+    const uint32_t row_bytes = static_cast<uint32_t>(a.row_bytes);
+    const MmaStream<D> stream(row_bytes, w.lane);
+    const uintptr_t w_base = reinterpret_cast<uintptr_t>(Wm) + static_cast<uintptr_t>(sb0) * D::kBytes;
+    const uintptr_t w_end = (reinterpret_cast<uintptr_t>(Wm) + static_cast<uintptr_t>(Nm) * row_bytes) & ~uintptr_t(15);
+    const uint64_t policy = l2_policy_evict_first();
 
-        const int set = warp / g.wpg, wi = warp - set * g.wpg;
-        const int set_tid = wi * 32 + lane;
-        const uint32_t img = smem_u32(smem);
-        const uint32_t xq0 = img + (lane >> 2) * 32 + 8 * (lane & 3);
-        const uint32_t xs0 = img + nblk * 256 + (lane & 3) * (D::kSums ? 16 : 8);
-        const uint32_t ring0 = smem_u32(ring) + static_cast<uint32_t>(set * g.ring) * stage_bytes;
-        int s = 0, buf = 0;
-        uint32_t phase = 0;
-        for (int gi = set; gi < groups; gi += nsets, buf ^= 1) {
-            const int r0 = row_begin + gi * 16;
-            mma_row_group<D>(g, lane, wi, static_cast<uint32_t>(w_base) + static_cast<uint32_t>(r0) * static_cast<uint32_t>(a.row_bytes) +
-                                              static_cast<uint32_t>(sb0) * D::kBytes,
-                             static_cast<uint32_t>(a.row_bytes), nsb, xq0, xs0, ring0, full + set * g.ring, empty + set * g.ring, s,
-                             phase, abort_flag, a.status, a.wait_limit, part + ((set * 2 + buf) * g.wpg + wi) * 128);
-            asm volatile("bar.sync %0, %1;" ::"r"(2 + set), "r"(g.wpg * 32) : "memory");
-            const float* all = part + (set * 2 + buf) * g.wpg * 128;
-            for (int i = set_tid; i < 128; i += g.wpg * 32) {
-                const int col = i >> 4, r = i & 15;
-                float v = all[r * 8 + col];
-                for (int w = 1; w < g.wpg; ++w) v += all[w * 128 + r * 8 + col];
-                if (g.ksplit > 1) sums[(gi * 16 + r) * 8 + col] = v;
-                else if (col < a.M && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + r0 + r, v);
+    // The stream's cursor: the next block to be copied and the slot it goes to.  Weights are
+    // constants of the model, so the ring fills before the wait for the kernel in front.
+    int pg = w.wi < nsb ? w.set : groups, psb = w.wi, pslot = 0;
+    auto prefetch = [&]() {
+        if (pg < groups) {
+            const int r0 = row_begin + pg * 16;
+            stream.issue(w.slot(pslot), w_base + static_cast<uintptr_t>(r0) * row_bytes + static_cast<uint32_t>(psb * D::kBytes), row_end - r0,
+                         w_end, policy);
+            psb += g.wpg;
+            if (psb >= nsb) {
+                psb = w.wi;
+                pg += nsets;
             }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (++pslot == w.depth) pslot = 0;
+    };
+    for (int i = 0; i + 1 < w.depth; ++i) prefetch();
+
+    if (a.dep_mode != 2) pdl_wait_prior();
+    if (a.dep_mode == 1) pdl_launch_dependents();
+    if (Am) mma_image_bf16<D>(smem, Am, a.M, a.K, sb0 * 8, nsb * 8, tid, kMmaThreads);
+    else mma_image_q8_1<D>(smem, xqm, a.M, a.K / 32, sb0 * 8, nsb * 8, tid, kMmaThreads);
+    __syncthreads();
+
+    int slot = 0, buf = 0;
+    for (int gi = w.set; gi < groups; gi += nsets, buf ^= 1) {
+        const int r0 = row_begin + gi * 16;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int sb = w.wi; sb < nsb; sb += g.wpg) {
+            prefetch();
+            mma_wait_block(w.depth);
+            __syncwarp();
+            w.multiply(slot, sb, static_cast<uint32_t>(w_base) + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes),
+                       row_bytes, acc);
+            __syncwarp();   // every lane has read the slot before it is filled again
+            if (++slot == w.depth) slot = 0;
+        }
+        mma_add_tiles(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int col, float v) {
+            if (g.ksplit > 1) sums[(gi * 16 + r) * 8 + col] = v;
+            else if (col < a.M && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + r0 + r, v);
+        });
     }
     if (g.ksplit > 1) {
         __syncwarp();
@@ -622,115 +686,82 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
 // Grouped (MoE) form: the segments of the device-built list (expert, first row, up to eight rows)
 // times the expert's row groups are one virtual space, cut into equal contiguous ranges of row
 // groups, one per persistent CTA.  A CTA rebuilds its activation image where its range crosses
-// into another segment; row groups go to the sets round robin across segments, so every set's
-// ring is one sequence.  K fits one CTA's share (no clusters).
+// into another segment, while the copies of the next blocks are under way; row groups go to the
+// sets round robin across segments.  K fits one CTA (no clusters).
 template <int T>
 __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_grouped_kernel(const MmaGroupedArgs args) {
     using D = MmaDec<T>;
     const GroupedArgs& a = args.v;
     const MmaCut& g = args.c;
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* ring = smem + g.img_bytes;
     float* part = reinterpret_cast<float*>(smem + g.part_off);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + g.bar_off);
-    const int nsets = kMmaWarps / g.wpg;
-    uint64_t* empty = full + nsets * g.ring;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + nsets * g.ring);
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int stage_bytes = 16 * g.pitch;
-    if (tid < nsets * g.ring) {
-        mbar_init(&full[tid], 1);
-        mbar_init(&empty[tid], g.wpg);
-        mbar_fence_init();
-    }
-    if (tid == 0) *abort_flag = 0;
-    __syncthreads();
     pdl_launch_dependents();
     pdl_wait_prior();   // the segment list and the activations come from earlier kernels
 
     const int gn = (a.N + 15) >> 4;   // row groups of an expert
     const long long V = static_cast<long long>(a.seg[0]) * gn;
-    const long long vb = V * blockIdx.x / gridDim.x, ve = V * (blockIdx.x + 1) / gridDim.x;
+    const long long vb = V * blockIdx.x / gridDim.x;
+    const int total = static_cast<int>(V * (blockIdx.x + 1) / gridDim.x - vb);   // row groups of this CTA
+    if (total == 0) return;
+    const int sg0 = static_cast<int>(vb / gn), first0 = static_cast<int>(vb - static_cast<long long>(sg0) * gn);
 
-    if (warp == kMmaWarps) {
-        const uint64_t policy = l2_policy_evict_first();
-        bool ok = true;
-        int slot0 = 0, set = 0;   // ring position of the round's first stage, set of the next row group
-        uint32_t lap0 = 0;
-        for (long long cur = vb; cur < ve && ok;) {
-            const int sg = static_cast<int>(cur / gn);
-            const int first = static_cast<int>(cur - static_cast<long long>(sg) * gn);
-            const int last = static_cast<int>(min(static_cast<long long>(gn), first + (ve - cur)));
-            const uintptr_t w_base = reinterpret_cast<uintptr_t>(a.B_ptrs[a.seg[1 + 3 * sg]]);
-            // a matrix off a 16-byte boundary is moved with byte loads rather than read before its start
-            const uintptr_t w_end_al = (w_base & 15) ? 0 : (w_base + static_cast<uintptr_t>(a.N) * a.row_bytes) & ~uintptr_t(15);
-            for (int gi = first; gi < last && ok; ++gi) {
-                int slot = slot0;
-                uint32_t lap = lap0;
-                for (int c = 0; c < g.nc && ok; ++c) {
-                    const int s = set * g.ring + slot;
-                    if (lap > 0) {
-                        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], (lap - 1) & 1, a.status, kDevWaitEmpty));
-                        if (!ok) break;
-                    }
-                    mma_copy_stage(ring + static_cast<size_t>(s) * stage_bytes,
-                                   w_base + static_cast<uintptr_t>(gi * 16) * a.row_bytes + static_cast<uintptr_t>(c * g.chunk) * g.sb_bytes,
-                                   min(16, a.N - gi * 16), a.row_bytes, min(g.chunk, g.nsb - c * g.chunk) * g.sb_bytes, g.pitch,
-                                   w_end_al, D::kBytes % 16 != 0, &full[s], policy);
-                    if (++slot == g.ring) {
-                        slot = 0;
-                        ++lap;
-                    }
-                }
-                if (++set == nsets) {
-                    set = 0;
-                    slot0 = slot;
-                    lap0 = lap;
-                }
+    const MmaWarp<D> w(g, smem, g.nsb * 8);
+    const int nsets = kMmaWarps / g.wpg;
+    const uint32_t row_bytes = static_cast<uint32_t>(a.row_bytes);
+    const MmaStream<D> stream(row_bytes, w.lane);
+    const uint64_t policy = l2_policy_evict_first();
+
+    // The stream's cursor: row group pn of the range (pgi of segment psg), block psb of it.
+    int pn = w.wi < g.nsb ? w.set : total, psg = sg0, pgi = first0 + w.set, psb = w.wi, pslot = 0;
+    auto prefetch = [&]() {
+        if (pn < total) {
+            while (pgi >= gn) {
+                pgi -= gn;
+                ++psg;
             }
-            cur += last - first;
+            const uintptr_t base = reinterpret_cast<uintptr_t>(a.B_ptrs[a.seg[1 + 3 * psg]]);
+            // a matrix off a 16-byte boundary is moved byte by byte rather than read before its start
+            const uintptr_t end = (base & 15) ? 0 : (base + static_cast<uintptr_t>(a.N) * row_bytes) & ~uintptr_t(15);
+            stream.issue(w.slot(pslot), base + static_cast<uintptr_t>(pgi * 16) * row_bytes + static_cast<uint32_t>(psb * D::kBytes),
+                         a.N - pgi * 16, end, policy);
+            psb += g.wpg;
+            if (psb >= g.nsb) {
+                psb = w.wi;
+                pn += nsets;
+                pgi += nsets;
+            }
         }
-        if (!ok) *abort_flag = 1;
-        return;
-    }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (++pslot == w.depth) pslot = 0;
+    };
+    for (int i = 0; i + 1 < w.depth; ++i) prefetch();
 
-    const int n_cons = kMmaWarps * 32;
-    const int set = warp / g.wpg, wi = warp - set * g.wpg;
-    const int set_tid = wi * 32 + lane;
-    const int nblk = g.nsb * 8;
-    const uint32_t img = smem_u32(smem);
-    const uint32_t xq0 = img + (lane >> 2) * 32 + 8 * (lane & 3);
-    const uint32_t xs0 = img + nblk * 256 + (lane & 3) * (D::kSums ? 16 : 8);
-    const uint32_t ring0 = smem_u32(ring) + static_cast<uint32_t>(set * g.ring) * stage_bytes;
-    int s = 0, buf = 0, next = set;   // next: this set's next row group, counted from the range's first
-    uint32_t phase = 0;
-    int done = 0;                     // row groups of the segments before this one
-    for (long long cur = vb; cur < ve;) {
-        const int sg = static_cast<int>(cur / gn);
-        const int first = static_cast<int>(cur - static_cast<long long>(sg) * gn);
-        const int last = static_cast<int>(min(static_cast<long long>(gn), first + (ve - cur)));
+    int slot = 0, buf = 0, next = w.set;   // next: this set's next row group of the range
+    int done = 0;                          // row groups of the segments before this one
+    for (int sg = sg0, first = first0; done < total; ++sg, first = 0) {
+        const int last = min(gn, first + total - done);
         const int arow0 = a.seg[2 + 3 * sg], mcount = a.seg[3 + 3 * sg];
         const uint32_t w_lo = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(a.B_ptrs[a.seg[1 + 3 * sg]]));
-        if (done > 0) asm volatile("bar.sync 1, %0;" ::"r"(n_cons) : "memory");   // the previous image is no longer read
-        mma_image_q8_1<D>(smem, a.xq + static_cast<size_t>(arow0) * (a.K / 32) * kQ8_1Bytes, mcount, a.K / 32, 0, nblk, tid, n_cons);
-        asm volatile("bar.sync 1, %0;" ::"r"(n_cons) : "memory");
+        if (done > 0) __syncthreads();   // the previous image is no longer read
+        mma_image_q8_1<D>(smem, a.xq + static_cast<size_t>(arow0) * (a.K / 32) * kQ8_1Bytes, mcount, a.K / 32, 0, g.nsb * 8, threadIdx.x,
+                          kMmaThreads);
+        __syncthreads();
         for (; next < done + last - first; next += nsets, buf ^= 1) {
             const int r0 = (first + next - done) * 16;
-            mma_row_group<D>(g, lane, wi, w_lo + static_cast<uint32_t>(r0) * static_cast<uint32_t>(a.row_bytes),
-                             static_cast<uint32_t>(a.row_bytes), g.nsb, xq0, xs0, ring0, full + set * g.ring, empty + set * g.ring, s,
-                             phase, abort_flag, a.status, kWaitLimitCycles, part + ((set * 2 + buf) * g.wpg + wi) * 128);
-            asm volatile("bar.sync %0, %1;" ::"r"(2 + set), "r"(g.wpg * 32) : "memory");
-            const float* all = part + (set * 2 + buf) * g.wpg * 128;
-            for (int i = set_tid; i < 128; i += g.wpg * 32) {
-                const int col = i >> 4, r = i & 15;
-                float v = all[r * 8 + col];
-                for (int w = 1; w < g.wpg; ++w) v += all[w * 128 + r * 8 + col];
-                if (col < mcount && r0 + r < a.N) store_out(a.D, a.out_f32, static_cast<size_t>(arow0 + col) * a.N + r0 + r, v);
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int sb = w.wi; sb < g.nsb; sb += g.wpg) {
+                prefetch();
+                mma_wait_block(w.depth);
+                __syncwarp();
+                w.multiply(slot, sb, w_lo + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes), row_bytes, acc);
+                __syncwarp();
+                if (++slot == w.depth) slot = 0;
             }
+            mma_add_tiles(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int col, float v) {
+                if (col < mcount && r0 + r < a.N) store_out(a.D, a.out_f32, static_cast<size_t>(arow0 + col) * a.N + r0 + r, v);
+            });
         }
         done += last - first;
-        cur += last - first;
     }
 }
 

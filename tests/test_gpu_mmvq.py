@@ -135,17 +135,18 @@ def test_mmvq_q4k_golden_fixture(ops, golden_dir):
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "Q4_0"])
 @pytest.mark.parametrize("M,N,K", [
-    (2, 1, 256),        # one block, one row
-    (3, 17, 768),       # three blocks, a row group with one live row
+    (5, 1, 256),        # one block, one row
+    (7, 17, 768),       # three blocks, a row group with one live row
     (8, 2400, 1280),    # several row groups per CTA, the last one ragged
     (5, 300, 4096),     # the longest row one CTA takes
     (8, 33, 4352),      # K shared by two CTAs, odd number of blocks
-    (4, 161, 8448),     # by four
+    (6, 161, 8448),     # by four
     (7, 700, 14336),    # activations quantized by a kernel of their own
-    (2, 40, 16640),     # by eight, the last one with fewer blocks
+    (5, 40, 16640),     # by eight, the last one with fewer blocks
+    (4, 300, 4352),     # one row fewer than that kernel takes
 ])
 def test_mmvq_tensor_core_edges(ops, name, M, N, K):
-    """Two to eight batch rows, at the edges of the row groups and of the cuts of K: same integers
+    """Five to eight batch rows, at the edges of the row groups and of the cuts of K: same integers
     as the oracle, so only the order of the fp32 sums differs (TOL_F32); and independent of what
     shares the launch."""
     t = T[name]
