@@ -586,10 +586,14 @@ def bf16_to_nvfp4(x):
     single-problem quantizer (launch_bf16_to_nvfp4, csrc/smxx/quant/bf16_to_nvfp4.cu:136-140)."""
     _require(x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.is_contiguous(),
              "bf16_to_nvfp4: x must be contiguous BF16 [M, K] on CUDA")
+    return _bf16_to_nvfp4(x, torch.zeros)
+
+
+def _bf16_to_nvfp4(x, scale_buffer):
     M, K = x.shape
     _require(K % 16 == 0, "bf16_to_nvfp4: K must be divisible by 16")
     packed = torch.empty((M, K // 2), dtype=torch.uint8, device=x.device)
-    scales = torch.zeros((_lib.lsg_nvfp4_sf_buffer_bytes(M, K),), dtype=torch.uint8, device=x.device)
+    scales = scale_buffer((_lib.lsg_nvfp4_sf_buffer_bytes(M, K),), dtype=torch.uint8, device=x.device)
     capi.check(_lib.lsg_bf16_to_nvfp4(_ptr(x), _ptr(packed), _ptr(scales), M, K, _stream()))
     return packed, scales
 
@@ -647,7 +651,9 @@ def nvfp4_gemm_from_bf16(x_bf16, weight_packed_uint8, weight_scales, weight_scal
         sfb = weight_scales
     else:
         sfb = nvfp4_gemm_preprocess(weight_scales, N, K)
-    codes, sfa = bf16_to_nvfp4(x_bf16)
+    # whole 64-value K blocks: every scale the GEMM uses is written by the quantizer (the padding
+    # rows' are multiplied by zero codes into rows that are not stored), so nothing has to be cleared
+    codes, sfa = _bf16_to_nvfp4(x_bf16, torch.empty if K % 64 == 0 else torch.zeros)
     return nvfp4_gemm(codes, weight_packed_uint8, sfa, sfb, M, N, K, float(weight_scale_global), "bf16")
 
 
