@@ -151,26 +151,48 @@ __device__ __forceinline__ void q8_round8(const float* x, float d, float rcp, ui
     w1 = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
 }
 
-// The Q8_1 round trip of eight values of one block, dh * rn(fl(x / d)) as floats, on the arithmetic
-// of q8_round8 (the rounded quotient is read back by subtracting the magic number instead of being
-// taken off the mantissa; a quotient that rounds to -0 comes out as +0).
-__device__ __forceinline__ void q8_roundtrip8(const float* x, float d, float rcp, float dh, float* out) {
-    const float magic = 12582912.0f;
-    float km[8];
+// The Q8_1 round trip of half a block: sixteen bf16 values (eight packed pairs; the other half is
+// in the neighbouring lane, `lanes` are the lanes that call) -> dh * rn(fl(x / d)) as fp16 pairs.
+// The kernels that do this are bound by instruction issue, so: the largest magnitude and the test
+// for NaN are taken on packed pairs; the quotient is rounded by adding 1.5 * 2^23 as in q8_round8;
+// and one fma takes that number off again and scales, fma(k + magic, dh, -magic * dh), which is
+// exact (k has seven bits, dh eleven, magic two).  A quotient that rounds to -0 comes out as +0.
+// Scales outside [1e-28, 6e4] (zero blocks, infinities, an fp16 scale that overflows) and groups
+// with a NaN take the plain path.
+__device__ __forceinline__ void q8_roundtrip16(const uint32_t (&w)[8], unsigned lanes, uint32_t (&out)[8]) {
+    auto bits = [](uint32_t v) { return *reinterpret_cast<const __nv_bfloat162*>(&v); };
+    __nv_bfloat162 m = __habs2(bits(w[0])), mn = m;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float t = x[i] * rcp;
-        km[i] = fmaf(fmaf(-t, d, x[i]), rcp, t) + magic;
+    for (int i = 1; i < 8; ++i) {
+        const __nv_bfloat162 v = __habs2(bits(w[i]));
+        m = __hmax2(m, v);        // the number where one operand is NaN
+        mn = __hmax2_nan(mn, v);  // NaN there
     }
-    const float m = max_nan(max_nan(max_nan(km[0], km[1]), max_nan(km[2], km[3])),
-                            max_nan(max_nan(km[4], km[5]), max_nan(km[6], km[7])));
-    if (!(d >= 1e-28f && d <= 1e30f) || m != m) {
+    const uint32_t mb = *reinterpret_cast<const uint32_t*>(&m), nb = *reinterpret_cast<const uint32_t*>(&mn);
+    float amax = fmaxf(fmaxf(__uint_as_float(mb << 16), __uint_as_float(mb & 0xFFFF0000u)), 0.0f);
+    amax = fmaxf(amax, __shfl_xor_sync(lanes, amax, 1));
+    const float d = amax / 127.0f;
+    const float rcp = (amax == 0.0f) ? 0.0f : 1.0f / d;
+    const float dh = __half2float(__float2half(d));
+    const bool nan = (nb & 0x7FFFu) > 0x7F80u || (nb & 0x7FFF0000u) > 0x7F800000u;
+    if (nan || !(d >= 1e-28f && d <= 6e4f)) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) out[i] = dh * q8_round_f(x[i], d, rcp);
+        for (int i = 0; i < 8; ++i) {
+            const __half2 h = __floats2half2_rn(dh * q8_round_f(__uint_as_float(w[i] << 16), d, rcp),
+                                                dh * q8_round_f(__uint_as_float(w[i] & 0xFFFF0000u), d, rcp));
+            out[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
         return;
     }
+    const float magic = 12582912.0f, off = -magic * dh;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) out[i] = dh * (km[i] - magic);
+    for (int i = 0; i < 8; ++i) {
+        const float x0 = __uint_as_float(w[i] << 16), x1 = __uint_as_float(w[i] & 0xFFFF0000u);
+        const float t0 = x0 * rcp, t1 = x1 * rcp;
+        const float k0 = fmaf(fmaf(-t0, d, x0), rcp, t0) + magic, k1 = fmaf(fmaf(-t1, d, x1), rcp, t1) + magic;
+        const __half2 h = __floats2half2_rn(fmaf(k0, dh, off), fmaf(k1, dh, off));
+        out[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

@@ -89,21 +89,6 @@ constexpr int kFPartRow = 2 * FN * 4 + 16;   // bytes of a parked accumulator ro
                                              // eight lanes' 16-byte pieces hit different banks
 static_assert(FM * kFPartRow <= kFStages * kFStageBytes, "the parked tile takes the ring's place");
 
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
-    uint32_t addr;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "r"(addr)
-                 : "memory");
-    return v;
-}
-
 // Shared-memory matrix descriptor of one scale atom for tcgen05.cp: 32 rows of 16 bytes, no
 // swizzle, 8-row core matrices 128 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc_sf_atom(uint32_t smem_addr) {

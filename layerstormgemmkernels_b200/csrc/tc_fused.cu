@@ -34,11 +34,12 @@
 // decoder warps + the TMA transaction); tcgen05.commit releases it.  All waits are
 // time-limited; a time-out ends every role and is reported in the status word.
 //
-// Small token counts with few weight rows would leave most SMs idle, so the K range of an
-// output tile can be split over several CTAs.  Each split stores its fp32 partial tile; per
-// 32-row slice the warp that arrives last at the slice's counter adds the partials in split
-// order (deterministic) and writes C.  The counters are zeroed by the activation-preparation
-// kernel of the same call.
+// A dense call with fewer output tiles than SMs shares the K range of a tile among the CTAs of a
+// cluster: every CTA parks its fp32 tile in its own shared memory, in the place of the token tiles,
+// and after a cluster barrier the CTAs add the tiles in rank order, each its share, reading the
+// peers' through distributed shared memory (the same bits on every run, no workspace).  When the
+// splits stored their tiles to global memory and the last to arrive added them, that alone took
+// 15 us of 44 (4096 x 14336, 48 rows).
 #include "common.cuh"
 #include "formats.cuh"
 #include "host.h"
@@ -86,10 +87,8 @@ struct FusedArgs {
     int stages;
     int raw_depth;                // K blocks of packed weights in flight per decoder (0: none)
     int raw_bytes;                // shared memory of that ring
-    int ksplit;                   // CTAs per output tile along K
-    int kb_per_split;             // K blocks per split
-    float* partial;               // [items][ksplit][128][nt] fp32, only with ksplit > 1
-    unsigned int* counters;       // [tiles][4 epilogue warps], zero on entry
+    int ksplit;                   // CTAs of a cluster sharing an output tile's K range (1: no cluster)
+    int kb_per_split;             // K blocks of each
     const float* row_scale;       // optional per-token output scale (the unquantized-activation route)
     void* const* C_ptrs;          // optional: n_out output matrices (this GPU's and its peers'); every
     int n_out;                    //   element is stored into each of them (GEMM + all-gather)
@@ -204,10 +203,10 @@ struct DecGeneric {
     }
 };
 
-// Work item -> tile coordinates.  Items are ordered weight tile fastest, then K split, then
-// token tile, so CTAs running together share a token tile (and, grouped, an expert).
+// Work item -> tile coordinates.  Items are ordered weight tile fastest, then token tile, so CTAs
+// running together share a token tile (and, grouped, an expert).
 struct Item {
-    int tt, wt, ks;
+    int tt, wt;
     int expert;       // -1 dense
     int mstart, mend;
     bool live;
@@ -216,9 +215,7 @@ struct Item {
 __device__ __forceinline__ Item decode_item(const FusedArgs& a, int w, const int* tab) {
     Item it;
     it.wt = w % a.n_wtiles;
-    const int rest = w / a.n_wtiles;
-    it.ks = rest % a.ksplit;
-    it.tt = rest / a.ksplit;
+    it.tt = w / a.n_wtiles;
     it.expert = -1;
     it.mstart = it.tt * a.tile_rows;
     it.mend = min(a.M, it.mstart + a.tile_rows);
@@ -470,7 +467,7 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    pdl_wait_prior();  // x16, the tile map and the zeroed counters come from earlier kernels
+    pdl_wait_prior();  // x16 and the tile map come from earlier kernels
 
     // Grouped calls: every role looks every item's tile up, and three dependent global loads per
     // look-up sit in front of each item's first copy, decode and MMA.  The tile map is small, so
@@ -495,7 +492,11 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
     }
 
     const int kblocks_all = (a.K + BK - 1) / BK;
-    const int total = a.t_tiles * a.ksplit * a.n_wtiles;
+    const int total = a.t_tiles * a.n_wtiles;
+    const int rank = static_cast<int>(blockIdx.x) % a.ksplit;   // of this CTA in its cluster
+    const int w0 = static_cast<int>(blockIdx.x) / a.ksplit, w_step = static_cast<int>(gridDim.x) / a.ksplit;
+    const int kb0 = rank * a.kb_per_split;
+    const int kb1 = min(kblocks_all, kb0 + a.kb_per_split);
     const uint32_t hint = 2000u;  // suspend-time hint of the barrier waits, ns
 
     if (warp == 4) {
@@ -505,11 +506,9 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
             TCF_T0();
             Ring ring = {0, 0u, a.stages};
             bool ok = true;
-            for (int w = blockIdx.x; w < total && ok && !*abort_flag; w += gridDim.x) {
+            for (int w = w0; w < total && ok && !*abort_flag; w += w_step) {
                 const Item im = decode_item(a, w, tab);
                 if (!im.live) continue;
-                const int kb0 = im.ks * a.kb_per_split;
-                const int kb1 = min(kblocks_all, kb0 + a.kb_per_split);
                 const int live_rows = min(a.nt, im.mend - im.mstart);
                 const int live_boxes = max(1, (live_rows + a.box_rows - 1) / a.box_rows);
                 for (int kb = kb0; kb < kb1; ++kb) {
@@ -542,11 +541,9 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
         int tile_i = 0, ab = 0;
         uint32_t acc_lap = 0;  // how often the accumulator set has been cycled through
         bool ok = true;
-        for (int w = blockIdx.x; w < total && ok && !*abort_flag; w += gridDim.x) {
+        for (int w = w0; w < total && ok && !*abort_flag; w += w_step) {
             const Item im = decode_item(a, w, tab);
             if (!im.live) continue;
-            const int kb0 = im.ks * a.kb_per_split;
-            const int kb1 = min(kblocks_all, kb0 + a.kb_per_split);
             TCF_TIMED(1, if (acc_lap > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_empty[ab], (acc_lap - 1) & 1, a.status, kDevWaitTmem, hint)));
             if (!ok) break;
             TCF_COUNT(0, 1); TCF_COUNT(1, kb1 - kb0);
@@ -610,11 +607,9 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
 #endif
         TCF_T0();
         Ring ring = {0, 0u, a.stages};
-        for (int w = blockIdx.x; w < total && !*abort_flag; w += gridDim.x) {
+        for (int w = w0; w < total && !*abort_flag; w += w_step) {
             const Item im = decode_item(a, w, tab);
             if (!im.live) continue;
-            const int kb0 = im.ks * a.kb_per_split;
-            const int kb1 = min(kblocks_all, kb0 + a.kb_per_split);
             const bool second = a.B_ptrs2 != nullptr && im.wt >= a.split_wt;
             const uint8_t* base = a.B_ptrs ? static_cast<const uint8_t*>((second ? a.B_ptrs2 : a.B_ptrs)[im.expert])
                                            : a.W;
@@ -656,7 +651,7 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
         TCF_T0();
         int tile_i = 0, ab = 0;
         uint32_t acc_lap = 0;
-        for (int w = blockIdx.x; w < total && !*abort_flag; w += gridDim.x) {
+        for (int w = w0; w < total && !*abort_flag; w += w_step) {
             const Item im = decode_item(a, w, tab);
             if (!im.live) continue;
             bool landed = false;
@@ -729,69 +724,17 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[ab]);
             } else {
-                // Split K: park this split's fp32 tile [token][128 weight rows]; per 32-row
-                // slice of the tile, the warp that arrives last at the slice's counter adds
-                // the splits in order and writes C.  Each epilogue warp works alone, so no
-                // CTA-wide barrier sits inside a loop that a time-out may leave.
-                const int tile_id = im.tt * a.n_wtiles + im.wt;
-                const size_t tile_elems = static_cast<size_t>(WM) * a.nt;
-                float* mine = a.partial + (static_cast<size_t>(tile_id) * a.ksplit + im.ks) * tile_elems;
+                // Split K: park this CTA's fp32 tile as [token][128 weight rows]; one item per cluster
+                float* mine = reinterpret_cast<float*>(smem) + warp * 32 + lane;
                 const int live_rows = min(a.nt, im.mend - im.mstart);
 #pragma unroll 1
                 for (int c = 0; c < live_rows; c += 32) {
                     uint32_t v[32];
                     tmem_ld32(t_lane + c, v);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        mine[static_cast<size_t>(c + i) * WM + warp * 32 + lane] = __uint_as_float(v[i]);
+                    for (int i = 0; i < 32; ++i) mine[(c + i) * WM] = __uint_as_float(v[i]);
                 }
-                tc_fence_before();
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[ab]);
-                unsigned int prev = 0;
-                if (lane == 0) prev = atomicAdd(&a.counters[tile_id * 4 + warp], 1u);
-                prev = __shfl_sync(0xffffffffu, prev, 0);
-                if (prev == static_cast<unsigned int>(a.ksplit - 1)) {
-                    __threadfence();
-                    const float* tile0 = a.partial + static_cast<size_t>(tile_id) * a.ksplit * tile_elems;
-                    if (n_ok) {
-                        // 32 token rows at a time: the loads of one split are independent and all
-                        // in flight together; the splits are added in order.
-                        for (int i0 = 0; i0 < live_rows; i0 += 32) {
-                            float acc[32];
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
-                            const float* col = tile0 + static_cast<size_t>(i0) * WM + warp * 32 + lane;
-                            for (int sp = 0; sp < a.ksplit; ++sp) {
-                                float v[32];
-#pragma unroll
-                                for (int i = 0; i < 32; ++i)
-                                    v[i] = (i0 + i < live_rows) ? __ldcg(col + sp * tile_elems + static_cast<size_t>(i) * WM)
-                                                                : 0.0f;
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) acc[i] += v[i];
-                            }
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) {
-                                if (i0 + i < live_rows) {
-                                    if (a.row_scale) acc[i] *= __ldg(a.row_scale + im.mstart + i0 + i);
-                                    const size_t o = static_cast<size_t>(im.mstart + i0 + i) * a.ldc + n;
-                                    const int n_out = a.n_out > 0 ? a.n_out : 1;
-                                    for (int po = 0; po < n_out; ++po) {
-                                        void* Cb = a.n_out > 0 ? a.C_ptrs[po] : a.C;
-                                        if (a.out_dtype == LSG_DTYPE_F32)
-                                            static_cast<float*>(Cb)[o] = acc[i];
-                                        else if (a.out_dtype == LSG_DTYPE_F16)
-                                            static_cast<uint16_t*>(Cb)[o] = __half_as_ushort(__float2half_rn(acc[i]));
-                                        else
-                                            static_cast<uint16_t*>(Cb)[o] = __bfloat16_as_ushort(__float2bfloat16_rn(acc[i]));
-                                    }
-                                }
-                            }
-                        }
-                    }
-                }
+                break;
             }
             ++tile_i;
             if (++ab == nacc) {
@@ -808,11 +751,56 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
     }
+    if (a.ksplit > 1) {
+        // Every thread of every CTA of the cluster comes here, after a time-out too.
+        __syncwarp();
+        cluster_sync();
+        const Item im = decode_item(a, w0, nullptr);
+        const uint32_t base = smem_u32(smem);
+        const int pieces = max(0, min(a.nt, im.mend - im.mstart)) * (WM / 4);   // four weight rows of a token
+        const int n_out = a.n_out > 0 ? a.n_out : 1;
+        for (int i = rank * kFusedThreads + threadIdx.x; i < pieces; i += a.ksplit * kFusedThreads) {
+            const int tok = i / (WM / 4), q = i % (WM / 4);
+            const int n = im.wt * WM + 4 * q;
+            if (n >= a.N) continue;
+            const uint32_t at = base + static_cast<uint32_t>(tok * WM + 4 * q) * 4u;
+            float4 v = ld_cluster_f4(at, 0);
+            for (int k = 1; k < a.ksplit; ++k) {
+                const float4 p = ld_cluster_f4(at, k);
+                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            }
+            if (a.row_scale) {
+                const float rs = __ldg(a.row_scale + im.mstart + tok);
+                v.x *= rs; v.y *= rs; v.z *= rs; v.w *= rs;
+            }
+            const float e[4] = {v.x, v.y, v.z, v.w};
+            const size_t o = static_cast<size_t>(im.mstart + tok) * a.ldc + a.col_off + n;
+            for (int po = 0; po < n_out; ++po) {
+                void* Cb = a.n_out > 0 ? a.C_ptrs[po] : a.C;
+                const bool whole = n + 4 <= a.N;
+                if (a.out_dtype == LSG_DTYPE_BF16 && whole && (reinterpret_cast<uintptr_t>(static_cast<uint16_t*>(Cb) + o) & 7) == 0) {
+                    const __nv_bfloat162 h0 = __floats2bfloat162_rn(e[0], e[1]), h1 = __floats2bfloat162_rn(e[2], e[3]);
+                    *reinterpret_cast<uint2*>(static_cast<uint16_t*>(Cb) + o) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+                    continue;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (n + j >= a.N) break;
+                    if (a.out_dtype == LSG_DTYPE_F32) static_cast<float*>(Cb)[o + j] = e[j];
+                    else if (a.out_dtype == LSG_DTYPE_F16) static_cast<uint16_t*>(Cb)[o + j] = __half_as_ushort(__float2half_rn(e[j]));
+                    else static_cast<uint16_t*>(Cb)[o + j] = __bfloat16_as_ushort(__float2bfloat16_rn(e[j]));
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();   // no CTA leaves while a peer still reads its tile
+    }
 }
 
 // ---------------------------------------------------------------------------
 // Activation preparation: bf16 -> fp16 of the Q8_1 round trip (d_h * rn(x / d), the values
-// the integer kernels multiply by), plus zeroing of the split-K tile counters.
+// the integer kernels multiply by).
 //
 // SWIGLU = false: x[rows, K].  With a permutation the rows are gathered on the way in: row i
 // of the output is token perm[i] / top_k of x (the permute pass of a MoE layer folded in).
@@ -820,105 +808,96 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
 //   act = bf16( silu(g) * u )  with silu(g) = g / (1 + exp(-g)) in fp32
 // (what a caller computing the activation in fp32 and storing bf16 gets), then the round trip.
 //
-// Four lanes per 32-value block, eight values (one 16-byte vector) each.  The thread block is
-// (vectors of a row, rows); every thread handles RB rows, so RB (2 RB with SwiGLU) independent
-// loads are in flight per thread and no index needs a division.  Grouped callers may hold
-// fewer rows than the buffer they pass: the row count then lives on the device (live_rows).
+// Two lanes per 32-value block, sixteen values (two 16-byte vectors) each: the pass is bound by
+// instruction issue, and what a thread does once (the block's scale and its reciprocal, the row's
+// source, addresses) is shared by sixteen values (q8_roundtrip16 has the rest).  32768 x 2048
+// gathered rows: 59.3 us with eight values per thread.  The thread block is (vector pairs of a row,
+// rows); every thread handles RB rows, so 2 RB (4 RB with SwiGLU) independent loads are in flight
+// per thread.  Grouped callers may hold fewer rows than the buffer they pass: the row count then
+// lives on the device (live_rows).
 // ---------------------------------------------------------------------------
 template <int RB, bool SWIGLU>
 __global__ void __launch_bounds__(256)
-x_prep_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ out, int rows, int vpr,
-              unsigned int* __restrict__ counters, int n_counters, const int32_t* __restrict__ live_rows,
-              const int32_t* __restrict__ perm, int top_k, const int32_t* __restrict__ first_row) {
-    const unsigned lanes = __activemask();   // a block of K/8 x rows threads may end in a partial warp
+x_prep_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ out, int rows, int ppr, const int32_t* __restrict__ live_rows,
+              const int32_t* __restrict__ perm, int top_k, uint32_t top_k_magic, const int32_t* __restrict__ first_row) {
+    const unsigned lanes = __activemask();   // a block of K/16 x rows threads may end in a partial warp
     pdl_launch_dependents();
     pdl_wait_prior();
     const int tx = threadIdx.x, ty = threadIdx.y;
-    if (counters) {
-        const int nthreads = blockDim.x * blockDim.y;
-        const long long stride = static_cast<long long>(gridDim.x) * gridDim.y * nthreads;
-        for (long long i = (static_cast<long long>(blockIdx.y) * gridDim.x + blockIdx.x) * nthreads + ty * blockDim.x + tx;
-             i < n_counters; i += stride)
-            counters[i] = 0;
-    }
     const int live = live_rows ? min(rows, __ldg(live_rows)) : rows;
     if (static_cast<int>(blockIdx.x * (blockDim.y * RB)) >= live) return;   // the whole block lies past the live rows
     // ... or before the first row any expert of this call owns (a call on a group of experts)
     if (first_row && static_cast<int>((blockIdx.x + 1) * (blockDim.y * RB)) <= __ldg(first_row)) return;
-    const int v = blockIdx.y * blockDim.x + tx;
+    const int v = blockIdx.y * blockDim.x + tx;   // sixteen-value pair of vectors inside the row
     const int rbase = blockIdx.x * (blockDim.y * RB) + ty;
-    const int ld_in = SWIGLU ? 2 * vpr : vpr;
+    const int ld_in = SWIGLU ? 4 * ppr : 2 * ppr;
     const uint4* xin = reinterpret_cast<const uint4*>(x);
-    uint4 g[RB], u[RB];
+    uint4 g[RB][2], u[RB][2];
     bool ok[RB];
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
         const int r = rbase + j * blockDim.y;
-        ok[j] = v < vpr && r < live;
-        g[j] = make_uint4(0, 0, 0, 0);
-        u[j] = make_uint4(0, 0, 0, 0);
+        ok[j] = v < ppr && r < live;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) g[j][h] = u[j][h] = make_uint4(0, 0, 0, 0);
         if (ok[j]) {
-            const int sr = perm ? __ldg(perm + r) / top_k : r;
-            const uint4* src = xin + static_cast<size_t>(sr) * ld_in + v;
-            g[j] = __ldg(src);
-            if (SWIGLU) u[j] = __ldg(src + vpr);
+            int sr = r;
+            if (perm) {
+                // quotient by multiply-high, exact while n * top_k < 2^32
+                const int n = __ldg(perm + r);
+                sr = top_k == 1 ? n
+                     : (static_cast<uint32_t>(n) < 0xFFFFFFFFu / 1024u && top_k <= 1024)
+                         ? static_cast<int>(__umulhi(static_cast<uint32_t>(n), top_k_magic))
+                         : n / top_k;
+            }
+            const uint4* src = xin + static_cast<size_t>(sr) * ld_in + 2 * v;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                g[j][h] = __ldg(src + h);
+                if (SWIGLU) u[j][h] = __ldg(src + 2 * ppr + h);
+            }
         }
     }
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
-        const uint32_t gw[4] = {g[j].x, g[j].y, g[j].z, g[j].w}, uw[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
-        float val[8];
+        uint32_t w[8] = {g[j][0].x, g[j][0].y, g[j][0].z, g[j][0].w, g[j][1].x, g[j][1].y, g[j][1].z, g[j][1].w};
+        if (SWIGLU) {
+            const uint32_t uw[8] = {u[j][0].x, u[j][0].y, u[j][0].z, u[j][0].w, u[j][1].x, u[j][1].y, u[j][1].z, u[j][1].w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const float a = __uint_as_float(hh ? (gw[i] & 0xFFFF0000u) : (gw[i] << 16));
-                if (SWIGLU) {
-                    const float b = __uint_as_float(hh ? (uw[i] & 0xFFFF0000u) : (uw[i] << 16));
-                    val[2 * i + hh] = __bfloat162float(__float2bfloat16_rn((a / (1.0f + expf(-a))) * b));
-                } else {
-                    val[2 * i + hh] = a;
-                }
-            }
+            for (int i = 0; i < 8; ++i) w[i] = silu_mul_bf16x2(w[i], uw[i]);
         }
-        float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(val[i]));
-        amax = fmaxf(amax, __shfl_xor_sync(lanes, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(lanes, amax, 2));
-        const float d = amax / 127.0f;
-        const float rcp = (amax == 0.0f) ? 0.0f : 1.0f / d;
-        const float dh = __half2float(__float2half(d));
-        float q[8];
-        q8_roundtrip8(val, d, rcp, dh, q);
-        const uint32_t pk[4] = {pack_h2(q[0], q[1]), pack_h2(q[2], q[3]), pack_h2(q[4], q[5]), pack_h2(q[6], q[7])};
+        uint32_t pk[8];
+        q8_roundtrip16(w, lanes, pk);
         if (ok[j]) {
-            const int r = rbase + j * blockDim.y;
-            reinterpret_cast<uint4*>(out)[static_cast<size_t>(r) * vpr + v] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            uint4* dst = reinterpret_cast<uint4*>(out) + static_cast<size_t>(rbase + j * blockDim.y) * (2 * ppr) + 2 * v;
+            dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
         }
     }
 }
 
-// rows x K values (K a multiple of 32).  The block is (min(K/8, 256) vectors, 256 / that rows).
+// rows x K values (K a multiple of 32).
 template <bool SWIGLU>
-int launch_x_prep(const __nv_bfloat16* x, __half* out, long long rows, int K, unsigned int* counters, int n_counters,
-                  const int32_t* live_rows, const int32_t* perm, int top_k, cudaStream_t s,
+int launch_x_prep(const __nv_bfloat16* x, __half* out, long long rows, int K, const int32_t* live_rows, const int32_t* perm, int top_k, cudaStream_t s,
                   const int32_t* first_row = nullptr) {
     if (rows <= 0 || rows > 0x7fffffffll) return rows == 0 ? LSG_OK : fail(LSG_ERR_UNSUPPORTED, "activation preparation: too many rows");
-    const int vpr = K / 8;
-    const int bx = vpr < 256 ? vpr : 256;
-    const int by = 256 / bx > 0 ? 256 / bx : 1;
-    const int gy = (vpr + bx - 1) / bx;
-    // four rows per thread once there are enough rows to fill the GPU that way
-    const bool rb4 = rows >= 4ll * by * 2 * sm_count();
-    const int rows_per_block = by * (rb4 ? 4 : 1);
+    const int ppr = K / 16;
+    // two rows per thread once there are enough rows to fill the GPU that way; below that, blocks of
+    // 64 threads, so that a few rows spread over the SMs (48 x 4096: 1 us less than in blocks of 256)
+    const bool rb2 = rows * ppr >= 2ll * 256 * 2 * sm_count();
+    const int bmax = rb2 ? 256 : 64;
+    const int bx = ppr < bmax ? ppr : bmax;
+    const int by = bmax / bx;
+    const int gy = (ppr + bx - 1) / bx;
+    const uint32_t magic = top_k > 1 ? static_cast<uint32_t>((0x100000000ull + top_k - 1) / top_k) : 0u;
+    const int rows_per_block = by * (rb2 ? 2 : 1);
     const unsigned gx = static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block);
-    if (rb4)
-        LSG_CUDA_TRY(launch_kernel(x_prep_kernel<4, SWIGLU>, dim3(gx, gy), dim3(bx, by), 0, s, true, x, out,
-                                   static_cast<int>(rows), vpr, counters, n_counters, live_rows, perm, top_k, first_row));
+    if (rb2)
+        LSG_CUDA_TRY(launch_kernel(x_prep_kernel<2, SWIGLU>, dim3(gx, gy), dim3(bx, by), 0, s, true, x, out,
+                                   static_cast<int>(rows), ppr, live_rows, perm, top_k, magic, first_row));
     else
         LSG_CUDA_TRY(launch_kernel(x_prep_kernel<1, SWIGLU>, dim3(gx, gy), dim3(bx, by), 0, s, true, x, out,
-                                   static_cast<int>(rows), vpr, counters, n_counters, live_rows, perm, top_k, first_row));
+                                   static_cast<int>(rows), ppr, live_rows, perm, top_k, magic, first_row));
     return LSG_OK;
 }
 
@@ -927,10 +906,9 @@ int launch_x_prep(const __nv_bfloat16* x, __half* out, long long rows, int K, un
 // One warp per row.  Rows of zeros (or with no finite value) keep scale 1.
 __global__ void __launch_bounds__(256)
 x_rows_to_f16_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ out, float* __restrict__ scale, int M,
-                     int K, unsigned int* __restrict__ counters, int n_counters) {
+                     int K) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < n_counters; i += gridDim.x * 256) counters[i] = 0;
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= M) return;
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * K);
@@ -978,36 +956,64 @@ bool staged_decoder(int type) { return type == LSG_GGUF_Q4_K; }
 
 struct Plan {
     int nt, box_rows, a_col_base, stages, raw_depth, raw_bytes, t_tiles, n_wtiles, ksplit, kb_per_split;
-    size_t x_bytes, partial_bytes, counter_bytes;
-    size_t total() const { return x_bytes + partial_bytes + counter_bytes; }
+    size_t x_bytes;
+    size_t total() const { return x_bytes; }
 };
 
-int pick_nt(long long rows_per_problem) {
+// How a dense call is cut: token rows per tile and CTAs of a cluster per tile along K.
+struct DenseCut {
+    int nt, ksplit;
+};
+DenseCut dense_cut(int M, int N, int K) {
     static const int force = [] {
         const char* e = getenv("LSG_TC_FUSED_DENSE_NT");
         return e ? atoi(e) : 0;
     }();
-    if (force == 32 || force == 64 || force == 128 || force == 256 || force == 320 || force == 384) return force;
-    if (rows_per_problem <= 32) return 32;
-    if (rows_per_problem <= 64) return 64;
-    if (rows_per_problem <= 128) return 128;
+    if (force == 32 || force == 64 || force == 128 || force == 256 || force == 320 || force == 384) return {force, 1};
     // Every token tile repeats the decoding of the weights, so above 256 rows the height that
     // needs the fewest tiles wins; at equal count the lower one (more stages in shared memory).
     // Measured on 14336 x 4096 Q4_K: M = 4096 0.474 ms with 256-row tiles, 0.399 ms with 384.
-    int best = 256;
-    long long best_tiles = (rows_per_problem + 255) / 256;
-    for (int nt : {320, 384}) {
-        const long long tiles = (rows_per_problem + nt - 1) / nt;
-        if (tiles < best_tiles) {
-            best = nt;
-            best_tiles = tiles;
+    int nt = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256));
+    long long tiles = (M + nt - 1) / nt;
+    for (int h : {320, 384}) {
+        const long long t = (M + h - 1) / h;
+        if (M > 256 && t < tiles) {
+            nt = h;
+            tiles = t;
+        }
+    }
+    // With fewer tiles than SMs K is shared among the CTAs of a cluster, as far as they are all
+    // resident together.  A K block of 64 values takes a CTA 0.40 us at up to 64 token rows, 0.45 at
+    // 128 and 0.53 at 256 (the weights' decoding, not the rows); the parked tile, the barriers and
+    // the sum about 3 us, more with taller tiles.  48 rows: 4096 x 14336 44.4 us with the splits
+    // added through global memory, 89.8 unsplit; 14336 x 4096 (112 tiles, not worth a split) 45.5 in
+    // two waves of halves, 30.6 unsplit.
+    const int sms = sm_count(), wtiles = (N + WM - 1) / WM, kblocks = (K + BK - 1) / BK;
+    DenseCut best = {nt, 1};
+    if (tiles * wtiles >= sms) return best;
+    double best_us = 1e30;
+    for (int h : {32, 64, 128, 256, 320, 384}) {
+        const long long t = (M + h - 1) / h;
+        if (h < nt && h < 256) continue;   // shorter tiles than the rows only above 256
+        if (h > nt && h > 32) continue;
+        const double kb_us = h <= 64 ? 0.40 : (h <= 128 ? 0.45 : (h <= 256 ? 0.53 : (h <= 320 ? 0.61 : 0.69)));
+        for (int ks = 1; ks <= 8; ks *= 2) {
+            const long long ctas = t * wtiles * ks;
+            const int kps = (((kblocks + ks - 1) / ks) + 3) & ~3;
+            // the parked tile has to fit the token stages, whole 256-value blocks per split, none empty
+            if (ks > 1 && (h > 256 || ctas > (ks == 2 ? sms : sms - sms / 8) || (ks - 1) * kps >= kblocks)) continue;
+            const double us = static_cast<double>((ctas + sms - 1) / sms) * kps * kb_us + (ks > 1 ? 3.0 + 0.01 * h : 0.0);
+            if (us < best_us) {
+                best_us = us;
+                best = {h, ks};
+            }
         }
     }
     return best;
 }
 
 // rows: token rows of the whole call; t_tiles: dense tile count or the tile map's capacity.
-Plan make_plan(long long rows, int nt, int t_tiles, int N, int K, bool allow_split, bool staged) {
+Plan make_plan(long long rows, int nt, int t_tiles, int N, int K, int ksplit, bool staged) {
     Plan p = {};
     p.nt = nt;
     const int stage_bytes = nt * 128;
@@ -1023,27 +1029,10 @@ Plan make_plan(long long rows, int nt, int t_tiles, int N, int K, bool allow_spl
     p.t_tiles = t_tiles;
     p.n_wtiles = (N + WM - 1) / WM;
     const int kblocks = (K + BK - 1) / BK;
-    p.ksplit = 1;
-    if (allow_split) {
-        // split K until every SM has an item, keeping at least 8 K blocks per split
-        const int items = p.t_tiles * p.n_wtiles;
-        const int sms = sm_count();
-        int want = (sms + items - 1) / items;
-        const int cap = kblocks / 8 > 0 ? kblocks / 8 : 1;
-        if (want > cap) want = cap;
-        // the last arrival adds ksplit partial tiles; keep that short next to the main loop
-        const int most = nt <= 32 ? 16 : (nt <= 64 ? 4 : (nt <= 128 ? 2 : 1));
-        if (want > most) want = most;
-        if (want > 1) p.ksplit = want;
-    }
-    p.kb_per_split = (kblocks + p.ksplit - 1) / p.ksplit;
+    p.kb_per_split = (kblocks + ksplit - 1) / ksplit;
     p.kb_per_split = (p.kb_per_split + 3) & ~3;  // splits cover whole 256-value blocks
-    p.ksplit = (kblocks + p.kb_per_split - 1) / p.kb_per_split;  // no empty splits
+    p.ksplit = ksplit;
     p.x_bytes = align256(static_cast<size_t>(rows) * K * 2);
-    if (p.ksplit > 1) {
-        p.partial_bytes = align256(static_cast<size_t>(p.t_tiles) * p.n_wtiles * p.ksplit * WM * nt * 4);
-        p.counter_bytes = align256(static_cast<size_t>(p.t_tiles) * p.n_wtiles * 4 * 4);
-    }
     return p;
 }
 
@@ -1058,7 +1047,25 @@ int launch_fused_t(const CUtensorMap& tmX, const FusedArgs& a, cudaStream_t s) {
                                           227 * 1024));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    const long long items = static_cast<long long>(a.t_tiles) * a.ksplit * a.n_wtiles;
+    const long long items = static_cast<long long>(a.t_tiles) * a.n_wtiles;
+    if (a.ksplit > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(items * a.ksplit));
+        cfg.blockDim = dim3(kFusedThreads);
+        cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = static_cast<unsigned>(a.ksplit);
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc_fused_kernel<T>, tmX, a));
+        return LSG_OK;
+    }
     int grid = sm_count();
     if (grid > items) grid = static_cast<int>(items);
     if (grid < 1) grid = 1;
@@ -1111,8 +1118,7 @@ bool tc_fused_available(int type) {
 bool tc_fused_forced() { return env_mode() >= 2; }
 
 size_t tc_fused_dense_scratch_bytes(int M, int N, int K) {
-    const int nt = pick_nt(M);
-    return make_plan(M, nt, (M + nt - 1) / nt, N, K, true, false).total();
+    return make_plan(M, 32, (M + 31) / 32, N, K, 1, false).total();
 }
 
 // Token rows per tile of a grouped call, from the average rows per expert.  Routed batches
@@ -1142,7 +1148,7 @@ int tc_fused_grouped_tile_m(long long T, int E) {
 
 size_t tc_fused_grouped_scratch_bytes(long long T, int E, int N, int K) {
     const int nt = tc_fused_grouped_tile_m(T, E);
-    return make_plan(T, nt, static_cast<int>((T + nt - 1) / nt) + E, N, K, false, false).total();
+    return make_plan(T, nt, static_cast<int>((T + nt - 1) / nt) + E, N, K, 1, false).total();
 }
 
 // Dense: C[M, N] (ldc) = x . W^T with W packed GGUF rows.
@@ -1150,8 +1156,9 @@ int tc_fused_dense(int type, int M, int N, int K, const void* A_bf16, const void
                    int out_dtype, void* ws, size_t ws_bytes, cudaStream_t s, const MmqOutputs* outs) {
     if (M == 0 || N == 0) return LSG_OK;
     if (K % 32 != 0) return fail(LSG_ERR_UNSUPPORTED, "gguf fused mmq: K must be a multiple of 32");
-    const int nt = pick_nt(M);
-    const Plan p = make_plan(M, nt, (M + nt - 1) / nt, N, K, true, staged_decoder(type));
+    const DenseCut cut = dense_cut(M, N, K);
+    const int nt = cut.nt;
+    const Plan p = make_plan(M, nt, (M + nt - 1) / nt, N, K, cut.ksplit, staged_decoder(type));
     if (!ws || ws_bytes < p.total())
         return fail(LSG_ERR_WORKSPACE, "gguf_mmq: workspace too small (have %zu, need %zu)",
                     ws ? ws_bytes : size_t(0), p.total());
@@ -1159,12 +1166,8 @@ int tc_fused_dense(int type, int M, int N, int K, const void* A_bf16, const void
         return fail(LSG_ERR_ALIGNMENT, "gguf_mmq: workspace must be 256-byte aligned");
     uint8_t* wsb = static_cast<uint8_t*>(ws);
     __half* x16 = reinterpret_cast<__half*>(wsb);
-    float* partial = reinterpret_cast<float*>(wsb + p.x_bytes);
-    unsigned int* counters = reinterpret_cast<unsigned int*>(wsb + p.x_bytes + p.partial_bytes);
-    const int n_counters = p.ksplit > 1 ? p.t_tiles * p.n_wtiles * 4 : 0;
     int rc = launch_x_prep<false>(static_cast<const __nv_bfloat16*>(A_bf16), x16, M, K,
-                                  n_counters ? counters : static_cast<unsigned int*>(nullptr), n_counters, nullptr,
-                                  nullptr, 1, s);
+                                  nullptr, nullptr, 1, s);
     if (rc != LSG_OK) return rc;
     CUtensorMap tmX;
     rc = make_map(&tmX, x16, M, K, p.box_rows);
@@ -1179,7 +1182,6 @@ int tc_fused_dense(int type, int M, int N, int K, const void* A_bf16, const void
     a.K = K; a.N = N; a.M = M;
     a.nt = nt; a.tile_rows = balanced_tile_rows(M, nt); a.box_rows = p.box_rows; a.a_col_base = p.a_col_base; a.n_wtiles = p.n_wtiles; a.t_tiles = p.t_tiles; a.stages = p.stages; a.raw_depth = p.raw_depth; a.raw_bytes = p.raw_bytes;
     a.ksplit = p.ksplit; a.kb_per_split = p.kb_per_split;
-    a.partial = partial; a.counters = counters;
     a.status = device_status_word();
 #ifdef LSG_TCF_EXP
     a.dbg = getenv("LSG_TCF_EXP") ? atoi(getenv("LSG_TCF_EXP")) : 0;
@@ -1193,8 +1195,7 @@ int tc_fused_dense(int type, int M, int N, int K, const void* A_bf16, const void
 // back in the epilogue.  Only elements more than 2^28 below their row's largest magnitude lose
 // bits, which is below what fp32 accumulation resolves.
 size_t tc_fused_bf16_scratch_bytes(int M, int N, int K) {
-    const int nt = pick_nt(M);
-    return make_plan(M, nt, (M + nt - 1) / nt, N, K, true, false).total() + align256(static_cast<size_t>(M) * 4);
+    return make_plan(M, 32, (M + 31) / 32, N, K, 1, false).total() + align256(static_cast<size_t>(M) * 4);
 }
 
 int tc_fused_dense_bf16(int type, int M, int N, int K, const void* A_bf16, const void* W, void* C, int ldc,
@@ -1203,8 +1204,9 @@ int tc_fused_dense_bf16(int type, int M, int N, int K, const void* A_bf16, const
     if (K % 32 != 0) return fail(LSG_ERR_UNSUPPORTED, "gguf_gemm_bf16: K must be a multiple of 32");
     if (reinterpret_cast<uintptr_t>(A_bf16) & 15)
         return fail(LSG_ERR_ALIGNMENT, "gguf_gemm_bf16: activations must be 16-byte aligned");
-    const int nt = pick_nt(M);
-    const Plan p = make_plan(M, nt, (M + nt - 1) / nt, N, K, true, staged_decoder(type));
+    const DenseCut cut = dense_cut(M, N, K);
+    const int nt = cut.nt;
+    const Plan p = make_plan(M, nt, (M + nt - 1) / nt, N, K, cut.ksplit, staged_decoder(type));
     const size_t need = p.total() + align256(static_cast<size_t>(M) * 4);
     if (!ws || ws_bytes < need)
         return fail(LSG_ERR_WORKSPACE, "gguf_gemm_bf16: workspace too small (have %zu, need %zu)",
@@ -1213,14 +1215,10 @@ int tc_fused_dense_bf16(int type, int M, int N, int K, const void* A_bf16, const
         return fail(LSG_ERR_ALIGNMENT, "gguf_gemm_bf16: workspace must be 256-byte aligned");
     uint8_t* wsb = static_cast<uint8_t*>(ws);
     __half* x16 = reinterpret_cast<__half*>(wsb);
-    float* partial = reinterpret_cast<float*>(wsb + p.x_bytes);
-    unsigned int* counters = reinterpret_cast<unsigned int*>(wsb + p.x_bytes + p.partial_bytes);
     float* row_scale = reinterpret_cast<float*>(wsb + p.total());
-    const int n_counters = p.ksplit > 1 ? p.t_tiles * p.n_wtiles * 4 : 0;
-    // one warp per activation row; the first CTAs also zero the split-K counters
+    // one warp per activation row
     LSG_CUDA_TRY(launch_kernel(x_rows_to_f16_kernel, dim3(static_cast<unsigned>((M + 7) / 8)), dim3(256), 0, s, true,
-                               static_cast<const __nv_bfloat16*>(A_bf16), x16, row_scale, M, K,
-                               n_counters ? counters : static_cast<unsigned int*>(nullptr), n_counters));
+                               static_cast<const __nv_bfloat16*>(A_bf16), x16, row_scale, M, K));
     CUtensorMap tmX;
     int rc = make_map(&tmX, x16, M, K, p.box_rows);
     if (rc != LSG_OK) return rc;
@@ -1232,7 +1230,6 @@ int tc_fused_dense_bf16(int type, int M, int N, int K, const void* A_bf16, const
     a.nt = nt; a.tile_rows = balanced_tile_rows(M, nt); a.box_rows = p.box_rows; a.a_col_base = p.a_col_base; a.n_wtiles = p.n_wtiles; a.t_tiles = p.t_tiles; a.stages = p.stages;
     a.raw_depth = p.raw_depth; a.raw_bytes = p.raw_bytes;
     a.ksplit = p.ksplit; a.kb_per_split = p.kb_per_split;
-    a.partial = partial; a.counters = counters;
     a.row_scale = row_scale;
     a.status = device_status_word();
 #ifdef LSG_TCF_EXP
@@ -1249,12 +1246,12 @@ int tc_fused_grouped(int type, int T, int E, int N, int K, const void* A_bf16, c
                      cudaStream_t s) {
     if (T == 0 || N == 0) return LSG_OK;
     if (K % 32 != 0) return fail(LSG_ERR_UNSUPPORTED, "gguf fused grouped mmq: K must be a multiple of 32");
-    const Plan p = make_plan(T, tile_m, t_max, N, K, false, staged_decoder(type));
+    const Plan p = make_plan(T, tile_m, t_max, N, K, 1, staged_decoder(type));
     if (!scratch || scratch_bytes < p.total())
         return fail(LSG_ERR_WORKSPACE, "gguf grouped mmq: scratch too small (have %zu, need %zu)",
                     scratch ? scratch_bytes : size_t(0), p.total());
     __half* x16 = static_cast<__half*>(scratch);
-    int rc = launch_x_prep<false>(static_cast<const __nv_bfloat16*>(A_bf16), x16, T, K, nullptr, 0, expert_offsets + E,
+    int rc = launch_x_prep<false>(static_cast<const __nv_bfloat16*>(A_bf16), x16, T, K, expert_offsets + E,
                                   nullptr, 1, s);
     if (rc != LSG_OK) return rc;
     CUtensorMap tmX;
@@ -1302,11 +1299,11 @@ int tc_fused_moe_ffn(int type, int T, int E, int H, int I, const void* A_bf16, c
     const int qk = gguf_block_values(type), qb = gguf_block_bytes(type);
 
     // gate | up
-    int rc = launch_x_prep<false>(static_cast<const __nv_bfloat16*>(A_bf16), x16, T, H, nullptr, 0, expert_offsets + E,
+    int rc = launch_x_prep<false>(static_cast<const __nv_bfloat16*>(A_bf16), x16, T, H, expert_offsets + E,
                                   perm, top_k, s, expert_offsets);
     if (rc != LSG_OK) return rc;
     CUtensorMap tmX;
-    Plan p = make_plan(T, tile_m, t_max, I, H, false, staged);
+    Plan p = make_plan(T, tile_m, t_max, I, H, 1, staged);
     rc = make_map(&tmX, x16, T, H, p.box_rows);
     if (rc != LSG_OK) return rc;
     FusedArgs a = {};
@@ -1326,10 +1323,10 @@ int tc_fused_moe_ffn(int type, int T, int E, int H, int I, const void* A_bf16, c
     if (rc != LSG_OK) return rc;
 
     // SwiGLU + preparation, then down
-    rc = launch_x_prep<true>(gu, act16, T, I, nullptr, 0, expert_offsets + E, nullptr, 1, s, expert_offsets);
+    rc = launch_x_prep<true>(gu, act16, T, I, expert_offsets + E, nullptr, 1, s, expert_offsets);
     if (rc != LSG_OK) return rc;
     CUtensorMap tmA;
-    p = make_plan(T, tile_m, t_max, H, I, false, staged);
+    p = make_plan(T, tile_m, t_max, H, I, 1, staged);
     rc = make_map(&tmA, act16, T, I, p.box_rows);
     if (rc != LSG_OK) return rc;
     FusedArgs b = {};

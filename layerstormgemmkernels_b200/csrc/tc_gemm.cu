@@ -530,41 +530,22 @@ weights_to_f16_staged_kernel(const uint8_t* __restrict__ W, const void* const* _
 }
 
 // bf16 x[M,K] -> fp16 of the Q8_1 round trip: d_h * rn(x / d) with d = amax/127 per 32
-// values and d_h its fp16 rounding (what the integer paths multiply by).  Four lanes per
-// block, eight values per lane.
+// values and d_h its fp16 rounding (what the integer paths multiply by).  Two lanes per
+// block, sixteen values per lane.
 __global__ void __launch_bounds__(256)
 x_q8_1_roundtrip_f16_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ out, long long n_blocks) {
     pdl_launch_dependents();
     pdl_wait_prior();
     const long long task = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-    const bool live = task < n_blocks * 4;
+    const bool live = task < n_blocks * 2;
     const long long tk = live ? task : 0;
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(x) + tk);
-    float v[8];
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        v[2 * i] = __uint_as_float(w[i] << 16);
-        v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(x) + 2 * tk), b = __ldg(reinterpret_cast<const uint4*>(x) + 2 * tk + 1);
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t p[8];
+    q8_roundtrip16(w, 0xffffffffu, p);
     if (!live) return;
-    const float d = amax / 127.0f;
-    const float rcp = (amax == 0.0f) ? 0.0f : 1.0f / d;
-    const float dh = __half2float(__float2half(d));
-    float r[8];
-    q8_roundtrip8(v, d, rcp, dh, r);
-    uint32_t p[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __half2 hv = __floats2half2_rn(r[2 * i], r[2 * i + 1]);
-        p[i] = *reinterpret_cast<const uint32_t*>(&hv);
-    }
-    reinterpret_cast<uint4*>(out)[tk] = make_uint4(p[0], p[1], p[2], p[3]);
+    reinterpret_cast<uint4*>(out)[2 * tk] = make_uint4(p[0], p[1], p[2], p[3]);
+    reinterpret_cast<uint4*>(out)[2 * tk + 1] = make_uint4(p[4], p[5], p[6], p[7]);
 }
 
 // ---------------------------------------------------------------------------
@@ -621,7 +602,7 @@ int weights_to_f16(int type, const void* W, const void* const* B_ptrs, const int
 int x_to_f16(const void* x_bf16, __half* out, long long rows, int K, cudaStream_t s) {
     const long long nb = rows * (K / 32);
     if (nb == 0) return LSG_OK;
-    LSG_CUDA_TRY(launch_kernel(x_q8_1_roundtrip_f16_kernel, dim3(static_cast<unsigned>((nb * 4 + 255) / 256)), dim3(256),
+    LSG_CUDA_TRY(launch_kernel(x_q8_1_roundtrip_f16_kernel, dim3(static_cast<unsigned>((nb * 2 + 255) / 256)), dim3(256),
                                0, s, true, static_cast<const __nv_bfloat16*>(x_bf16), out, nb));
     return LSG_OK;
 }

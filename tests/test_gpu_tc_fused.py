@@ -68,6 +68,26 @@ def test_fused_k_not_a_multiple_of_64(ops, weight_path, name):
     assert np.abs(got - ref).max() <= TOL_TC * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (9, 130, 4352),     # K in uneven parts, a weight tile with two live rows
+    (65, 1000, 2048),   # 128-row tile with one row more than half
+    (200, 520, 4096),   # 256-row tile
+    (256, 300, 8448),
+    (300, 260, 4096),   # two token tiles sharing the rows evenly
+    (640, 130, 1024),   # several token tiles, short K
+])
+def test_fused_q4k_cluster_split_k(ops, M, N, K):
+    """Tiles whose K range is shared by the CTAs of a cluster, for every tile height that can be:
+    against the oracle (fp16 operands: TOL_TC), bf16 results the rounding of the fp32 ones, same
+    bits on every run."""
+    A, W, Wd = make_case("Q4_K", M, N, K, seed=M)
+    ref = oracle.mmvq(T["Q4_K"], oracle.quantize_q8_1(bits_of(A)), W, K)
+    got = ops.gguf_mmq(A, Wd, T["Q4_K"], N, K, out_dtype=torch.float32)
+    assert np.abs(got.cpu().numpy() - ref).max() <= TOL_TC * np.abs(ref).max()
+    assert torch.equal(got, ops.gguf_mmq(A, Wd, T["Q4_K"], N, K, out_dtype=torch.float32))
+    assert torch.equal(got.to(torch.bfloat16), ops.gguf_mmq(A, Wd, T["Q4_K"], N, K))
+
+
 @pytest.mark.parametrize("M", [2, 4, 8, 16, 40])
 @pytest.mark.parametrize("N,K", [(1024, 4096), (4096, 4096), (512, 14336)])
 def test_fused_q4k_decode_batches_split_k(ops, weight_path, M, N, K):
