@@ -122,7 +122,8 @@ MmvqTune mmvq_tuning();  // current process-wide geometry, clamped to valid rang
 #define MMVQ_FN(name) LSG_CAT(LSG_CAT(mmvq_, name), LSG_CAT(_t, LSG_MMVQ_TYPE))
 #define LSG_DECLARE_MMVQ(id)                                         \
     int mmvq_launch_t##id(MmvqArgs a, const MmvqTune& tn, cudaStream_t stream, bool pdl); \
-    int mmvq_max_rows_t##id(int K);
+    int mmvq_max_rows_t##id(int K);                                                       \
+    bool mmvq_eight_rows_t##id(int K);
 LSG_DECLARE_MMVQ(0) LSG_DECLARE_MMVQ(1) LSG_DECLARE_MMVQ(2) LSG_DECLARE_MMVQ(3)
 LSG_DECLARE_MMVQ(4) LSG_DECLARE_MMVQ(5) LSG_DECLARE_MMVQ(6) LSG_DECLARE_MMVQ(7)
 

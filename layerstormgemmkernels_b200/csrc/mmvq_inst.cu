@@ -212,6 +212,12 @@ int MMVQ_FN(max_rows)(int K) {
     return rows < 1 ? 0 : rows;
 }
 
+// Whether eight batch rows of this K go to the tensor-core mat-vec.
+bool MMVQ_FN(eight_rows)(int K) {
+    MmaCut c = {};
+    return MmaDec<T>::kHas && mma_min_rows() <= kMmaCols && mma_cut_k(c, K, 8, kMmaSliceBlocks);
+}
+
 int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool pdl) {
     using F = Fmt<T>;
     a.row_bytes = (a.K / F::VALS) * F::BYTES;

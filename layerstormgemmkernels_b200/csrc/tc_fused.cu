@@ -884,8 +884,8 @@ int launch_x_prep(const __nv_bfloat16* x, __half* out, long long rows, int K, co
     const int ppr = K / 16;
     // two rows per thread once there are enough rows to fill the GPU that way; below that, blocks of
     // 64 threads, so that a few rows spread over the SMs (48 x 4096: 1 us less than in blocks of 256)
-    const bool rb2 = rows * ppr >= 2ll * 256 * 2 * sm_count();
-    const int bmax = rb2 ? 256 : 64;
+    const bool rb2 = rows * ppr >= 16ll * 256 * 2 * sm_count();
+    const int bmax = rows * ppr >= 2ll * 256 * 2 * sm_count() ? 256 : 64;
     const int bx = ppr < bmax ? ppr : bmax;
     const int by = bmax / bx;
     const int gy = (ppr + bx - 1) / bx;

@@ -162,6 +162,27 @@ def test_mmvq_tensor_core_edges(ops, name, M, N, K):
     assert torch.equal(both[0], ops.gguf_mmvq(A, W2, t, 50, K, out_dtype=torch.float32))
 
 
+@pytest.mark.parametrize("name", ["Q5_K", "Q6_K", "Q8_0", "Q4_0"])
+@pytest.mark.parametrize("M", [9, 13, 24])
+def test_few_rows_of_expanded_types_take_the_matvec(ops, name, M):
+    """Up to 24 rows of the types without a decoder in the tensor-core GEMM run as mat-vec passes
+    of eight rows: exact integer sums, so the mat-vec's tolerance holds; 25 rows and an unaligned
+    matrix keep the GEMM and its 1e-3."""
+    t, N, K = T[name], 300, 4352
+    A = torch.randn(M + 1, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
+    W = Q.random_gguf_weight(name, N, K, seed=M)
+    Wd = torch.from_numpy(W).cuda()
+    ref = oracle.mmvq(t, oracle.quantize_q8_1(bf16_bits(A)), W, K)
+    got = ops.gguf_mmq(A[:M], Wd, t, N, K, out_dtype=torch.float32).cpu().numpy()
+    assert rel_err(got, ref[:M]) <= TOL_F32
+    assert rel_err(ops.gguf_mmvq(A, Wd, t, N, K, out_dtype=torch.float32).cpu().numpy(), ref) <= TOL_F32
+    off = torch.zeros(W.size + 1, dtype=torch.uint8, device="cuda")
+    off[1:] = Wd.flatten()
+    assert rel_err(ops.gguf_mmq(A[:M], off[1:], t, N, K, out_dtype=torch.float32).cpu().numpy(), ref[:M]) <= 1e-3
+    if M == 24:
+        assert rel_err(ops.gguf_mmq(A, Wd, t, N, K, out_dtype=torch.float32).cpu().numpy(), ref) <= 1e-3
+
+
 def test_mmvq_bit_deterministic(ops):
     """tests/test_gguf_mmvq.py:91-103."""
     N, K = 640, 1024
