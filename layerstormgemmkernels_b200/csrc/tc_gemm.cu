@@ -26,7 +26,10 @@
 //               512 TMEM columns) let the epilogue of tile i overlap the MMAs of tile i+1.
 // Work items are (m-tile, n-tile) pairs; m-tiles come either from a dense problem or from
 // the device-built tile map of the grouped problem (routing.cu), so expert routing never
-// touches the host.  Every mbarrier wait is time-limited; after a time-out all roles leave
+// touches the host.  A dense problem with fewer tiles than half the SMs shares the K range of a tile
+// among the CTAs of a cluster, which add their fp32 tiles in rank order through distributed shared
+// memory (4096 x 14336 with up to 128 rows is 16 tiles: the GEMM took 90 us of such a call's 126).
+// Every mbarrier wait is time-limited; after a time-out all roles leave
 // their loops, TMEM is freed, and the status word says so.
 #include "common.cuh"
 #include "formats.cuh"
@@ -71,7 +74,12 @@ struct TcArgs {
     const int* tile_mstart;
     const int* expert_offsets;
     unsigned int* status;
+    int ksplit;               // CTAs of a cluster sharing a tile's K range (1: no cluster)
+    int kb_per_split;         // K blocks of each
 };
+
+constexpr int kParkRow = BN * 4 + 16;   // bytes of a parked accumulator row (16 more: banks)
+static_assert(BM * kParkRow <= kStages * kStageBytes, "the parked tile takes the ring's place");
 
 // ---------------------------------------------------------------------------
 // The GEMM kernel
@@ -112,8 +120,11 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 
     pdl_wait_prior();  // operands were produced by the preparation kernels before this one
 
-    const int kblocks = (a.K + BK - 1) / BK;
     const int total = a.m_tiles * a.n_tiles;
+    const int rank = static_cast<int>(blockIdx.x) % a.ksplit;   // of this CTA in its cluster
+    const int w0 = static_cast<int>(blockIdx.x) / a.ksplit, w_step = static_cast<int>(gridDim.x) / a.ksplit;
+    const int kb0 = rank * a.kb_per_split;
+    const int kb1 = min((a.K + BK - 1) / BK, kb0 + a.kb_per_split);
 
     if (warp == 4) {
         // ------------------------------ TMA producer ------------------------------
@@ -122,7 +133,7 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             int s = 0;
             uint32_t lap = 0;
             bool ok = true;
-            for (int w = blockIdx.x; w < total && ok && !*abort_flag; w += gridDim.x) {
+            for (int w = w0; w < total && ok && !*abort_flag; w += w_step) {
                 const int t = w % a.m_tiles, j = w / a.m_tiles;
                 int mstart = t * BM, brow0 = j * BN;
                 if (a.tile_expert) {
@@ -131,7 +142,7 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     mstart = a.tile_mstart[t];
                     brow0 = e * a.N + j * BN;
                 }
-                for (int kb = 0; kb < kblocks; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (lap > 0)
                         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], (lap - 1) & 1, a.status, kDevWaitEmpty));
                     if (!ok) break;
@@ -160,7 +171,7 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         int s = 0, tile_i = 0;
         uint32_t lap = 0;
         bool ok = true;
-        for (int w = blockIdx.x; w < total && ok && !*abort_flag; w += gridDim.x) {
+        for (int w = w0; w < total && ok && !*abort_flag; w += w_step) {
             const int t = w % a.m_tiles;
             if (a.tile_expert && a.tile_expert[t] < 0) continue;
             const int ab = tile_i & 1;
@@ -169,7 +180,7 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             if (!ok) break;
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + ab * BN;
-            for (int kb = 0; kb < kblocks; ++kb) {
+            for (int kb = kb0; kb < kb1; ++kb) {
                 ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], lap & 1, a.status, kDevWaitFull));
                 if (!ok) break;
                 tc_fence_after();
@@ -181,7 +192,7 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     for (int k = 0; k < BK / 16; ++k) {
                         // 16 fp16 = 32 bytes further along K inside the swizzle atom: +2 in
                         // the (address >> 4) field of the descriptors
-                        tc_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        tc_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
                     }
                     tc_commit(&empty[s]);  // the stage is free once these MMAs have read it
                 }
@@ -200,7 +211,7 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     } else {
         // ------------------------------ epilogue (warps 0-3) ----------------------
         int tile_i = 0;
-        for (int w = blockIdx.x; w < total && !*abort_flag; w += gridDim.x) {
+        for (int w = w0; w < total && !*abort_flag; w += w_step) {
             const int t = w % a.m_tiles, j = w / a.m_tiles;
             int mstart = t * BM, mend = a.M;
             if (a.tile_expert) {
@@ -218,6 +229,21 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                 break;
             }
             tc_fence_after();
+            if (a.ksplit > 1) {
+                // split K: park the tile in the ring's place, the sum follows after the cluster barrier
+                const uint32_t mine = smem_u32(smem) + static_cast<uint32_t>((warp * 32 + lane) * kParkRow);
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + ab * BN + c, r);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(mine + (c + 4 * q) * 4), "r"(r[4 * q]),
+                                     "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3])
+                                     : "memory");
+                }
+                break;   // one tile per cluster
+            }
             const int row = mstart + warp * 32 + lane;
             const bool row_ok = row < mend;
             const int n0 = j * BN;
@@ -352,6 +378,40 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     if (warp == 5) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
+    }
+    if (a.ksplit > 1) {
+        // Every thread of every CTA of the cluster comes here, after a time-out too.
+        __syncwarp();
+        cluster_sync();
+        const int m0 = (w0 % a.m_tiles) * BM, n0 = (w0 / a.m_tiles) * BN;
+        const int live = min(BM, a.M - m0);
+        const int vecs = min(BN, a.N - n0) >> 2;   // 4-column pieces per row (N % 8 == 0)
+        const float alpha = a.alphas ? a.alphas[0] : a.alpha_host;
+        const uint32_t base = smem_u32(smem);
+        for (int i = rank * kTcThreads + threadIdx.x; i < live * vecs; i += a.ksplit * kTcThreads) {
+            const int r = i / vecs, c = (i - r * vecs) * 4;
+            const uint32_t at = base + static_cast<uint32_t>(r * kParkRow + c * 4);
+            float4 v = ld_cluster_f4(at, 0);
+            for (int k = 1; k < a.ksplit; ++k) {
+                const float4 p = ld_cluster_f4(at, k);
+                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            }
+            v.x *= alpha; v.y *= alpha; v.z *= alpha; v.w *= alpha;
+            const size_t o = static_cast<size_t>(m0 + r) * a.ldc + n0 + c;
+            if (a.out_f32 == LSG_DTYPE_F32) {
+                *reinterpret_cast<float4*>(static_cast<float*>(a.C) + o) = v;
+            } else if (a.out_f32 == LSG_DTYPE_F16) {
+                const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.C) + o) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            } else {
+                const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.C) + o) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            }
+        }
+        __syncwarp();
+        cluster_sync();   // no CTA leaves while a peer still reads its tile
     }
 }
 
@@ -551,13 +611,53 @@ x_q8_1_roundtrip_f16_kernel(const __nv_bfloat16* __restrict__ x, __half* __restr
 // ---------------------------------------------------------------------------
 // Host
 // ---------------------------------------------------------------------------
-int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const TcArgs& a, int max_items, cudaStream_t s) {
+// CTAs of a cluster per tile of a dense problem: as many as are resident together, where what they
+// save (0.5 us a K block of 64 values) is more than the parked tile, the barriers and the sum cost
+// (about 4 us).  The sum stores 4-column pieces of one output matrix.
+int pick_ksplit(const TcArgs& a) {
+    if (a.tile_expert || a.n_out > 0 || a.N % 8 != 0 || a.ldc != a.N || (reinterpret_cast<uintptr_t>(a.C) & 15)) return 1;
+    const int sms = sm_count(), items = a.m_tiles * a.n_tiles, kblocks = (a.K + BK - 1) / BK;
+    int best = 1;
+    double best_us = kblocks * 0.5;
+    for (int ks = 2; ks <= 8; ks *= 2) {
+        const int kps = (kblocks + ks - 1) / ks;
+        if (static_cast<long long>(items) * ks > (ks == 2 ? sms : sms - sms / 8) || (ks - 1) * kps >= kblocks) break;
+        const double us = kps * 0.5 + 4.0;
+        if (us < best_us) {
+            best = ks;
+            best_us = us;
+        }
+    }
+    return best;
+}
+
+int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, TcArgs a, int max_items, cudaStream_t s) {
     static bool configured[64] = {};
     int dev = 0;
     LSG_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev]) {
         LSG_CUDA_TRY(cudaFuncSetAttribute(tc_gemm_f16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    a.ksplit = pick_ksplit(a);
+    a.kb_per_split = ((a.K + BK - 1) / BK + a.ksplit - 1) / a.ksplit;
+    if (a.ksplit > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(max_items * a.ksplit));
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = kTcSmem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = static_cast<unsigned>(a.ksplit);
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc_gemm_f16_kernel, tmA, tmB, a));
+        return LSG_OK;
     }
     int grid = sm_count();
     if (grid > max_items) grid = max_items;
@@ -634,10 +734,10 @@ int mmq_dense(int type, int M, int N, int K, const void* A, const void* W, void*
         return fail(LSG_ERR_WORKSPACE, "gguf_mmq: workspace too small (have %zu, need %zu)",
                     ws ? ws_bytes : size_t(0), need);
     if (reinterpret_cast<uintptr_t>(ws) & 255) return fail(LSG_ERR_ALIGNMENT, "gguf_mmq: workspace must be 256-byte aligned");
-    // A few rows: expanding the weights costs more than passing over them once per eight rows with
-    // the tensor-core mat-vec, whose sums are exact.  Q6_K 4096 x 14336, us: 12 rows 124.7 expanded
-    // (128.9 at 100 rows), about 26 per eight rows on the mat-vec; 14336 x 4096 72 and 19.
-    if (!outs && M <= 24 && mmvq_eight_rows(type, K) && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
+    // A few rows: expanding the weights costs more than passing over them once or twice with the
+    // tensor-core mat-vec, eight rows at a time, whose sums are exact.  Q6_K 4096 x 14336, us:
+    // 12 rows 50.8, 24 rows 77.5 on the mat-vec, 48 rows 73.1 expanded; 14336 x 4096: 38.6, 68.7, 60.3.
+    if (!outs && M <= 16 && mmvq_eight_rows(type, K) && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(A) & 15) == 0) {
         const int rc = quantize_q8_1(A, ws, M, K, s, true);
         if (rc != LSG_OK) return rc;

@@ -163,10 +163,10 @@ def test_mmvq_tensor_core_edges(ops, name, M, N, K):
 
 
 @pytest.mark.parametrize("name", ["Q5_K", "Q6_K", "Q8_0", "Q4_0"])
-@pytest.mark.parametrize("M", [9, 13, 24])
+@pytest.mark.parametrize("M", [9, 13, 16])
 def test_few_rows_of_expanded_types_take_the_matvec(ops, name, M):
-    """Up to 24 rows of the types without a decoder in the tensor-core GEMM run as mat-vec passes
-    of eight rows: exact integer sums, so the mat-vec's tolerance holds; 25 rows and an unaligned
+    """Up to 16 rows of the types without a decoder in the tensor-core GEMM run as mat-vec passes
+    of eight rows: exact integer sums, so the mat-vec's tolerance holds; 17 rows and an unaligned
     matrix keep the GEMM and its 1e-3."""
     t, N, K = T[name], 300, 4352
     A = torch.randn(M + 1, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
@@ -179,7 +179,7 @@ def test_few_rows_of_expanded_types_take_the_matvec(ops, name, M):
     off = torch.zeros(W.size + 1, dtype=torch.uint8, device="cuda")
     off[1:] = Wd.flatten()
     assert rel_err(ops.gguf_mmq(A[:M], off[1:], t, N, K, out_dtype=torch.float32).cpu().numpy(), ref[:M]) <= 1e-3
-    if M == 24:
+    if M == 16:
         assert rel_err(ops.gguf_mmq(A, Wd, t, N, K, out_dtype=torch.float32).cpu().numpy(), ref) <= 1e-3
 
 

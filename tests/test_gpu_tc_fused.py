@@ -69,6 +69,22 @@ def test_fused_k_not_a_multiple_of_64(ops, weight_path, name):
 
 
 @pytest.mark.parametrize("M,N,K", [
+    (40, 264, 4352),    # K in uneven parts, a second column tile eight wide
+    (129, 512, 4096),   # a second row tile with one row
+    (300, 520, 2048),
+    (100, 260, 1024),   # N not a multiple of 8: never split
+])
+def test_expanded_types_cluster_split_k(ops, M, N, K):
+    """The same in the GEMM over expanded weights."""
+    A, W, Wd = make_case("Q6_K", M, N, K, seed=M)
+    ref = oracle.mmvq(T["Q6_K"], oracle.quantize_q8_1(bits_of(A)), W, K)
+    got = ops.gguf_mmq(A, Wd, T["Q6_K"], N, K, out_dtype=torch.float32)
+    assert np.abs(got.cpu().numpy() - ref).max() <= TOL_TC * np.abs(ref).max()
+    assert torch.equal(got, ops.gguf_mmq(A, Wd, T["Q6_K"], N, K, out_dtype=torch.float32))
+    assert torch.equal(got.to(torch.bfloat16), ops.gguf_mmq(A, Wd, T["Q6_K"], N, K))
+
+
+@pytest.mark.parametrize("M,N,K", [
     (9, 130, 4352),     # K in uneven parts, a weight tile with two live rows
     (65, 1000, 2048),   # 128-row tile with one row more than half
     (200, 520, 4096),   # 256-row tile
