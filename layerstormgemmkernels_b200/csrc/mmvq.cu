@@ -128,7 +128,8 @@ int mmvq_q8_1(int type, int M, int N, int K, const void* W, const void* xq, void
     // The dp4a kernel multiplies eight rows at a time however many one launch holds; where the
     // tensor-core kernel takes eight rows, launches of eight are faster (38.4 against 18.1 us a
     // pass over 4096 x 14336 of Q4_K).
-    if (M > 8 && mmvq_eight_rows(type, K)) batch = 8;
+    const bool eights = M > 8 && mmvq_eight_rows(type, K);
+    if (eights) batch = 8;
     const size_t xq_row = static_cast<size_t>(K / 32) * kQ8_1Bytes;
     const size_t c_elem = out_f32 ? 4 : 2;
     for (int m0 = 0; m0 < M; m0 += batch) {
@@ -144,6 +145,7 @@ int mmvq_q8_1(int type, int M, int N, int K, const void* W, const void* xq, void
         a.ldc = ldc;
         a.out_f32 = out_f32;
         a.dep_mode = (pdl && m0 == 0) ? dep_mode : 0;   // later row batches are fully serialized launches
+        a.eights = eights ? 1 : 0;
         const int rc = dispatch_launch(type, a, stream, pdl && m0 == 0);
         if (rc != LSG_OK) return rc;
     }
@@ -176,7 +178,8 @@ int mmvq_q8_1_joined(int type, int M, int K, int n, const void* const* W, void* 
     // The dp4a kernel multiplies eight rows at a time however many one launch holds; where the
     // tensor-core kernel takes eight rows, launches of eight are faster (38.4 against 18.1 us a
     // pass over 4096 x 14336 of Q4_K).
-    if (M > 8 && mmvq_eight_rows(type, K)) batch = 8;
+    const bool eights = M > 8 && mmvq_eight_rows(type, K);
+    if (eights) batch = 8;
     const size_t xq_row = static_cast<size_t>(K / 32) * kQ8_1Bytes;
     const size_t c_elem = out_f32 ? 4 : 2;
     for (int m0 = 0; m0 < M; m0 += batch) {
@@ -202,6 +205,7 @@ int mmvq_q8_1_joined(int type, int M, int K, int n, const void* const* W, void* 
                 a.xqx[j - 1] = static_cast<const uint8_t*>(xq_each && xq_each[j] ? xq_each[j] : xq) + static_cast<size_t>(m0) * xq_row;
         }
         a.dep_mode = (pdl && m0 == 0) ? dep_mode : 0;
+        a.eights = eights ? 1 : 0;
         const int rc = dispatch_launch(type, a, stream, pdl && m0 == 0);
         if (rc != LSG_OK) return rc;
     }

@@ -60,6 +60,7 @@ struct MmvqArgs {
     // start on the SMs the previous launch has left while its last CTAs still stream - and
     // the wait is made before the CTA exits, so that launches still complete in stream order.
     int dep_mode;
+    int eights;               // part of a call of more than eight rows in passes of eight: one kernel for all its rows
 #ifdef LSG_MMVQ_TRACE
     unsigned long long* trace;  // [grid][16] nanosecond timestamps of the phases of each CTA
 #endif

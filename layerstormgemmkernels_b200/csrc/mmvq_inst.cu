@@ -221,7 +221,7 @@ bool MMVQ_FN(eight_rows)(int K) {
 int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool pdl) {
     using F = Fmt<T>;
     a.row_bytes = (a.K / F::VALS) * F::BYTES;
-    if (a.M >= mma_min_rows() && !tn_in.skip_math) {
+    if ((a.M >= mma_min_rows() || a.eights) && !tn_in.skip_math) {
         const int rc = launch_mma<T>(a, stream, pdl);
         if (rc != kMmaNotTaken) return rc;
     }

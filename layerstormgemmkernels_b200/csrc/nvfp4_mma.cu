@@ -408,11 +408,7 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int i = rank * kFThreads + threadIdx.x; i < live * vecs; i += a.ksplit * kFThreads) {
             const int r = i / vecs, c = (i - r * vecs) * 4;
             const uint32_t at = base + static_cast<uint32_t>(r * kFPartRow + c * 4);
-            float4 v = ld_cluster_f4(at, 0);
-            for (int sp = 1; sp < a.ksplit; ++sp) {
-                const float4 p = ld_cluster_f4(at, sp);
-                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-            }
+            float4 v = sum_cluster_f4(at, a.ksplit);
             v.x *= alpha; v.y *= alpha; v.z *= alpha; v.w *= alpha;
             const size_t o = static_cast<size_t>(mstart + r) * a.ldd + n0 + c;
             if (a.out_dtype == LSG_DTYPE_F32) {

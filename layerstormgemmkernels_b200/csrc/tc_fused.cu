@@ -764,11 +764,7 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
             const int n = im.wt * WM + 4 * q;
             if (n >= a.N) continue;
             const uint32_t at = base + static_cast<uint32_t>(tok * WM + 4 * q) * 4u;
-            float4 v = ld_cluster_f4(at, 0);
-            for (int k = 1; k < a.ksplit; ++k) {
-                const float4 p = ld_cluster_f4(at, k);
-                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-            }
+            float4 v = sum_cluster_f4(at, a.ksplit);
             if (a.row_scale) {
                 const float rs = __ldg(a.row_scale + im.mstart + tok);
                 v.x *= rs; v.y *= rs; v.z *= rs; v.w *= rs;

@@ -391,11 +391,7 @@ tc_gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         for (int i = rank * kTcThreads + threadIdx.x; i < live * vecs; i += a.ksplit * kTcThreads) {
             const int r = i / vecs, c = (i - r * vecs) * 4;
             const uint32_t at = base + static_cast<uint32_t>(r * kParkRow + c * 4);
-            float4 v = ld_cluster_f4(at, 0);
-            for (int k = 1; k < a.ksplit; ++k) {
-                const float4 p = ld_cluster_f4(at, k);
-                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-            }
+            float4 v = sum_cluster_f4(at, a.ksplit);
             v.x *= alpha; v.y *= alpha; v.z *= alpha; v.w *= alpha;
             const size_t o = static_cast<size_t>(m0 + r) * a.ldc + n0 + c;
             if (a.out_f32 == LSG_DTYPE_F32) {

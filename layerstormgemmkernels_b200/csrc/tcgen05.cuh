@@ -101,6 +101,25 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t ra
     return v;
 }
 
+// The sum over the ranks 0..n-1 (n <= 8) of a cluster, in rank order; all loads are under way before
+// the first addition.
+__device__ __forceinline__ float4 sum_cluster_f4(uint32_t local_addr, int n) {
+    float4 p[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (k < n) p[k] = ld_cluster_f4(local_addr, k);
+    float4 v = p[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k)
+        if (k < n) {
+            v.x += p[k].x;
+            v.y += p[k].y;
+            v.z += p[k].z;
+            v.w += p[k].w;
+        }
+    return v;
+}
+
 // Shared-memory matrix descriptor, K-major operand, 128-byte swizzle: rows of 128 bytes,
 // 8-row groups 1024 bytes apart (stride byte offset), descriptor version 1.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
