@@ -11,10 +11,11 @@
 //
 // The scales change every 128 values of K, so the accumulator is drained once per K block: eight
 // warps read it out of tensor memory and add it, times its scale, to fp32 accumulators of their
-// own, while the tensor core fills the other of two accumulators.  Per K block of a 128 x 256 tile
-// the tensor core takes 512 cycles, the operands' way through shared memory (48 KB in, 48 KB out
-// at 128 B/clk) 750, the drain about 300 of tcgen05.ld and as many issue slots of FFMA: the drain
-// hides, and 256 columns are the tile because a narrower one moves more operand bytes per product.
+// own, while the tensor core fills the other of two accumulators.  The GEMM alone takes 48 us at
+// that size, 39 with the drain left out: the bytes that come out of L2 bound it first (48 KB per K
+// block of a 128 x 256 tile at about 42 B/clk and SM, against 512 cycles of tensor time), which is
+// why 256 columns are the tile (a narrower one moves more bytes per product), the drain second.
+// Sixteen drain warps with half the columns each: 57 us.
 //   warps 0-7   drain and epilogue: warp w owns tensor-memory lanes 32 (w % 4).. (= token rows)
 //               and column half w / 4; output rows are stored as 16-byte pieces
 //   warp 8      TMA producer: one box of 128 tokens x 128 bytes, one of NC weight rows

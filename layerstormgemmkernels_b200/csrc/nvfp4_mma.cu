@@ -432,7 +432,9 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // unsplit CTA takes 0.78 us per K tile of a pair and about 0.52 us per K tile of a single output
 // tile (the bytes it pulls out of L2); splitting adds the parked tile, two cluster barriers and
 // the sum, 2 us.  The cheapest of the combinations whose CTAs are all resident at once wins; a
-// call that fills the chip without splitting keeps pairs and no cluster.
+// call that fills the chip without splitting keeps pairs and no cluster.  77 x 4096 x 14336 with its
+// quantizer, in a row of calls: 41.3 us unsplit, 38.6 in clusters of eight (host bound there); a first
+// call 92 and 77.
 struct SplitPlan {
     int tile_cols, ksplit, kt_per_split;
 };

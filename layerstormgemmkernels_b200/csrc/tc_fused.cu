@@ -807,7 +807,7 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmX, const FusedArgs a) {
 // Two lanes per 32-value block, sixteen values (two 16-byte vectors) each: the pass is bound by
 // instruction issue, and what a thread does once (the block's scale and its reciprocal, the row's
 // source, addresses) is shared by sixteen values (q8_roundtrip16 has the rest).  32768 x 2048
-// gathered rows: 59.3 us with eight values per thread.  The thread block is (vector pairs of a row,
+// gathered rows: 43.7 us, 59.3 with eight values per thread.  The thread block is (vector pairs of a row,
 // rows); every thread handles RB rows, so 2 RB (4 RB with SwiGLU) independent loads are in flight
 // per thread.  Grouped callers may hold fewer rows than the buffer they pass: the row count then
 // lives on the device (live_rows).
