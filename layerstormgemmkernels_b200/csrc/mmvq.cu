@@ -80,16 +80,16 @@ int dispatch_max_rows(int type, int K) {
 
 }  // namespace
 
-bool mmvq_eight_rows(int type, int K) {
+bool mmvq_eight_rows(int type, int M, int K) {
     switch (type) {
-        case 0: return mmvq_eight_rows_t0(K);
-        case 1: return mmvq_eight_rows_t1(K);
-        case 2: return mmvq_eight_rows_t2(K);
-        case 3: return mmvq_eight_rows_t3(K);
-        case 4: return mmvq_eight_rows_t4(K);
-        case 5: return mmvq_eight_rows_t5(K);
-        case 6: return mmvq_eight_rows_t6(K);
-        case 7: return mmvq_eight_rows_t7(K);
+        case 0: return mmvq_eight_rows_t0(M, K);
+        case 1: return mmvq_eight_rows_t1(M, K);
+        case 2: return mmvq_eight_rows_t2(M, K);
+        case 3: return mmvq_eight_rows_t3(M, K);
+        case 4: return mmvq_eight_rows_t4(M, K);
+        case 5: return mmvq_eight_rows_t5(M, K);
+        case 6: return mmvq_eight_rows_t6(M, K);
+        case 7: return mmvq_eight_rows_t7(M, K);
     }
     return false;
 }
@@ -108,8 +108,19 @@ int check_gemm_params(const char* op, const lsg_gguf_mmvq_params* p) {
     return LSG_OK;
 }
 
-// xq: Q8_1 blocks of all M rows.  ldc: output row stride.  Rows are processed
-// in batches that fit the shared-memory activation image.
+// Batch rows of one launch of a call (0: not even one row of this K fits), and which kernel all its
+// launches take.  The dp4a kernel takes as many rows as its activation image holds, a multiple of
+// eight when possible (eight rows per register pass); where the tensor-core kernel takes the call,
+// launches of eight are faster (38.4 against 18.1 us a pass over 4096 x 14336 of Q4_K).
+int rows_per_launch(int type, int M, int K, bool& eights) {
+    const int max_rows = dispatch_max_rows(type, K);
+    eights = max_rows >= 1 && g_drop_slab < 0 && !sane_tuning().skip_math && mmvq_eight_rows(type, M, K);
+    if (eights) return 8;
+    const int batch = max_rows >= 8 ? (max_rows / 8) * 8 : max_rows;
+    return batch > 32 ? 32 : batch;
+}
+
+// xq: Q8_1 blocks of all M rows.  ldc: output row stride.
 int mmvq_q8_1(int type, int M, int N, int K, const void* W, const void* xq, void* C, int ldc,
               int out_f32, cudaStream_t stream, bool pdl, const void* A_bf16, int dep_mode) {
     if (M == 0 || N == 0) return LSG_OK;
@@ -119,17 +130,10 @@ int mmvq_q8_1(int type, int M, int N, int K, const void* W, const void* xq, void
         return fail(LSG_ERR_ALIGNMENT, "gguf_mmvq: packed weight must be 16-byte aligned");
     if (!A_bf16 && (reinterpret_cast<uintptr_t>(xq) & 3))
         return fail(LSG_ERR_ALIGNMENT, "gguf_mmvq: Q8_1 buffer must be 4-byte aligned");
-    const int max_rows = dispatch_max_rows(type, K);
-    if (max_rows < 1)
+    bool eights;
+    const int batch = rows_per_launch(type, M, K, eights);
+    if (batch < 1)
         return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: K=%d too large for the shared-memory pipeline", K);
-    // Eight rows per register pass; keep batches a multiple of eight when possible.
-    int batch = max_rows >= 8 ? (max_rows / 8) * 8 : max_rows;
-    if (batch > 32) batch = 32;
-    // The dp4a kernel multiplies eight rows at a time however many one launch holds; where the
-    // tensor-core kernel takes eight rows, launches of eight are faster (38.4 against 18.1 us a
-    // pass over 4096 x 14336 of Q4_K).
-    const bool eights = M > 8 && mmvq_eight_rows(type, K);
-    if (eights) batch = 8;
     const size_t xq_row = static_cast<size_t>(K / 32) * kQ8_1Bytes;
     const size_t c_elem = out_f32 ? 4 : 2;
     for (int m0 = 0; m0 < M; m0 += batch) {
@@ -170,16 +174,10 @@ int mmvq_q8_1_joined(int type, int M, int K, int n, const void* const* W, void* 
     }
     if (!A_bf16 && (reinterpret_cast<uintptr_t>(xq) & 3))
         return fail(LSG_ERR_ALIGNMENT, "gguf_mmvq: Q8_1 buffer must be 4-byte aligned");
-    const int max_rows = dispatch_max_rows(type, K);
-    if (max_rows < 1)
+    bool eights;
+    const int batch = rows_per_launch(type, M, K, eights);
+    if (batch < 1)
         return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: K=%d too large for the shared-memory pipeline", K);
-    int batch = max_rows >= 8 ? (max_rows / 8) * 8 : max_rows;
-    if (batch > 32) batch = 32;
-    // The dp4a kernel multiplies eight rows at a time however many one launch holds; where the
-    // tensor-core kernel takes eight rows, launches of eight are faster (38.4 against 18.1 us a
-    // pass over 4096 x 14336 of Q4_K).
-    const bool eights = M > 8 && mmvq_eight_rows(type, K);
-    if (eights) batch = 8;
     const size_t xq_row = static_cast<size_t>(K / 32) * kQ8_1Bytes;
     const size_t c_elem = out_f32 ? 4 : 2;
     for (int m0 = 0; m0 < M; m0 += batch) {

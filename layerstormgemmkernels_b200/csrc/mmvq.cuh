@@ -60,7 +60,7 @@ struct MmvqArgs {
     // start on the SMs the previous launch has left while its last CTAs still stream - and
     // the wait is made before the CTA exits, so that launches still complete in stream order.
     int dep_mode;
-    int eights;               // part of a call of more than eight rows in passes of eight: one kernel for all its rows
+    int eights;               // a pass of a call that goes to the tensor-core mat-vec (mmvq_mma.cuh), all its passes
 #ifdef LSG_MMVQ_TRACE
     unsigned long long* trace;  // [grid][16] nanosecond timestamps of the phases of each CTA
 #endif
@@ -124,7 +124,7 @@ MmvqTune mmvq_tuning();  // current process-wide geometry, clamped to valid rang
 #define LSG_DECLARE_MMVQ(id)                                         \
     int mmvq_launch_t##id(MmvqArgs a, const MmvqTune& tn, cudaStream_t stream, bool pdl); \
     int mmvq_max_rows_t##id(int K);                                                       \
-    bool mmvq_eight_rows_t##id(int K);
+    bool mmvq_eight_rows_t##id(int M, int K);
 LSG_DECLARE_MMVQ(0) LSG_DECLARE_MMVQ(1) LSG_DECLARE_MMVQ(2) LSG_DECLARE_MMVQ(3)
 LSG_DECLARE_MMVQ(4) LSG_DECLARE_MMVQ(5) LSG_DECLARE_MMVQ(6) LSG_DECLARE_MMVQ(7)
 

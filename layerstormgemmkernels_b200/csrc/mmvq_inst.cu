@@ -122,38 +122,76 @@ bool mma_cut_k(MmaCut& g, int K, int max_split, int max_blocks) {
     return true;
 }
 
-// Shared memory: the deepest rings that fit (`sum_rows` rows of cluster sums).  Returns the bytes,
-// 0 when not even two blocks per warp fit.
+// Shared memory: the cluster sums of `sum_rows` rows, in chunks where they do not fit beside rings of
+// two blocks, and then the deepest rings that do.  Returns the bytes.
 template <class D>
 int mma_place(MmaCut& g, int sum_rows) {
-    const long long sum_bytes = static_cast<long long>(sum_rows + 15) / 16 * 16 * kMmaCols * 4;
-    constexpr int part_bytes = kMmaWarps * 2 * 128 * 4;
+    constexpr int part_bytes = kMmaWarps * 2 * 128 * 4, ring_bytes = kMmaWarps * 16 * D::kPitch, group_bytes = 16 * kMmaCols * 4;
+    static_assert(mma_image_bytes<D>(kMmaSliceBlocks * 8) + part_bytes + 2 * ring_bytes + kMmaWarps * group_bytes <= kSmemCap,
+                  "every K has room for two blocks per warp and the sums of a row group per set of warps");
     g.ring_off = mma_image_bytes<D>(g.slice * 8);
-    const long long avail = kSmemCap - g.ring_off - part_bytes - sum_bytes;
-    const long long depth = avail / (kMmaWarps * 16 * D::kPitch);
-    if (avail < 0 || depth < 2) return 0;
-    g.depth = depth > kMmaMaxDepth ? kMmaMaxDepth : static_cast<int>(depth);
-    g.part_off = g.ring_off + kMmaWarps * g.depth * 16 * D::kPitch;
+    const int avail = kSmemCap - g.ring_off - part_bytes, sets = kMmaWarps / g.wpg;
+    const int most = (avail - 2 * ring_bytes) / group_bytes / sets * sets;   // every set has a group in each round
+    g.chunk = (sum_rows + 15) / 16;
+    if (g.chunk > most) g.chunk = most;
+    const int sum_bytes = g.chunk * group_bytes;
+    const int depth = (avail - sum_bytes) / ring_bytes;
+    g.depth = depth > kMmaMaxDepth ? kMmaMaxDepth : depth;
+    g.part_off = g.ring_off + g.depth * ring_bytes;
     g.sum_off = g.part_off + part_bytes;
-    return g.sum_off + static_cast<int>(sum_bytes);
+    if (sum_rows == 0) g.chunk = 1 << 26;   // no sums: one chunk, of all row groups
+    return g.sum_off + sum_bytes;
 }
 
-// The tensor-core mat-vec (mmvq_mma.cuh), or kMmaNotTaken.
-constexpr int kMmaNotTaken = 1;
+// How many clusters of `ksplit` CTAs of the tensor-core mat-vec are resident at a time (0: the device
+// cannot hold one); asked for once per device, which also lets the kernel have its shared memory.
+template <int TT>
+int mma_slots(int ksplit, int& slots) {
+    if constexpr (MmaDec<TT>::kHas) {
+        auto kernel = mmvq_mma_kernel<TT>;
+        static std::atomic<int> clusters[64][4];   // of 1, 2, 4, 8 CTAs: their number + 1
+        int dev = 0;
+        LSG_CUDA_TRY(cudaGetDevice(&dev));
+        const int log_split = ksplit == 1 ? 0 : (ksplit == 2 ? 1 : (ksplit == 4 ? 2 : 3));
+        const bool known = dev >= 0 && dev < 64;
+        slots = (known ? clusters[dev][log_split].load(std::memory_order_relaxed) : 0) - 1;
+        if (slots >= 0) return LSG_OK;
+        LSG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
+        slots = sm_count();
+        if (ksplit > 1) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(static_cast<unsigned>(ksplit));
+            cfg.blockDim = dim3(kMmaThreads);
+            cfg.dynamicSmemBytes = kSmemCap;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = static_cast<unsigned>(ksplit);
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            LSG_CUDA_TRY(cudaOccupancyMaxActiveClusters(&slots, kernel, &cfg));
+            if (slots < 0) slots = 0;
+        }
+        if (known) clusters[dev][log_split].store(slots + 1, std::memory_order_relaxed);
+    }
+    return LSG_OK;
+}
+
+// The tensor-core mat-vec (mmvq_mma.cuh) of a call that MMVQ_FN(eight_rows) sends to it.
 template <int TT>
 int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
     if constexpr (MmaDec<TT>::kHas) {
         MmaArgs g = {};
         g.v = v;
-        if (v.M > kMmaCols || v.drop_slab >= 0 || !mma_cut_k(g.c, v.K, 8, kMmaSliceBlocks)) return kMmaNotTaken;
+        int slots = 0;
+        if (v.M > kMmaCols || !mma_cut_k(g.c, v.K, 8, kMmaSliceBlocks))
+            return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: M=%d K=%d do not fit the tensor-core mat-vec", v.M, v.K);
+        const int rc = mma_slots<TT>(g.c.ksplit, slots);
+        if (rc != LSG_OK) return rc;
         auto kernel = mmvq_mma_kernel<TT>;
-        static std::atomic<int> clusters[64][4];   // resident clusters of 1, 2, 4, 8 CTAs, per device
-        int dev = 0;
-        LSG_CUDA_TRY(cudaGetDevice(&dev));
-        const int log_split = g.c.ksplit == 1 ? 0 : (g.c.ksplit == 2 ? 1 : (g.c.ksplit == 4 ? 2 : 3));
         cudaLaunchConfig_t cfg = {};
         cfg.blockDim = dim3(kMmaThreads);
-        cfg.dynamicSmemBytes = kSmemCap;
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -163,18 +201,6 @@ int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int slots = dev >= 0 && dev < 64 ? clusters[dev][log_split].load(std::memory_order_relaxed) : 0;
-        if (slots == 0) {
-            LSG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
-            slots = sm_count();
-            if (g.c.ksplit > 1) {
-                cfg.gridDim = dim3(static_cast<unsigned>(g.c.ksplit));
-                LSG_CUDA_TRY(cudaOccupancyMaxActiveClusters(&slots, kernel, &cfg));
-                if (slots < 1) return kMmaNotTaken;
-            }
-            if (dev >= 0 && dev < 64) clusters[dev][log_split].store(slots, std::memory_order_relaxed);
-        }
         MmvqArgs& a = g.v;
         a.row_bytes = g.c.nsb * g.c.sb_bytes;
         const int n_prob = 1 + a.n_extra;
@@ -184,12 +210,11 @@ int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
             n_rows[1 + j] = a.Nx[j];
             n_total += a.Nx[j];
         }
-        const int grid = n_total < slots ? n_total : slots;
-        if (grid < n_prob) return kMmaNotTaken;
+        int grid = n_total < slots ? n_total : slots;
+        if (grid < n_prob) grid = n_prob;
         const int rows = share_ctas(grid, n_prob, n_rows, n_total, ctas_of);
         place_matrices(a, n_rows, ctas_of);
         const int smem = mma_place<MmaDec<TT>>(g.c, g.c.ksplit > 1 ? rows : 0);
-        if (smem == 0) return kMmaNotTaken;
         cfg.gridDim = dim3(static_cast<unsigned>(grid * g.c.ksplit));
         cfg.dynamicSmemBytes = static_cast<size_t>(smem);
         if (g.c.ksplit == 1) cfg.attrs = attr + 1;   // no cluster
@@ -197,7 +222,7 @@ int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
         LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, g));
         return LSG_OK;
     }
-    return kMmaNotTaken;
+    return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: type %d has no tensor-core mat-vec", TT);
 }
 
 }  // namespace
@@ -212,19 +237,18 @@ int MMVQ_FN(max_rows)(int K) {
     return rows < 1 ? 0 : rows;
 }
 
-// Whether eight batch rows of this K go to the tensor-core mat-vec.
-bool MMVQ_FN(eight_rows)(int K) {
+// Whether a call of M batch rows goes to the tensor-core mat-vec, in passes of eight.
+bool MMVQ_FN(eight_rows)(int M, int K) {
     MmaCut c = {};
-    return MmaDec<T>::kHas && mma_min_rows() <= kMmaCols && mma_cut_k(c, K, 8, kMmaSliceBlocks);
+    int slots = 0;
+    return MmaDec<T>::kHas && M >= mma_min_rows() && mma_min_rows() <= kMmaCols && mma_cut_k(c, K, 8, kMmaSliceBlocks) &&
+           mma_slots<T>(c.ksplit, slots) == LSG_OK && slots > 0;
 }
 
 int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool pdl) {
     using F = Fmt<T>;
     a.row_bytes = (a.K / F::VALS) * F::BYTES;
-    if ((a.M >= mma_min_rows() || a.eights) && !tn_in.skip_math) {
-        const int rc = launch_mma<T>(a, stream, pdl);
-        if (rc != kMmaNotTaken) return rc;
-    }
+    if (a.eights) return launch_mma<T>(a, stream, pdl);
     // Small matrices (a CTA's share of the weights is at most 40 KB, e.g. a 1024 x 4096 Q4_K
     // k or v projection launched alone): eleven
     // consumer warps and half the shared memory, so that two consecutive launches of a
@@ -363,7 +387,7 @@ bool grouped_mma(int K, MmaCut& c, int& smem) {
     if constexpr (MmaDec<TT>::kHas) {
         if (mma_min_rows() > kMmaCols || !mma_cut_k(c, K, 1, kMmaGroupedBlocks)) return false;
         smem = mma_place<MmaDec<TT>>(c, 0);
-        return smem > 0;
+        return true;
     }
     return false;
 }

@@ -25,9 +25,11 @@
 //     tiles are added in warp order through shared memory.  16 / wpg groups are in work at a time.
 //   * Long rows are split along K over the CTAs of a cluster (4096 values each): a CTA then
 //     quantizes and holds only its part of the activations, and the cluster has more rows.
-//     The CTAs add their sums in rank order through distributed shared memory.
-// How K is cut depends on K and the type alone, so a result does not depend on the number of
-// weight rows, on what shares the launch, or on the launch geometry.
+//     The CTAs add their sums in rank order through distributed shared memory, in as many pieces
+//     (`chunk` row groups) as the sums of the cluster's rows take beside the image and the rings.
+// Whether a call comes here depends on its type, K and batch rows alone, and how K is cut on the
+// type and K, so a result does not depend on the number of weight rows, on what shares the launch,
+// or on the launch geometry.
 #pragma once
 
 #include "mmvq_grouped.cuh"
@@ -48,6 +50,7 @@ struct MmaCut {
     int ksplit, slice;   // CTAs of a cluster along K, blocks of each
     int wpg;             // warps of a row group
     int depth;           // 16-row blocks of a warp's ring
+    int chunk;           // row groups between two cluster sums
     int ring_off, part_off, sum_off;   // image (at 0), rings, partial tiles, cluster sums
 };
 
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
     const MmaCut& g = args.c;
     extern __shared__ __align__(128) uint8_t smem[];
     float* part = reinterpret_cast<float*>(smem + g.part_off);     // [set][2][wpg][16 rows][8]
-    float* sums = reinterpret_cast<float*>(smem + g.sum_off);      // [row][8], with ksplit > 1
+    float* sums = reinterpret_cast<float*>(smem + g.sum_off);      // [row of the chunk][8], with ksplit > 1
 
     const int tid = threadIdx.x;
     const int rank = static_cast<int>(blockIdx.x) % g.ksplit;
@@ -648,38 +651,41 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
     else mma_image_q8_1<D>(smem, xqm, a.M, a.K / 32, sb0 * 8, nsb * 8, tid, kMmaThreads);
     __syncthreads();
 
-    int slot = 0, buf = 0;
-    for (int gi = w.set; gi < groups; gi += nsets, buf ^= 1) {
-        const int r0 = row_begin + gi * 16;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int sb = w.wi; sb < nsb; sb += g.wpg) {
-            prefetch();
-            mma_wait_block(w.depth);
+    int slot = 0, buf = 0, gi = w.set;
+    for (int c0 = 0; c0 < groups; c0 += g.chunk) {   // the same chunks in every CTA of the cluster
+        const int c1 = min(groups, c0 + g.chunk);
+        for (; gi < c1; gi += nsets, buf ^= 1) {
+            const int r0 = row_begin + gi * 16;
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int sb = w.wi; sb < nsb; sb += g.wpg) {
+                prefetch();
+                mma_wait_block(w.depth);
+                __syncwarp();
+                w.multiply(slot, sb, static_cast<uint32_t>(w_base) + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes),
+                           row_bytes, acc);
+                __syncwarp();   // every lane has read the slot before it is filled again
+                if (++slot == w.depth) slot = 0;
+            }
+            mma_add_tiles(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int col, float v) {
+                if (g.ksplit > 1) sums[((gi - c0) * 16 + r) * 8 + col] = v;
+                else if (col < a.M && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + r0 + r, v);
+            });
+        }
+        if (g.ksplit > 1) {
             __syncwarp();
-            w.multiply(slot, sb, static_cast<uint32_t>(w_base) + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes),
-                       row_bytes, acc);
-            __syncwarp();   // every lane has read the slot before it is filled again
-            if (++slot == w.depth) slot = 0;
+            mma_cluster_sync();
+            const uint32_t base = smem_u32(sums);
+            const int first = row_begin + c0 * 16, rows = min(row_end - first, (c1 - c0) * 16);
+            for (int i = rank * kMmaThreads + tid; i < rows * a.M; i += g.ksplit * kMmaThreads) {
+                const int col = i / rows, r = i - col * rows;
+                const uint32_t at = base + static_cast<uint32_t>(r * 8 + col) * 4u;
+                float v = mma_ld_cluster(at, 0);
+                for (int k = 1; k < g.ksplit; ++k) v += mma_ld_cluster(at, k);
+                store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + first + r, v);
+            }
+            __syncwarp();
+            mma_cluster_sync();   // no CTA leaves, or writes the next chunk, while a peer still reads its sums
         }
-        mma_add_tiles(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int col, float v) {
-            if (g.ksplit > 1) sums[(gi * 16 + r) * 8 + col] = v;
-            else if (col < a.M && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + r0 + r, v);
-        });
-    }
-    if (g.ksplit > 1) {
-        __syncwarp();
-        mma_cluster_sync();
-        const uint32_t base = smem_u32(sums);
-        const int rows = row_end - row_begin;
-        for (int i = rank * kMmaThreads + tid; i < rows * a.M; i += g.ksplit * kMmaThreads) {
-            const int col = i / rows, r = i - col * rows;
-            const uint32_t at = base + static_cast<uint32_t>(r * 8 + col) * 4u;
-            float v = mma_ld_cluster(at, 0);
-            for (int k = 1; k < g.ksplit; ++k) v += mma_ld_cluster(at, k);
-            store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + row_begin + r, v);
-        }
-        __syncwarp();
-        mma_cluster_sync();   // no CTA leaves while a peer still reads its sums
     }
     if (a.dep_mode == 2) pdl_wait_prior();
 }

@@ -733,7 +733,7 @@ int mmq_dense(int type, int M, int N, int K, const void* A, const void* W, void*
     // A few rows: expanding the weights costs more than passing over them once or twice with the
     // tensor-core mat-vec, eight rows at a time, whose sums are exact.  Q6_K 4096 x 14336, us:
     // 12 rows 50.8, 24 rows 77.5 on the mat-vec, 48 rows 73.1 expanded; 14336 x 4096: 38.6, 68.7, 60.3.
-    if (!outs && M <= 16 && mmvq_eight_rows(type, K) && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
+    if (!outs && M <= 16 && mmvq_eight_rows(type, 8, K) && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(A) & 15) == 0) {
         const int rc = quantize_q8_1(A, ws, M, K, s, true);
         if (rc != LSG_OK) return rc;

@@ -162,6 +162,34 @@ def test_mmvq_tensor_core_edges(ops, name, M, N, K):
     assert torch.equal(both[0], ops.gguf_mmvq(A, W2, t, 50, K, out_dtype=torch.float32))
 
 
+@pytest.mark.parametrize("name,M,N,K", [
+    ("Q6_K", 9, 36000, 18432),    # clusters of eight; dp4a holds seven rows of this K
+    ("Q8_0", 16, 23000, 32768),   # the longest K, four rows
+    ("Q6_K", 8, 93000, 8192),     # clusters of two
+    ("Q4_K", 8, 700, 28672),      # all sums fit; dp4a holds five rows
+    ("Q6_K", 7, 300, 28672),      # .. and four
+])
+def test_mmvq_route_does_not_depend_on_the_weight_rows(ops, name, M, N, K):
+    """A K of which the dp4a kernel holds fewer rows than the call has, and more weight rows than the
+    sums of a cluster have room for beside the weight rings: every call is taken, and a result is the
+    same whatever shares the call - equal weight rows, a slice of the matrix, a joined matrix, the
+    batch rows in another order.  Same integers as the oracle (TOL_F32)."""
+    t, U = T[name], 64
+    A = torch.randn(M, K, generator=torch.Generator().manual_seed(N)).to(torch.bfloat16).cuda()
+    Wu = Q.random_gguf_weight(name, U, K, seed=K)
+    Wd = torch.from_numpy(Wu).cuda().repeat((N + U - 1) // U, 1)[:N].contiguous()   # row j is row j % U
+    ref = oracle.mmvq(t, oracle.quantize_q8_1(bf16_bits(A)), Wu, K)
+    got = ops.gguf_mmvq(A, Wd, t, N, K, out_dtype=torch.float32)
+    assert rel_err(got[:, :U].cpu().numpy(), ref) <= TOL_F32
+    assert torch.equal(got, got[:, :U].repeat(1, (N + U - 1) // U)[:, :N])
+    assert torch.equal(got[:, 128:228], ops.gguf_mmvq(A, Wd[128:228].clone(), t, 100, K, out_dtype=torch.float32))
+    assert torch.equal(got, ops.gguf_mmvq(A.flip(0).contiguous(), Wd, t, N, K, out_dtype=torch.float32).flip(0))
+    both = ops.gguf_mmvq_batch(A, [(Wd[:50].clone(), 50), (Wd, N)], t, out_dtype=torch.float32)
+    assert torch.equal(both[0], got[:, :50]) and torch.equal(both[1], got)
+    if M > 8:
+        assert torch.equal(ops.gguf_mmq(A, Wd, t, N, K, out_dtype=torch.float32), got)
+
+
 @pytest.mark.parametrize("name", ["Q5_K", "Q6_K", "Q8_0", "Q4_0"])
 @pytest.mark.parametrize("M", [9, 13, 16])
 def test_few_rows_of_expanded_types_take_the_matvec(ops, name, M):
