@@ -78,11 +78,12 @@ int check_common(const lsg_gguf_grouped_gemm_params* p) {
 // The grouped mat-vec over a device-built segment list: activations quantized into the
 // workspace (skipped when `xq_ready`: the caller, or the call in front with the same A_base, K
 // and workspace, left them there) and segments built from the offsets (`seg_ready` is the list of
-// a call in front with the same offsets and the same rows per segment that skipped the same
-// experts - the caller guarantees that an expert has a weight here when it had one there), then
+// a call in front with the same offsets, the same rows per segment and the same pointer arrays:
+// p->B_ptrs, also1 and also2, an expert with a null entry in any of them being left out), then
 // one launch.
 int grouped_matvec_tail(const lsg_gguf_grouped_gemm_params* p, int T, uint8_t* base, const WsLayout& w,
-                        cudaStream_t s, bool xq_ready, const int* seg_ready) {
+                        cudaStream_t s, bool xq_ready, const int* seg_ready, const void* const* also1 = nullptr,
+                        const void* const* also2 = nullptr) {
     int rc = LSG_OK;
     if (!xq_ready) {
         rc = quantize_q8_1(p->A_base, base, T, p->K, s, true);
@@ -93,7 +94,7 @@ int grouped_matvec_tail(const lsg_gguf_grouped_gemm_params* p, int T, uint8_t* b
     const int max_rows = grouped_max_rows(p->type, p->K, tn);
     if (!seg_ready) {
         rc = build_segment_list(static_cast<const int32_t*>(p->expert_offsets), p->B_ptrs, p->num_experts,
-                                max_rows, w.max_segments, seg, s, T);
+                                max_rows, w.max_segments, seg, s, T, also1, also2);
         if (rc != LSG_OK) return rc;
     }
     GroupedArgs a = {};
@@ -211,14 +212,15 @@ int grouped_hostloop(const lsg_gguf_grouped_gemm_params* p, void* ws, size_t ws_
 }  // namespace
 
 // The mat-vec route of lsg_gguf_grouped_gemm for a caller inside the library that runs several
-// projections of the same rows through the same workspace (gate and up of an expert block):
+// projections of the same rows through the same workspace (gate, up and down of an expert block):
 // `xq_ready` skips the activation quantizer (the Q8_1 blocks of all T rows are at the start of
-// the workspace already).  `seg_k` is the K of an earlier call of the block whose segment list is
-// still in the workspace, 0 when there is none (every expert with rows has all its weights:
-// lsg_gguf_moe_ffn's contract); the list serves when it was cut into segments of the same rows and
-// this call's Q8_1 blocks end in front of it.  A_base may be null with `xq_ready`.
+// the workspace already).  also1 and also2 are the pointer arrays of the block's other projections:
+// an expert that lacks one of its matrices is skipped by all of them.  `seg_k` is the K of an earlier
+// call of the block whose segment list is still in the workspace, 0 when there is none; the list
+// serves when it was cut into segments of the same rows and this call's Q8_1 blocks end in front of
+// it.  A_base may be null with `xq_ready`.
 int grouped_gemm_matvec(const lsg_gguf_grouped_gemm_params* p, int T, void* ws, size_t ws_bytes, cudaStream_t s,
-                        bool xq_ready, int seg_k) {
+                        bool xq_ready, int seg_k, const void* const* also1, const void* const* also2) {
     int rc = check_common(p);
     if (rc != LSG_OK) return rc;
     if (p->num_experts <= 0 || T <= 0) return LSG_OK;
@@ -237,7 +239,7 @@ int grouped_gemm_matvec(const lsg_gguf_grouped_gemm_params* p, int T, void* ws, 
         if (w.q8_bytes <= first.seg_off && grouped_max_rows(p->type, seg_k, tn) == grouped_max_rows(p->type, p->K, tn))
             seg = reinterpret_cast<const int*>(static_cast<uint8_t*>(ws) + first.seg_off);
     }
-    return grouped_matvec_tail(p, T, static_cast<uint8_t*>(ws), w, s, xq_ready, seg);
+    return grouped_matvec_tail(p, T, static_cast<uint8_t*>(ws), w, s, xq_ready, seg, also1, also2);
 }
 
 }  // namespace lsg

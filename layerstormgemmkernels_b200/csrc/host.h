@@ -33,7 +33,8 @@ int build_active_expert_list(const int32_t* offs, int E, int cap, int* active, c
 int build_mmq_tile_map(const int32_t* offs, int E, int tile_m, int T_max, int* tile_expert,
                        int* tile_mstart, cudaStream_t s, int rows = 0x7fffffff, bool balanced = false);
 int build_segment_list(const int32_t* offs, const void* const* B_ptrs, int E, int max_rows,
-                       int max_segments, int* seg, cudaStream_t s, int rows = 0x7fffffff);
+                       int max_segments, int* seg, cudaStream_t s, int rows = 0x7fffffff,
+                       const void* const* also1 = nullptr, const void* const* also2 = nullptr);
 
 size_t mmq_scratch_bytes(long long rows, int K, int E, int N);
 // Several output matrices for one GEMM (this GPU's and its peers'): every tile is stored
@@ -75,7 +76,7 @@ bool tc_fused_available(int type);
 bool tc_fused_forced();   // weight path 2: every call takes the fused kernel
 size_t tc_fused_dense_scratch_bytes(int M, int N, int K);
 int grouped_gemm_matvec(const lsg_gguf_grouped_gemm_params* p, int T, void* ws, size_t ws_bytes, cudaStream_t s,
-                        bool xq_ready, int seg_k);
+                        bool xq_ready, int seg_k, const void* const* also1, const void* const* also2);
 int tc_fused_grouped_tile_m(long long T, int E);
 size_t tc_fused_grouped_scratch_bytes(long long T, int E, int N, int K);
 int tc_fused_dense(int type, int M, int N, int K, const void* A_bf16, const void* W, void* C, int ldc,

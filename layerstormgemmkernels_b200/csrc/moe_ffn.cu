@@ -151,23 +151,24 @@ extern "C" int lsg_gguf_moe_ffn(const lsg_gguf_moe_ffn_params* p, int total_toke
     // and at these sizes the launches are the cost.  The routed rows are quantized straight
     // from the token matrix through the permutation (no gathered copy), up reads the Q8_1
     // blocks and the segment list gate's call left in the workspace (down the list as well, where
-    // its segments have the same height), and the activation is formed inside the quantizer of the
-    // down projection (no bf16 activation buffer): seven launches instead of twelve.
+    // its segments have the same height and its Q8_1 blocks end in front of the list), and the
+    // activation is formed inside the quantizer of the down projection (no bf16 activation buffer):
+    // six launches, seven with a list of down's own, instead of twelve.
     if (T / E <= 8 && H % 8 == 0 && I % 8 == 0 && (reinterpret_cast<uintptr_t>(p->A_base) & 15) == 0) {
         int rc = p->perm ? quantize_q8_1_gather(p->A_base, p->perm, p->top_k, gws, T, H, s, true)
                          : quantize_q8_1(p->A_base, gws, T, H, s, true);
         if (rc != LSG_OK) return rc;
         g.A_base = nullptr;
         g.D_base = base + l.g_off; g.B_ptrs = p->gate_ptrs;
-        rc = grouped_gemm_matvec(&g, T, gws, l.grouped_bytes, s, true, 0);
+        rc = grouped_gemm_matvec(&g, T, gws, l.grouped_bytes, s, true, 0, p->up_ptrs, p->down_ptrs);
         if (rc != LSG_OK) return rc;
         g.D_base = base + l.u_off; g.B_ptrs = p->up_ptrs;
-        rc = grouped_gemm_matvec(&g, T, gws, l.grouped_bytes, s, true, H);
+        rc = grouped_gemm_matvec(&g, T, gws, l.grouped_bytes, s, true, H, p->gate_ptrs, p->down_ptrs);
         if (rc != LSG_OK) return rc;
         rc = quantize_q8_1_silu_mul(base + l.g_off, base + l.u_off, gws, T, I, s, true);
         if (rc != LSG_OK) return rc;
         g.N = H; g.K = I; g.D_base = p->D_base; g.B_ptrs = p->down_ptrs; g.out_dtype = p->out_dtype;
-        return grouped_gemm_matvec(&g, T, gws, l.grouped_bytes, s, true, H);
+        return grouped_gemm_matvec(&g, T, gws, l.grouped_bytes, s, true, H, p->gate_ptrs, p->up_ptrs);
     }
 
     const void* rows = p->A_base;

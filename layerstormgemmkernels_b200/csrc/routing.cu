@@ -101,8 +101,10 @@ __global__ void mmq_tile_map_kernel(const int32_t* __restrict__ offs, int E, int
 
 // seg[0] = number of segments; then triples (expert, first row, rows).  Experts with a
 // null weight pointer are skipped, as the reference's host loop skips them
-// (gguf_grouped_gemm.cu:114-118 with B_e == nullptr guarded in the engine).
+// (gguf_grouped_gemm.cu:114-118 with B_e == nullptr guarded in the engine); also1 and also2 (may
+// be null) are the pointers of further matrices that the list is used with.
 __global__ void segment_list_kernel(const int32_t* __restrict__ offs, const void* const* __restrict__ B_ptrs,
+                                    const void* const* __restrict__ also1, const void* const* __restrict__ also2,
                                     int E, int max_rows, int max_segments, int rows, int* __restrict__ seg) {
     pdl_launch_dependents();
     pdl_wait_prior();
@@ -113,7 +115,7 @@ __global__ void segment_list_kernel(const int32_t* __restrict__ offs, const void
         if (e < E) {
             off = min(offs[e], rows);
             m = min(offs[e + 1], rows) - off;
-            if (m < 0 || B_ptrs[e] == nullptr) m = 0;
+            if (m < 0 || B_ptrs[e] == nullptr || (also1 && also1[e] == nullptr) || (also2 && also2[e] == nullptr)) m = 0;
             ns = (m + max_rows - 1) / max_rows;
         }
         int all;
@@ -149,8 +151,9 @@ int build_mmq_tile_map(const int32_t* offs, int E, int tile_m, int T_max, int* t
 }
 
 int build_segment_list(const int32_t* offs, const void* const* B_ptrs, int E, int max_rows,
-                       int max_segments, int* seg, cudaStream_t s, int rows) {
-    LSG_CUDA_TRY(launch_kernel(segment_list_kernel, dim3(1), dim3(kScanThreads), 0, s, true, offs, B_ptrs, E,
+                       int max_segments, int* seg, cudaStream_t s, int rows, const void* const* also1,
+                       const void* const* also2) {
+    LSG_CUDA_TRY(launch_kernel(segment_list_kernel, dim3(1), dim3(kScanThreads), 0, s, true, offs, B_ptrs, also1, also2, E,
                                max_rows, max_segments, rows, seg));
     return LSG_OK;
 }

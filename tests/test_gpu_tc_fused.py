@@ -2,6 +2,8 @@
 (weight rows on the 128-lane side, tokens on the N side, optional split of K).  The
 checker is the CPU oracle of the reference's integer path (gguf_mmvq.cu:66-187 after
 quantize_bf16_to_q8_1); the bound is the GEMM tolerance max|y - ref| <= 1e-3 max|ref|."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -229,6 +231,49 @@ def test_moe_ffn_equals_three_grouped_gemms(ops, name, counts):
     # both sides round gate/up to bf16 before the activation; a last-bit difference there moves
     # the activation by one bf16 ulp, hence the bf16-sized slack on top of the GEMM bound
     assert (got[live] - ref[live]).abs().max().item() <= (TOL_TC + 2.0 ** -8) * scale
+
+
+@pytest.mark.parametrize("name,H,I", [
+    ("Q4_K", 512, 256),     # down reads the segment list that gate's call built
+    ("Q4_K", 256, 768),     # down's Q8_1 blocks reach over that list: a list of its own
+    ("Q6_K", 256, 4352),    # .. of a longer row than the tensor-core mat-vec takes
+    ("Q8_0", 8192, 256),    # the list would survive, but down's segments have another height
+])
+def test_moe_ffn_few_rows_lists_and_missing_matrices(ops, name, H, I):
+    """The mat-vec route of the expert block (a few rows per expert): against the three grouped GEMMs
+    with the activation in between, and with a null pointer in gate, up or down - the expert's rows
+    are then untouched, and the others keep their bits."""
+    from layerstormgemmkernels_b200 import capi
+    counts = [2, 11, 0, 3, 1]
+    A, offs, ws, gp, up, dp = _ffn_case(name, counts, H, I, seed=H + I)
+    t, rows = T[name], sum(counts)
+    g = ops.gguf_grouped_gemm(A, offs, gp, t, 1, I, H, 1)
+    u = ops.gguf_grouped_gemm(A, offs, up, t, 1, I, H, 1)
+    act = (torch.nn.functional.silu(g.float()) * u.float()).to(torch.bfloat16)
+    ref = ops.gguf_grouped_gemm(act, offs, dp, t, 1, H, I, 1, out_dtype=torch.float32)
+
+    def block(gate, up_, down):
+        D = torch.full((rows, H), 7.0, device="cuda")
+        p = capi.GgufMoeFfnParams(type=t, num_experts=len(counts), H=H, I=I, A_base=A.data_ptr(), D_base=D.data_ptr(),
+                                  expert_offsets=offs.data_ptr(), gate_ptrs=gate.data_ptr(), up_ptrs=up_.data_ptr(),
+                                  down_ptrs=down.data_ptr(), out_dtype=capi.DTYPE_F32, perm=None, top_k=1)
+        n = capi.lib.lsg_gguf_moe_ffn_workspace_bytes(rows, H, I, len(counts))
+        w = torch.empty(n, dtype=torch.uint8, device="cuda")
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        capi.check(capi.lib.lsg_gguf_moe_ffn(ctypes.byref(p), rows, ctypes.c_void_p(w.data_ptr()), n, stream))
+        return D
+
+    full = block(gp, up, dp)
+    # the bound of test_moe_ffn_equals_three_grouped_gemms without the tensor-core GEMM's part, the
+    # int8 step of a rounded activation in its place
+    assert (full - ref).abs().max().item() <= 2.0 ** -6 * ref.abs().max().item()
+    o = offs.tolist()
+    for j in range(3):
+        ptrs = [x.clone() for x in (gp, up, dp)]
+        ptrs[j][1] = 0
+        got = block(*ptrs)
+        assert torch.equal(got[o[1]:o[2]], torch.full_like(got[o[1]:o[2]], 7.0))
+        assert torch.equal(got[:o[1]], full[:o[1]]) and torch.equal(got[o[2]:], full[o[2]:])
 
 
 def test_moe_ffn_matvec_threshold(ops):
