@@ -201,7 +201,7 @@ int grouped_hostloop(const lsg_gguf_grouped_gemm_params* p, void* ws, size_t ws_
                             ws ? ws_bytes : size_t(0), need);
             rc = quantize_q8_1(A_e, ws, M_e, p->K, s, false);
             if (rc == LSG_OK)
-                rc = mmvq_q8_1(p->type, M_e, p->N, p->K, ptrs[e], ws, D_e, p->N,
+                rc = mmvq_q8_1(p->type, M_e, p->N, p->K, ptrs[e], ws, D_e,
                                p->out_dtype == LSG_DTYPE_F32, s, false);
         }
         if (rc != LSG_OK) return rc;

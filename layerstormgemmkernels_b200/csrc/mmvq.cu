@@ -108,11 +108,10 @@ int check_gemm_params(const char* op, const lsg_gguf_mmvq_params* p) {
     return LSG_OK;
 }
 
-// Batch rows of one launch of a call (0: not even one row of this K fits), and which kernel all its
-// launches take.  The dp4a kernel takes as many rows as its activation image holds, a multiple of
-// eight when possible (eight rows per register pass); where the tensor-core kernel takes the call,
-// launches of eight are faster (38.4 against 18.1 us a pass over 4096 x 14336 of Q4_K).
-int rows_per_launch(int type, int M, int K, bool& eights) {
+// Batch rows of one pass of a call (0: not even one row of this K fits), and which kernel all its
+// passes take.  The dp4a kernel takes as many rows as its activation image holds, a multiple of
+// eight when possible (eight rows per register pass); the tensor-core kernel takes eight.
+int rows_per_pass(int type, int M, int K, bool& eights) {
     const int max_rows = dispatch_max_rows(type, K);
     eights = max_rows >= 1 && g_drop_slab < 0 && !sane_tuning().skip_math && mmvq_eight_rows(type, M, K);
     if (eights) return 8;
@@ -120,50 +119,16 @@ int rows_per_launch(int type, int M, int K, bool& eights) {
     return batch > 32 ? 32 : batch;
 }
 
-// xq: Q8_1 blocks of all M rows.  ldc: output row stride.
-int mmvq_q8_1(int type, int M, int N, int K, const void* W, const void* xq, void* C, int ldc,
-              int out_f32, cudaStream_t stream, bool pdl, const void* A_bf16, int dep_mode) {
-    if (M == 0 || N == 0) return LSG_OK;
-    if (K == 0) return fail(LSG_ERR_INVALID, "gguf_mmvq: K must be positive");
-    if (!W || (!xq && !A_bf16) || !C) return fail(LSG_ERR_INVALID, "gguf_mmvq: null pointer");
-    if (reinterpret_cast<uintptr_t>(W) & 15)
-        return fail(LSG_ERR_ALIGNMENT, "gguf_mmvq: packed weight must be 16-byte aligned");
-    if (!A_bf16 && (reinterpret_cast<uintptr_t>(xq) & 3))
-        return fail(LSG_ERR_ALIGNMENT, "gguf_mmvq: Q8_1 buffer must be 4-byte aligned");
-    bool eights;
-    const int batch = rows_per_launch(type, M, K, eights);
-    if (batch < 1)
-        return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: K=%d too large for the shared-memory pipeline", K);
-    const size_t xq_row = static_cast<size_t>(K / 32) * kQ8_1Bytes;
-    const size_t c_elem = out_f32 ? 4 : 2;
-    for (int m0 = 0; m0 < M; m0 += batch) {
-        MmvqArgs a = {};
-        a.W = static_cast<const uint8_t*>(W);
-        a.xq = xq ? static_cast<const uint8_t*>(xq) + static_cast<size_t>(m0) * xq_row : nullptr;
-        a.A = A_bf16 ? static_cast<const __nv_bfloat16*>(A_bf16) + static_cast<size_t>(m0) * K : nullptr;
-        a.C = static_cast<uint8_t*>(C) + static_cast<size_t>(m0) * ldc * c_elem;
-        a.status = device_status_word();
-        a.M = (M - m0) < batch ? (M - m0) : batch;
-        a.N = N;
-        a.K = K;
-        a.ldc = ldc;
-        a.out_f32 = out_f32;
-        a.dep_mode = (pdl && m0 == 0) ? dep_mode : 0;   // later row batches are fully serialized launches
-        a.eights = eights ? 1 : 0;
-        const int rc = dispatch_launch(type, a, stream, pdl && m0 == 0);
-        if (rc != LSG_OK) return rc;
-    }
-    return LSG_OK;
-}
-
-// The same activations against n <= 4 weight matrices of one type and K, as one launch
-// per batch of rows.  Matrix j writes C[j], [M][N[j]] row-major.
+// The same activations (or, with A_each / xq_each, activations of their own) against n <= 6 weight
+// matrices of one type and K.  Matrix j writes C[j], [M][N[j]] row-major; xq: Q8_1 blocks of all M
+// rows.  One launch per pass over the batch rows; on the tensor-core kernel the passes are further
+// matrices of the launch, up to six in all: one after the other, the passes of a call of 9 to 32 rows
+// took twice the dp4a kernel's time on small matrices, which do not fill the chip.
 int mmvq_q8_1_joined(int type, int M, int K, int n, const void* const* W, void* const* C, const int* N,
                      const void* xq, int out_f32, cudaStream_t stream, bool pdl, const void* A_bf16, int dep_mode = 0,
                      const void* const* A_each = nullptr, const void* const* xq_each = nullptr) {
     if (n < 1 || n > 1 + kMmvqMaxExtra) return fail(LSG_ERR_INVALID, "gguf_mmvq: 1..6 matrices per joined launch");
-    if (n == 1) return mmvq_q8_1(type, M, N[0], K, W[0], xq, C[0], N[0], out_f32, stream, pdl, A_bf16, dep_mode);
-    if (M == 0) return LSG_OK;
+    if (M == 0 || (n == 1 && N[0] == 0)) return LSG_OK;
     if (K == 0) return fail(LSG_ERR_INVALID, "gguf_mmvq: K must be positive");
     if (!xq && !A_bf16) return fail(LSG_ERR_INVALID, "gguf_mmvq: null pointer");
     for (int j = 0; j < n; ++j) {
@@ -175,39 +140,61 @@ int mmvq_q8_1_joined(int type, int M, int K, int n, const void* const* W, void* 
     if (!A_bf16 && (reinterpret_cast<uintptr_t>(xq) & 3))
         return fail(LSG_ERR_ALIGNMENT, "gguf_mmvq: Q8_1 buffer must be 4-byte aligned");
     bool eights;
-    const int batch = rows_per_launch(type, M, K, eights);
+    const int batch = rows_per_pass(type, M, K, eights);
     if (batch < 1)
         return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: K=%d too large for the shared-memory pipeline", K);
     const size_t xq_row = static_cast<size_t>(K / 32) * kQ8_1Bytes;
     const size_t c_elem = out_f32 ? 4 : 2;
-    for (int m0 = 0; m0 < M; m0 += batch) {
+    // Items are (matrix, pass) pairs, a matrix's passes next to each other (they read the same weights
+    // at the same time); `per` of them share a launch.
+    const int passes = (M + batch - 1) / batch, items = n * passes;
+    const int launches = eights ? (items + kMmvqMaxExtra) / (1 + kMmvqMaxExtra) : passes;
+    for (int l = 0; l < launches; ++l) {
+        const int i0 = static_cast<int>(static_cast<long long>(items) * l / launches);
+        const int i1 = static_cast<int>(static_cast<long long>(items) * (l + 1) / launches);
         MmvqArgs a = {};
-        a.W = static_cast<const uint8_t*>(W[0]);
-        a.xq = xq ? static_cast<const uint8_t*>(xq) + static_cast<size_t>(m0) * xq_row : nullptr;
-        a.A = A_bf16 ? static_cast<const __nv_bfloat16*>(A_bf16) + static_cast<size_t>(m0) * K : nullptr;
-        a.C = static_cast<uint8_t*>(C[0]) + static_cast<size_t>(m0) * N[0] * c_elem;
         a.status = device_status_word();
-        a.M = (M - m0) < batch ? (M - m0) : batch;
-        a.N = N[0];
         a.K = K;
-        a.ldc = N[0];
         a.out_f32 = out_f32;
-        a.n_extra = n - 1;
-        for (int j = 1; j < n; ++j) {
-            a.Wx[j - 1] = static_cast<const uint8_t*>(W[j]);
-            a.Cx[j - 1] = static_cast<uint8_t*>(C[j]) + static_cast<size_t>(m0) * N[j] * c_elem;
-            a.Nx[j - 1] = N[j];
-            if (A_bf16)
-                a.Ax[j - 1] = static_cast<const __nv_bfloat16*>(A_each && A_each[j] ? A_each[j] : A_bf16) + static_cast<size_t>(m0) * K;
-            else
-                a.xqx[j - 1] = static_cast<const uint8_t*>(xq_each && xq_each[j] ? xq_each[j] : xq) + static_cast<size_t>(m0) * xq_row;
-        }
-        a.dep_mode = (pdl && m0 == 0) ? dep_mode : 0;
+        a.n_extra = i1 - i0 - 1;
         a.eights = eights ? 1 : 0;
-        const int rc = dispatch_launch(type, a, stream, pdl && m0 == 0);
+        for (int i = i0; i < i1; ++i) {
+            const int j = eights ? i / passes : i - i0, m0 = (eights ? i % passes : l) * batch;
+            const int rows = (M - m0) < batch ? (M - m0) : batch;
+            const uint8_t* w = static_cast<const uint8_t*>(W[j]);
+            void* c = static_cast<uint8_t*>(C[j]) + static_cast<size_t>(m0) * N[j] * c_elem;
+            const void* aj = A_each && A_each[j] ? A_each[j] : A_bf16;
+            const void* qj = xq_each && xq_each[j] ? xq_each[j] : xq;
+            const __nv_bfloat16* x = A_bf16 ? static_cast<const __nv_bfloat16*>(aj) + static_cast<size_t>(m0) * K : nullptr;
+            const uint8_t* q = A_bf16 ? nullptr : static_cast<const uint8_t*>(qj) + static_cast<size_t>(m0) * xq_row;
+            if (i == i0) {
+                a.W = w;
+                a.A = x;
+                a.xq = q;
+                a.C = c;
+                a.M = rows;
+                a.N = a.ldc = N[j];
+            } else {
+                const int e = i - i0 - 1;
+                a.Wx[e] = w;
+                a.Ax[e] = x;
+                a.xqx[e] = q;
+                a.Cx[e] = c;
+                a.Mx[e] = rows;
+                a.Nx[e] = N[j];
+            }
+        }
+        a.dep_mode = (pdl && l == 0) ? dep_mode : 0;   // later launches are fully serialized
+        const int rc = dispatch_launch(type, a, stream, pdl && l == 0);
         if (rc != LSG_OK) return rc;
     }
     return LSG_OK;
+}
+
+// One matrix.  C is [M][N] row-major.
+int mmvq_q8_1(int type, int M, int N, int K, const void* W, const void* xq, void* C, int out_f32, cudaStream_t stream,
+              bool pdl, const void* A_bf16, int dep_mode) {
+    return mmvq_q8_1_joined(type, M, K, 1, &W, &C, &N, xq, out_f32, stream, pdl, A_bf16, dep_mode);
 }
 
 bool fused_quant_ok(int M, int K, const void* A) {
@@ -230,7 +217,7 @@ extern "C" size_t lsg_gguf_mmvq_workspace_bytes(int M, int K) {
 extern "C" int lsg_gguf_mmvq_q8_1(const lsg_gguf_mmvq_params* p, const void* xq, void* stream) {
     int rc = check_gemm_params("gguf_mmvq", p);
     if (rc != LSG_OK) return rc;
-    return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, xq, p->C, p->N,
+    return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, xq, p->C,
                      p->out_dtype == LSG_DTYPE_F32, static_cast<cudaStream_t>(stream), true);
 }
 
@@ -247,11 +234,11 @@ extern "C" int lsg_gguf_mmvq(const lsg_gguf_mmvq_params* p, void* workspace,
     // Few activation values: every CTA quantizes them itself while its first weights are
     // in flight, which saves a launch and a dependency.  Otherwise quantize once, here.
     if (fused_quant_ok(p->M, p->K, p->A))
-        return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, nullptr, p->C, p->N,
+        return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, nullptr, p->C,
                          p->out_dtype == LSG_DTYPE_F32, s, true, p->A);
     rc = quantize_q8_1(p->A, workspace, p->M, p->K, s, true);
     if (rc != LSG_OK) return rc;
-    return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, workspace, p->C, p->N,
+    return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, workspace, p->C,
                      p->out_dtype == LSG_DTYPE_F32, s, true);
 }
 

@@ -82,6 +82,7 @@ struct MmvqArgs {
     const uint8_t* xqx[kMmvqMaxExtra];        // Q8_1 blocks of matrix j (set when A is null)
     void* Cx[kMmvqMaxExtra];
     int Nx[kMmvqMaxExtra];
+    int Mx[kMmvqMaxExtra];                    // batch rows of matrix j, in a launch with `eights`
     int cta0x[kMmvqMaxExtra];
     int rows_qx[kMmvqMaxExtra], rows_rx[kMmvqMaxExtra];
 };

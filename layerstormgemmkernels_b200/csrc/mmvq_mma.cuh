@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
     const __nv_bfloat16* Am = a.A;
     const uint8_t* xqm = a.xq;
     void* Cm = a.C;
-    int Nm = a.N, ldcm = a.ldc, rows_q = a.rows_q, rows_r = a.rows_r;
+    int Mm = a.M, Nm = a.N, ldcm = a.ldc, rows_q = a.rows_q, rows_r = a.rows_r;
     if (a.n_extra > 0) {
         const int b = bx;
         int jm = -1;
@@ -603,6 +603,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
             Am = a.Ax[jm];
             xqm = a.xqx[jm];
             Cm = a.Cx[jm];
+            Mm = a.Mx[jm];
             Nm = ldcm = a.Nx[jm];
             rows_q = a.rows_qx[jm];
             rows_r = a.rows_rx[jm];
@@ -647,8 +648,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
 
     if (a.dep_mode != 2) pdl_wait_prior();
     if (a.dep_mode == 1) pdl_launch_dependents();
-    if (Am) mma_image_bf16<D>(smem, Am, a.M, a.K, sb0 * 8, nsb * 8, tid, kMmaThreads);
-    else mma_image_q8_1<D>(smem, xqm, a.M, a.K / 32, sb0 * 8, nsb * 8, tid, kMmaThreads);
+    if (Am) mma_image_bf16<D>(smem, Am, Mm, a.K, sb0 * 8, nsb * 8, tid, kMmaThreads);
+    else mma_image_q8_1<D>(smem, xqm, Mm, a.K / 32, sb0 * 8, nsb * 8, tid, kMmaThreads);
     __syncthreads();
 
     int slot = 0, buf = 0, gi = w.set;
@@ -668,7 +669,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
             }
             mma_add_tiles(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int col, float v) {
                 if (g.ksplit > 1) sums[((gi - c0) * 16 + r) * 8 + col] = v;
-                else if (col < a.M && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + r0 + r, v);
+                else if (col < Mm && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + r0 + r, v);
             });
         }
         if (g.ksplit > 1) {
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
             mma_cluster_sync();
             const uint32_t base = smem_u32(sums);
             const int first = row_begin + c0 * 16, rows = min(row_end - first, (c1 - c0) * 16);
-            for (int i = rank * kMmaThreads + tid; i < rows * a.M; i += g.ksplit * kMmaThreads) {
+            for (int i = rank * kMmaThreads + tid; i < rows * Mm; i += g.ksplit * kMmaThreads) {
                 const int col = i / rows, r = i - col * rows;
                 const uint32_t at = base + static_cast<uint32_t>(r * 8 + col) * 4u;
                 float v = mma_ld_cluster(at, 0);

@@ -75,6 +75,6 @@ extern "C" int lsg_gguf_mmvq_noalloc(const lsg_gguf_mmvq_params* p, void* stream
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     rc = quantize_q8_1(p->A, scratch, p->M, p->K, s, true);
     if (rc != LSG_OK) return rc;
-    return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, scratch, p->C, p->N,
+    return mmvq_q8_1(p->type, p->M, p->N, p->K, p->B, scratch, p->C,
                      p->out_dtype == LSG_DTYPE_F32, s, true);
 }

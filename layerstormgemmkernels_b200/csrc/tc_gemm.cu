@@ -737,7 +737,7 @@ int mmq_dense(int type, int M, int N, int K, const void* A, const void* W, void*
         (reinterpret_cast<uintptr_t>(A) & 15) == 0) {
         const int rc = quantize_q8_1(A, ws, M, K, s, true);
         if (rc != LSG_OK) return rc;
-        return mmvq_q8_1(type, M, N, K, W, ws, C, N, out_f32, s, true);
+        return mmvq_q8_1(type, M, N, K, W, ws, C, out_f32, s, true);
     }
     __half* x16 = static_cast<__half*>(ws);
     __half* w16 = reinterpret_cast<__half*>(static_cast<uint8_t*>(ws) + align256(static_cast<size_t>(M) * K * 2));

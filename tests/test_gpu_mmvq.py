@@ -190,6 +190,30 @@ def test_mmvq_route_does_not_depend_on_the_weight_rows(ops, name, M, N, K):
         assert torch.equal(ops.gguf_mmq(A, Wd, t, N, K, out_dtype=torch.float32), got)
 
 
+@pytest.mark.parametrize("name,M,K,Ns", [
+    ("Q4_K", 13, 1024, (300,)),             # two passes in a launch, the second with five rows
+    ("Q6_K", 9, 4352, (33,)),               # .. with one row, K shared by two CTAs
+    ("Q8_0", 50, 768, (130, 5, 64)),        # 21 (matrix, pass) pairs: four launches
+    ("Q5_K", 16, 4352, (40, 300)),
+    ("Q4_0", 24, 2048, (17, 1, 9, 30, 2, 513)),
+])
+def test_mmvq_passes_of_eight_share_launches(ops, name, M, K, Ns):
+    """More than eight batch rows: the passes are further matrices of a launch.  Each gives the bits of
+    a call with its rows alone (those take the same kernel from five rows on), joined or not."""
+    t = T[name]
+    A = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).cuda()
+    Wn = [Q.random_gguf_weight(name, N, K, seed=60 + i) for i, N in enumerate(Ns)]
+    Ws = [torch.from_numpy(W).cuda() for W in Wn]
+    xq = oracle.quantize_q8_1(bf16_bits(A))
+    outs = ops.gguf_mmvq_batch(A, list(zip(Ws, Ns)), t, out_dtype=torch.float32)
+    for W, Wd, N, out in zip(Wn, Ws, Ns, outs):
+        assert rel_err(out.cpu().numpy(), oracle.mmvq(t, xq, W, K)) <= TOL_F32
+        assert torch.equal(out, ops.gguf_mmvq(A, Wd, t, N, K, out_dtype=torch.float32))
+        for m in range(0, M - 4, 8):
+            rows = A[m:m + 8].contiguous()
+            assert torch.equal(out[m:m + 8], ops.gguf_mmvq(rows, Wd, t, N, K, out_dtype=torch.float32))
+
+
 @pytest.mark.parametrize("name", ["Q5_K", "Q6_K", "Q8_0", "Q4_0"])
 @pytest.mark.parametrize("M", [9, 13, 16])
 def test_few_rows_of_expanded_types_take_the_matvec(ops, name, M):
