@@ -116,6 +116,7 @@ struct MmaWords {
 //   r0, r1  shared addresses of the block in rows g and g + 8
 //   xq      codes of this lane's column g: block j of the 256 values at xq + 256 j, lane offset in
 //   xs      scales of columns 2t, 2t + 1 (and what kKind says): block j at xs + j * kScaleBytes
+// ODD false: the odd columns hold nothing (their accumulators are left alone).
 // kHalves: the words of a block's two 16-value halves alternate in the image.
 // kKind: 0 scales {d}; 1 {d, d * sum of the codes}; 2 {d} and, behind the scales of all blocks, the
 // accumulator starts of the block's two halves, bias - 32 * sum of the half's codes, for columns
@@ -127,6 +128,7 @@ template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
     static constexpr int kBytes = FIVE ? 176 : 144;
     static constexpr int kPitch = FIVE ? 176 : 160;   // 8-byte loads of four rows: no bank twice with 160 (224 would not fit)
 
+    template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
                                                 float (&acc)[4]) {
         constexpr int QS = FIVE ? 48 : 16;
@@ -155,7 +157,14 @@ template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
                     a3 |= ((f1.y >> j) & 0x01010101u) << 4;
                 }
                 const uint2 xb = lds64(xq + 256 * j);
-                const uint4 xv = lds128(xs + 64 * j);
+                uint4 xv = make_uint4(0, 0, 0, 0);
+                if (ODD) {
+                    xv = lds128(xs + 64 * j);
+                } else {
+                    const uint2 e = lds64(xs + 64 * j);
+                    xv.x = e.x;
+                    xv.y = e.y;
+                }
                 const float dx0 = __uint_as_float(xv.x), sx0 = __uint_as_float(xv.y);
                 const float dx1 = __uint_as_float(xv.z), sx1 = __uint_as_float(xv.w);
                 int c[4];
@@ -164,21 +173,25 @@ template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
                 const float m0 = byte_f(mn0[j >> 2], j & 3), m1 = byte_f(mn1[j >> 2], j & 3);
                 const float n0 = -kMmaBias * c0, n1 = -kMmaBias * c1;
                 s1[0] = fmaf(dx0, mma_scaled(c[0], c0, n0), s1[0]);
-                s1[1] = fmaf(dx1, mma_scaled(c[1], c0, n0), s1[1]);
                 s1[2] = fmaf(dx0, mma_scaled(c[2], c1, n1), s1[2]);
-                s1[3] = fmaf(dx1, mma_scaled(c[3], c1, n1), s1[3]);
                 s2[0] = fmaf(m0, sx0, s2[0]);
-                s2[1] = fmaf(m0, sx1, s2[1]);
                 s2[2] = fmaf(m1, sx0, s2[2]);
-                s2[3] = fmaf(m1, sx1, s2[3]);
+                if (ODD) {
+                    s1[1] = fmaf(dx1, mma_scaled(c[1], c0, n0), s1[1]);
+                    s1[3] = fmaf(dx1, mma_scaled(c[3], c1, n1), s1[3]);
+                    s2[1] = fmaf(m0, sx1, s2[1]);
+                    s2[3] = fmaf(m1, sx1, s2[3]);
+                }
             }
         }
         const float d0 = fp16_bits_to_float(h0.x), e0 = fp16_bits_to_float(h0.x >> 16);
         const float d1 = fp16_bits_to_float(h1.x), e1 = fp16_bits_to_float(h1.x >> 16);
         acc[0] += d0 * s1[0] - e0 * s2[0];
-        acc[1] += d0 * s1[1] - e0 * s2[1];
         acc[2] += d1 * s1[2] - e1 * s2[2];
-        acc[3] += d1 * s1[3] - e1 * s2[3];
+        if (ODD) {
+            acc[1] += d0 * s1[1] - e0 * s2[1];
+            acc[3] += d1 * s1[3] - e1 * s2[3];
+        }
     }
 };
 template <> struct MmaDec<LSG_GGUF_Q4_K> : MmaDecK45<false> {};
@@ -191,6 +204,7 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
     static constexpr int kBytes = 210;
     static constexpr int kPitch = 240;   // 4-byte loads of eight rows: no bank twice
 
+    template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t xi,
                                                 float (&acc)[4]) {
         const MmaWords w[2] = {MmaWords(r0), MmaWords(r1)};
@@ -237,15 +251,18 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
                     const float sa = sbyte_f(scw[r][e >> 2], e & 3), sb = sbyte_f(scw[r][(e + 1) >> 2], (e + 1) & 3);
                     const float na = -kMmaBias * sa, nb = -kMmaBias * sb;
                     s[2 * r] = fmaf(dx0, mma_scaled(c[0][2 * r], sa, na) + mma_scaled(c[1][2 * r], sb, nb), s[2 * r]);
-                    s[2 * r + 1] = fmaf(dx1, mma_scaled(c[0][2 * r + 1], sa, na) + mma_scaled(c[1][2 * r + 1], sb, nb), s[2 * r + 1]);
+                    if (ODD)
+                        s[2 * r + 1] = fmaf(dx1, mma_scaled(c[0][2 * r + 1], sa, na) + mma_scaled(c[1][2 * r + 1], sb, nb), s[2 * r + 1]);
                 }
             }
         }
         const float d0 = fp16_bits_to_float(lds16(r0 + 208)), d1 = fp16_bits_to_float(lds16(r1 + 208));
         acc[0] += d0 * s[0];
-        acc[1] += d0 * s[1];
         acc[2] += d1 * s[2];
-        acc[3] += d1 * s[3];
+        if (ODD) {
+            acc[1] += d0 * s[1];
+            acc[3] += d1 * s[3];
+        }
     }
 };
 
@@ -256,6 +273,7 @@ template <> struct MmaDec<LSG_GGUF_Q8_0> {   // eight 34-byte blocks
     static constexpr int kBytes = 272;
     static constexpr int kPitch = 272;
 
+    template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
                                                 float (&acc)[4]) {
 #pragma unroll
@@ -282,9 +300,11 @@ template <> struct MmaDec<LSG_GGUF_Q8_0> {   // eight 34-byte blocks
             const float d0 = fp16_bits_to_float(lds16(r0 + 34 * j)), d1 = fp16_bits_to_float(lds16(r1 + 34 * j));
             const float dx0 = __uint_as_float(xv.x), dx1 = __uint_as_float(xv.y);
             acc[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, acc[0]);
-            acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
             acc[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, acc[2]);
-            acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
+            if (ODD) {
+                acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
+                acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
+            }
         }
     }
 };
@@ -301,6 +321,7 @@ template <> struct MmaDec<LSG_GGUF_Q4_0> {   // eight 18-byte blocks; byte i: va
         const uint32_t x = v ^ 0x08080808u;
         return x | ((x & 0x08080808u) * 30u);
     }
+    template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
                                                 float (&acc)[4]) {
 #pragma unroll
@@ -317,16 +338,21 @@ template <> struct MmaDec<LSG_GGUF_Q4_0> {   // eight 18-byte blocks; byte i: va
             const float d0 = fp16_bits_to_float(lds16(r0 + 18 * j)), d1 = fp16_bits_to_float(lds16(r1 + 18 * j));
             const float dx0 = __uint_as_float(xv.x), dx1 = __uint_as_float(xv.y);
             acc[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, acc[0]);
-            acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
             acc[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, acc[2]);
-            acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
+            if (ODD) {
+                acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
+                acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
+            }
         }
     }
 };
 
 // ---------------------------------------------------------------------------
-// Activation image of `nblk` 32-value blocks from block b0 on, eight columns (batch rows from M
-// on are zeros): codes [block][column][32], then the scales and accumulator starts of D::kKind.
+// Activation image of `nblk` 32-value blocks from block b0 on: codes [block][column][32], then the
+// scales and accumulator starts of D::kKind.  Batch row m is column m, or column 2m where there are
+// at most four (mma_step): every lane then has one column with a row, and does the scale arithmetic
+// of one instead of two - with one row per expert 64 x (768 x 2048) of Q4_K took the grouped kernel
+// longer than dp4a.  Columns without a batch row keep what was there: it stays in their own sums.
 // ---------------------------------------------------------------------------
 template <class D>
 __device__ __forceinline__ void mma_put_half(uint8_t* img, int b, int col, int half, const uint4& q) {
@@ -341,6 +367,7 @@ __device__ __forceinline__ void mma_put_half(uint8_t* img, int b, int col, int h
         *reinterpret_cast<uint4*>(at + 16 * half) = q;
     }
 }
+__device__ __forceinline__ int mma_step(int M) { return M <= kMmaCols / 2 ? 2 : 1; }
 template <class D> __host__ __device__ constexpr int mma_image_bytes(int nblk) {
     return nblk * (256 + D::kScaleBytes + (D::kKind == 2 ? 128 : 0));
 }
@@ -362,25 +389,23 @@ __device__ __forceinline__ void mma_put_scale(uint8_t* img, int nblk, int b, int
 template <class D>
 __device__ __forceinline__ void mma_image_q8_1(uint8_t* img, const uint8_t* __restrict__ xq, int M, int row_blocks,
                                                int b0, int nblk, int tid, int nthreads) {
-    for (int idx = tid; idx < kMmaCols * nblk; idx += nthreads) {
-        const int m = idx / nblk, b = idx - m * nblk;
-        uint32_t w[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if (m < M) {
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(xq + (static_cast<size_t>(m) * row_blocks + b0 + b) * kQ8_1Bytes);
+    for (int idx = tid; idx < M * nblk; idx += nthreads) {
+        const int m = idx / nblk, b = idx - m * nblk, col = m * mma_step(M);
+        uint32_t w[9];
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(xq + (static_cast<size_t>(m) * row_blocks + b0 + b) * kQ8_1Bytes);
 #pragma unroll
-            for (int i = 0; i < 9; ++i) w[i] = __ldg(src + i);
-        }
+        for (int i = 0; i < 9; ++i) w[i] = __ldg(src + i);
         int sum[2] = {0, 0};
 #pragma unroll
         for (int i = 1; i < 9; ++i) sum[(i - 1) >> 2] = __dp4a(static_cast<int>(w[i]), 0x01010101, sum[(i - 1) >> 2]);
-        mma_put_half<D>(img, b, m, 0, make_uint4(w[1], w[2], w[3], w[4]));
-        mma_put_half<D>(img, b, m, 1, make_uint4(w[5], w[6], w[7], w[8]));
+        mma_put_half<D>(img, b, col, 0, make_uint4(w[1], w[2], w[3], w[4]));
+        mma_put_half<D>(img, b, col, 1, make_uint4(w[5], w[6], w[7], w[8]));
         const float d = fp16_bits_to_float(w[0]);
         if (D::kKind == 2) {
-            mma_put_scale<D>(img, nblk, b, m, 0, d, sum[0]);
-            mma_put_scale<D>(img, nblk, b, m, 1, d, sum[1]);
+            mma_put_scale<D>(img, nblk, b, col, 0, d, sum[0]);
+            mma_put_scale<D>(img, nblk, b, col, 1, d, sum[1]);
         } else {
-            mma_put_scale<D>(img, nblk, b, m, 0, d, sum[0] + sum[1]);
+            mma_put_scale<D>(img, nblk, b, col, 0, d, sum[0] + sum[1]);
         }
     }
 }
@@ -389,13 +414,6 @@ __device__ __forceinline__ void mma_image_q8_1(uint8_t* img, const uint8_t* __re
 template <class D>
 __device__ __forceinline__ void mma_image_bf16(uint8_t* img, const __nv_bfloat16* __restrict__ A, int M, int K, int b0,
                                                int nblk, int tid, int nthreads) {
-    // columns without a batch row: zeros (the quantizer would take its slow path for a scale of 0)
-    for (int idx = tid; idx < (kMmaCols - M) * nblk * 2; idx += nthreads) {
-        const int half = idx & 1, task = idx >> 1;
-        const int c = task / nblk, b = task - c * nblk;
-        mma_put_half<D>(img, b, M + c, half, make_uint4(0, 0, 0, 0));
-        if (D::kKind == 2 || half == 0) mma_put_scale<D>(img, nblk, b, M + c, half, 0.0f, 0);
-    }
     const int total = M * nblk * 2;
     for (int base = tid & ~31; base < total; base += nthreads) {   // whole warps: the two lanes of a block exchange values
         const int idx = min(base + (tid & 31), total - 1);
@@ -426,8 +444,9 @@ __device__ __forceinline__ void mma_image_bf16(uint8_t* img, const __nv_bfloat16
                   __dp4a(static_cast<int>(q.w), 0x01010101, 0))));
         if (D::kKind != 2) sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         if (live) {
-            mma_put_half<D>(img, b, m, half, q);
-            if (D::kKind == 2 || half == 0) mma_put_scale<D>(img, nblk, b, m, half, __half2float(__float2half(d)), sum);
+            const int col = m * mma_step(M);
+            mma_put_half<D>(img, b, col, half, q);
+            if (D::kKind == 2 || half == 0) mma_put_scale<D>(img, nblk, b, col, half, __half2float(__float2half(d)), sum);
         }
     }
 }
@@ -542,7 +561,7 @@ struct MmaWarp {
     }
     __device__ __forceinline__ uint32_t slot(int i) const { return ring + static_cast<uint32_t>(i * 16 * D::kPitch); }
     // The block in slot i times the columns; lo: low bits of the address of its first row.
-    __device__ __forceinline__ void multiply(int i, int sb, uint32_t lo, uint32_t row_bytes, float (&acc)[4]) const {
+    template <bool ODD> __device__ __forceinline__ void multiply(int i, int sb, uint32_t lo, uint32_t row_bytes, float (&acc)[4]) const {
         const int gl = lane >> 2;
         uint32_t p0 = slot(i) + static_cast<uint32_t>(gl * D::kPitch), p1 = p0 + 8 * D::kPitch;
         if (MmaStream<D>::kShifted) {
@@ -550,30 +569,37 @@ struct MmaWarp {
             p0 += a & 15u;
             p1 += (a + 8u * row_bytes) & 15u;
         }
-        D::tile(p0, p1, lane & 3, xq + sb * 2048, xs + sb * 8 * D::kScaleBytes, xi + sb * 1024, acc);
+        D::template tile<ODD>(p0, p1, lane & 3, xq + sb * 2048, xs + sb * 8 * D::kScaleBytes, xi + sb * 1024, acc);
     }
 };
 
 // The partial tiles of a row group's warps, added in warp order.  sink(row, column, value) takes
-// each of the 16 x 8 sums once.  Tiles alternate between two buffers: the one being read is not
+// each sum of a batch row's column once (column: the batch row).  Tiles alternate between two buffers: the one being read is not
 // written before every warp of the group has passed the next barrier.
-template <class Sink>
+template <bool ODD, class Sink>
 __device__ __forceinline__ void mma_add_tiles(const MmaCut& g, float* part, int set, int buf, int wi, int lane, const float (&acc)[4],
                                               Sink sink) {
     float* all = part + (set * 2 + buf) * g.wpg * 128;
     float* mine = all + wi * 128;
     const int gl = lane >> 2, t = lane & 3;
-    *reinterpret_cast<float2*>(mine + gl * 8 + 2 * t) = make_float2(acc[0], acc[1]);
-    *reinterpret_cast<float2*>(mine + (gl + 8) * 8 + 2 * t) = make_float2(acc[2], acc[3]);
+    if (ODD) {
+        *reinterpret_cast<float2*>(mine + gl * 8 + 2 * t) = make_float2(acc[0], acc[1]);
+        *reinterpret_cast<float2*>(mine + (gl + 8) * 8 + 2 * t) = make_float2(acc[2], acc[3]);
+    } else {
+        mine[gl * 8 + t] = acc[0];
+        mine[(gl + 8) * 8 + t] = acc[2];
+    }
     if (g.wpg == 1) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(2 + set), "r"(g.wpg * 32) : "memory");
-    for (int i = wi * 32 + lane; i < 128; i += g.wpg * 32) {
+    for (int i = wi * 32 + lane; i < (ODD ? 128 : 64); i += g.wpg * 32) {
         const int col = i >> 4, r = i & 15;
         float v = all[r * 8 + col];
         for (int w = 1; w < g.wpg; ++w) v += all[w * 128 + r * 8 + col];
         sink(r, col, v);
     }
 }
+
+template <bool B> struct MmaFlag { static constexpr bool value = B; };
 
 template <int T>
 __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs args) {
@@ -652,42 +678,47 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
     else mma_image_q8_1<D>(smem, xqm, Mm, a.K / 32, sb0 * 8, nsb * 8, tid, kMmaThreads);
     __syncthreads();
 
-    int slot = 0, buf = 0, gi = w.set;
-    for (int c0 = 0; c0 < groups; c0 += g.chunk) {   // the same chunks in every CTA of the cluster
-        const int c1 = min(groups, c0 + g.chunk);
-        for (; gi < c1; gi += nsets, buf ^= 1) {
-            const int r0 = row_begin + gi * 16;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int sb = w.wi; sb < nsb; sb += g.wpg) {
-                prefetch();
-                mma_wait_block(w.depth);
+    auto run = [&](auto odd) {
+        constexpr bool ODD = decltype(odd)::value;
+        int slot = 0, buf = 0, gi = w.set;
+        for (int c0 = 0; c0 < groups; c0 += g.chunk) {   // the same chunks in every CTA of the cluster
+            const int c1 = min(groups, c0 + g.chunk);
+            for (; gi < c1; gi += nsets, buf ^= 1) {
+                const int r0 = row_begin + gi * 16;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                for (int sb = w.wi; sb < nsb; sb += g.wpg) {
+                    prefetch();
+                    mma_wait_block(w.depth);
+                    __syncwarp();
+                    w.template multiply<ODD>(slot, sb, static_cast<uint32_t>(w_base) + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes),
+                                             row_bytes, acc);
+                    __syncwarp();   // every lane has read the slot before it is filled again
+                    if (++slot == w.depth) slot = 0;
+                }
+                mma_add_tiles<ODD>(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int m, float v) {
+                    if (g.ksplit > 1) sums[((gi - c0) * 16 + r) * 8 + m] = v;
+                    else if (m < Mm && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(m) * ldcm + r0 + r, v);
+                });
+            }
+            if (g.ksplit > 1) {
                 __syncwarp();
-                w.multiply(slot, sb, static_cast<uint32_t>(w_base) + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes),
-                           row_bytes, acc);
-                __syncwarp();   // every lane has read the slot before it is filled again
-                if (++slot == w.depth) slot = 0;
+                mma_cluster_sync();
+                const uint32_t base = smem_u32(sums);
+                const int first = row_begin + c0 * 16, rows = min(row_end - first, (c1 - c0) * 16);
+                for (int i = rank * kMmaThreads + tid; i < rows * Mm; i += g.ksplit * kMmaThreads) {
+                    const int m = i / rows, r = i - m * rows;
+                    const uint32_t at = base + static_cast<uint32_t>(r * 8 + m) * 4u;
+                    float v = mma_ld_cluster(at, 0);
+                    for (int k = 1; k < g.ksplit; ++k) v += mma_ld_cluster(at, k);
+                    store_out(Cm, a.out_f32, static_cast<size_t>(m) * ldcm + first + r, v);
+                }
+                __syncwarp();
+                mma_cluster_sync();   // no CTA leaves, or writes the next chunk, while a peer still reads its sums
             }
-            mma_add_tiles(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int col, float v) {
-                if (g.ksplit > 1) sums[((gi - c0) * 16 + r) * 8 + col] = v;
-                else if (col < Mm && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + r0 + r, v);
-            });
         }
-        if (g.ksplit > 1) {
-            __syncwarp();
-            mma_cluster_sync();
-            const uint32_t base = smem_u32(sums);
-            const int first = row_begin + c0 * 16, rows = min(row_end - first, (c1 - c0) * 16);
-            for (int i = rank * kMmaThreads + tid; i < rows * Mm; i += g.ksplit * kMmaThreads) {
-                const int col = i / rows, r = i - col * rows;
-                const uint32_t at = base + static_cast<uint32_t>(r * 8 + col) * 4u;
-                float v = mma_ld_cluster(at, 0);
-                for (int k = 1; k < g.ksplit; ++k) v += mma_ld_cluster(at, k);
-                store_out(Cm, a.out_f32, static_cast<size_t>(col) * ldcm + first + r, v);
-            }
-            __syncwarp();
-            mma_cluster_sync();   // no CTA leaves, or writes the next chunk, while a peer still reads its sums
-        }
-    }
+    };
+    if (mma_step(Mm) == 2) run(MmaFlag<false>{});
+    else run(MmaFlag<true>{});
     if (a.dep_mode == 2) pdl_wait_prior();
 }
 
@@ -707,11 +738,18 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_grouped_kernel(const 
     pdl_wait_prior();   // the segment list and the activations come from earlier kernels
 
     const int gn = (a.N + 15) >> 4;   // row groups of an expert
-    const long long V = static_cast<long long>(a.seg[0]) * gn;
-    const long long vb = V * blockIdx.x / gridDim.x;
-    const int total = static_cast<int>(V * (blockIdx.x + 1) / gridDim.x - vb);   // row groups of this CTA
+    // CTA b: quotient row groups, and one of the remainder.  Divisions in 32 bits where that is enough:
+    // four of 64 bits in a row stand in front of the first load.
+    const auto div = [](unsigned long long n, uint32_t d) {
+        return (n >> 32) == 0 ? static_cast<unsigned long long>(static_cast<uint32_t>(n) / d) : n / d;
+    };
+    const unsigned long long V = static_cast<unsigned long long>(a.seg[0]) * gn;
+    const unsigned long long vq = div(V, gridDim.x);
+    const uint32_t vr = static_cast<uint32_t>(V - vq * gridDim.x);
+    const unsigned long long vb = vq * blockIdx.x + min(blockIdx.x, vr);
+    const int total = static_cast<int>(vq) + (blockIdx.x < vr ? 1 : 0);   // row groups of this CTA
     if (total == 0) return;
-    const int sg0 = static_cast<int>(vb / gn), first0 = static_cast<int>(vb - static_cast<long long>(sg0) * gn);
+    const int sg0 = static_cast<int>(div(vb, gn)), first0 = static_cast<int>(vb - static_cast<unsigned long long>(sg0) * gn);
 
     const MmaWarp<D> w(g, smem, g.nsb * 8);
     const int nsets = kMmaWarps / g.wpg;
@@ -754,21 +792,26 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_grouped_kernel(const 
         mma_image_q8_1<D>(smem, a.xq + static_cast<size_t>(arow0) * (a.K / 32) * kQ8_1Bytes, mcount, a.K / 32, 0, g.nsb * 8, threadIdx.x,
                           kMmaThreads);
         __syncthreads();
-        for (; next < done + last - first; next += nsets, buf ^= 1) {
-            const int r0 = (first + next - done) * 16;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int sb = w.wi; sb < g.nsb; sb += g.wpg) {
-                prefetch();
-                mma_wait_block(w.depth);
-                __syncwarp();
-                w.multiply(slot, sb, w_lo + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes), row_bytes, acc);
-                __syncwarp();
-                if (++slot == w.depth) slot = 0;
+        auto run = [&](auto odd) {
+            constexpr bool ODD = decltype(odd)::value;
+            for (; next < done + last - first; next += nsets, buf ^= 1) {
+                const int r0 = (first + next - done) * 16;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                for (int sb = w.wi; sb < g.nsb; sb += g.wpg) {
+                    prefetch();
+                    mma_wait_block(w.depth);
+                    __syncwarp();
+                    w.template multiply<ODD>(slot, sb, w_lo + static_cast<uint32_t>(r0) * row_bytes + static_cast<uint32_t>(sb * D::kBytes), row_bytes, acc);
+                    __syncwarp();
+                    if (++slot == w.depth) slot = 0;
+                }
+                mma_add_tiles<ODD>(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int m, float v) {
+                    if (m < mcount && r0 + r < a.N) store_out(a.D, a.out_f32, static_cast<size_t>(arow0 + m) * a.N + r0 + r, v);
+                });
             }
-            mma_add_tiles(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int col, float v) {
-                if (col < mcount && r0 + r < a.N) store_out(a.D, a.out_f32, static_cast<size_t>(arow0 + col) * a.N + r0 + r, v);
-            });
-        }
+        };
+        if (mma_step(mcount) == 2) run(MmaFlag<false>{});
+        else run(MmaFlag<true>{});
         done += last - first;
     }
 }

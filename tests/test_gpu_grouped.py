@@ -126,6 +126,25 @@ def test_grouped_matvec_edges(ops, name, N, K):
     check(out.cpu().numpy(), ref, TOL_F32)
 
 
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "Q4_0"])
+@pytest.mark.parametrize("N,K", [(40, 768), (33, 1024), (300, 2048)])
+def test_grouped_matvec_rows_do_not_depend_on_the_segment(ops, name, N, K):
+    """Up to four rows of an expert take every second column of the image and half the arithmetic;
+    three, four and eight 256-value blocks per row.  A row's bits are the same in a segment of any
+    height, and those of the dense call."""
+    counts = [1, 8, 4, 5, 2, 3, 6, 7]
+    _, off, _, dev_w, host_w, offs = build_group(name, counts, N, K, seed=K)
+    x = (torch.randn(8, K, generator=torch.Generator().manual_seed(N)) * 0.4).to(torch.bfloat16).cuda()
+    A = torch.cat([x[:c] for c in counts])
+    ptrs = torch.tensor([dev_w[0].data_ptr()] * len(counts), dtype=torch.int64, device="cuda")
+    out = ops.gguf_grouped_gemm(A, off, ptrs, T[name], S_INT, N, K, F_MMVQ, out_dtype=torch.float32)
+    full = out[int(offs[1]):int(offs[2])]
+    ref = oracle_grouped(name, x, host_w[:1], [0, 8], K)
+    check(full.cpu().numpy(), ref, TOL_F32)
+    assert torch.equal(out, torch.cat([full[:c] for c in counts]))
+    assert torch.equal(full, ops.gguf_mmvq(x, dev_w[0], T[name], N, K, out_dtype=torch.float32))
+
+
 @pytest.mark.parametrize("name", ["Q8_0", "Q4_K", "Q6_K"])
 def test_grouped_topk_like_counts(ops, name):
     """Uneven counts as top-k routing produces (tests/test_gguf_grouped_gemm.py:202-221)."""
