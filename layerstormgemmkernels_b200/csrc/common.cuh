@@ -9,6 +9,8 @@
 #include <stdio.h>
 #include <stdarg.h>
 
+#include <atomic>
+
 #include "../../include/lsg.h"
 
 namespace lsg {
@@ -321,21 +323,72 @@ __device__ __forceinline__ float fp16_bits_to_float(uint32_t h) {
 
 #endif  // __CUDACC__
 
-// Launch helper: plain or with the programmatic-stream-serialization attribute.
+// Launch helpers: plain or with the programmatic-stream-serialization attribute; in clusters of
+// `ctas` neighbouring CTAs (1: none).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                 cudaStream_t stream, bool pdl, Args... args) {
+inline cudaError_t launch_clusters(void (*kernel)(KArgs...), int ctas, dim3 grid, dim3 block, size_t smem,
+                                   cudaStream_t stream, bool pdl, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (ctas > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(ctas);
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                 cudaStream_t stream, bool pdl, Args... args) {
+    return launch_clusters(kernel, 1, grid, block, smem, stream, pdl, args...);
+}
+
+// How many clusters of 1, 2, 4 or 8 CTAs of a kernel that takes an SM each are resident at a time,
+// 0 when the device cannot hold one.  Asked for (and the kernel allowed its shared memory) once per
+// device: a cluster lies inside a GPC, and a B200 holds 74 of two, 33 of four and 15 of eight CTAs.
+struct ClusterSlots {
+    std::atomic<int> n[64][4];   // number + 1, of 1, 2, 4, 8 CTAs
+};
+template <typename... KArgs>
+inline int cluster_slots(void (*kernel)(KArgs...), int ctas, int threads, size_t smem, ClusterSlots& seen) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::atomic<int>* at = dev >= 0 && dev < 64 ? &seen.n[dev][ctas == 1 ? 0 : (ctas == 2 ? 1 : (ctas == 4 ? 2 : 3))] : nullptr;
+    int slots = at ? at->load(std::memory_order_relaxed) - 1 : -1;
+    if (slots >= 0) return slots;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) return 0;
+    slots = sm_count();
+    if (ctas > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+        cfg.blockDim = dim3(static_cast<unsigned>(threads));
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&slots, kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+    }
+    if (at) at->store(slots + 1, std::memory_order_relaxed);
+    return slots;
 }
 
 }  // namespace lsg

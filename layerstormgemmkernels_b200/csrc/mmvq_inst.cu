@@ -145,39 +145,14 @@ int mma_place(MmaCut& g, int sum_rows) {
     return g.sum_off + sum_bytes;
 }
 
-// How many clusters of `ksplit` CTAs of the tensor-core mat-vec are resident at a time (0: the device
-// cannot hold one); asked for once per device, which also lets the kernel have its shared memory.
+// Clusters of `ksplit` CTAs of the tensor-core mat-vec that are resident at a time.
 template <int TT>
-int mma_slots(int ksplit, int& slots) {
+int mma_slots(int ksplit) {
     if constexpr (MmaDec<TT>::kHas) {
-        auto kernel = mmvq_mma_kernel<TT>;
-        static std::atomic<int> clusters[64][4];   // of 1, 2, 4, 8 CTAs: their number + 1
-        int dev = 0;
-        LSG_CUDA_TRY(cudaGetDevice(&dev));
-        const int log_split = ksplit == 1 ? 0 : (ksplit == 2 ? 1 : (ksplit == 4 ? 2 : 3));
-        const bool known = dev >= 0 && dev < 64;
-        slots = (known ? clusters[dev][log_split].load(std::memory_order_relaxed) : 0) - 1;
-        if (slots >= 0) return LSG_OK;
-        LSG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
-        slots = sm_count();
-        if (ksplit > 1) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(static_cast<unsigned>(ksplit));
-            cfg.blockDim = dim3(kMmaThreads);
-            cfg.dynamicSmemBytes = kSmemCap;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = static_cast<unsigned>(ksplit);
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            LSG_CUDA_TRY(cudaOccupancyMaxActiveClusters(&slots, kernel, &cfg));
-            if (slots < 0) slots = 0;
-        }
-        if (known) clusters[dev][log_split].store(slots + 1, std::memory_order_relaxed);
+        static ClusterSlots seen;
+        return cluster_slots(mmvq_mma_kernel<TT>, ksplit, kMmaThreads, kSmemCap, seen);
     }
-    return LSG_OK;
+    return 0;
 }
 
 // The tensor-core mat-vec (mmvq_mma.cuh) of a call that MMVQ_FN(eight_rows) sends to it.
@@ -186,23 +161,9 @@ int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
     if constexpr (MmaDec<TT>::kHas) {
         MmaArgs g = {};
         g.v = v;
-        int slots = 0;
         if (v.M > kMmaCols || !mma_cut_k(g.c, v.K, 8, kMmaSliceBlocks))
             return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: M=%d K=%d do not fit the tensor-core mat-vec", v.M, v.K);
-        const int rc = mma_slots<TT>(g.c.ksplit, slots);
-        if (rc != LSG_OK) return rc;
-        auto kernel = mmvq_mma_kernel<TT>;
-        cudaLaunchConfig_t cfg = {};
-        cfg.blockDim = dim3(kMmaThreads);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = static_cast<unsigned>(g.c.ksplit);
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
+        const int slots = mma_slots<TT>(g.c.ksplit);
         MmvqArgs& a = g.v;
         a.row_bytes = g.c.nsb * g.c.sb_bytes;
         const int n_prob = 1 + a.n_extra;
@@ -217,11 +178,8 @@ int launch_mma(const MmvqArgs& v, cudaStream_t stream, bool pdl) {
         const int rows = share_ctas(grid, n_prob, n_rows, n_total, ctas_of);
         place_matrices(a, n_rows, ctas_of);
         const int smem = mma_place<MmaDec<TT>>(g.c, g.c.ksplit > 1 ? rows : 0);
-        cfg.gridDim = dim3(static_cast<unsigned>(grid * g.c.ksplit));
-        cfg.dynamicSmemBytes = static_cast<size_t>(smem);
-        if (g.c.ksplit == 1) cfg.attrs = attr + 1;   // no cluster
-        cfg.numAttrs = (g.c.ksplit > 1 ? 1 : 0) + (pdl ? 1 : 0);
-        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, g));
+        LSG_CUDA_TRY(launch_clusters(mmvq_mma_kernel<TT>, g.c.ksplit, dim3(static_cast<unsigned>(grid * g.c.ksplit)), dim3(kMmaThreads),
+                                     static_cast<size_t>(smem), stream, pdl, g));
         return LSG_OK;
     }
     return fail(LSG_ERR_UNSUPPORTED, "gguf_mmvq: type %d has no tensor-core mat-vec", TT);
@@ -242,9 +200,8 @@ int MMVQ_FN(max_rows)(int K) {
 // Whether a call of M batch rows goes to the tensor-core mat-vec, in passes of eight.
 bool MMVQ_FN(eight_rows)(int M, int K) {
     MmaCut c = {};
-    int slots = 0;
     return MmaDec<T>::kHas && M >= mma_min_rows() && mma_min_rows() <= kMmaCols && mma_cut_k(c, K, 8, kMmaSliceBlocks) &&
-           mma_slots<T>(c.ksplit, slots) == LSG_OK && slots > 0;
+           mma_slots<T>(c.ksplit) > 0;
 }
 
 int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool pdl) {

@@ -430,15 +430,22 @@ nvfp4_mma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // How a dense call is cut: output tiles per work item (2 or 1) and CTAs per item along K.  An
 // unsplit CTA takes 0.78 us per K tile of a pair and about 0.52 us per K tile of a single output
-// tile (the bytes it pulls out of L2); splitting adds the parked tile, two cluster barriers and
-// the sum, 2 us.  The cheapest of the combinations whose CTAs are all resident at once wins; a
-// call that fills the chip without splitting keeps pairs and no cluster.  77 x 4096 x 14336 with its
-// quantizer, in a row of calls: 41.3 us unsplit, 38.6 in clusters of eight (host bound there); a first
-// call 92 and 77.
+// tile (the bytes it pulls out of L2); splitting adds the parked tile and two cluster barriers, 1 us,
+// and the sum: a rank adds `live` rows of its share of the columns out of all ranks' memory, in two
+// halves 0.015 us a row and output tile, in four or eight 0.006.  The cheapest of the combinations
+// whose clusters are all resident at once wins.  The GEMM alone, us, unsplit pairs / best:
+// 1 x 4096 x 14336 35.5 / 13.2 (single tiles in clusters of four), 128 x 4096 x 14336 37.9 / 15.3 (the
+// same; 27.1 in sixteen clusters of eight, of which fifteen are resident), 128 x 4096 x 4096 15.3 / 9.6,
+// 512 x 1024 x 4096 15.1 / 8.9 (19.2 in sixteen clusters of eight).
 struct SplitPlan {
     int tile_cols, ksplit, kt_per_split;
 };
-SplitPlan split_plan(int m_tiles, int n_tiles, int ktiles, int sms) {
+int resident_clusters(int ksplit) {
+    static ClusterSlots seen;
+    return cluster_slots(nvfp4_mma_kernel, ksplit, kFThreads, kFSmem, seen);
+}
+SplitPlan split_plan(int M, int m_tiles, int n_tiles, int ktiles) {
+    const int sms = sm_count(), live = M < FM ? M : FM;
     SplitPlan best = {2, 1, ktiles};
     double best_us = 1e30;
     for (int cols = 2; cols >= 1; --cols) {
@@ -446,8 +453,9 @@ SplitPlan split_plan(int m_tiles, int n_tiles, int ktiles, int sms) {
         const double us_kt = cols == 2 ? 0.78 : 0.52;
         for (int ks = 1; ks <= 8; ks *= 2) {
             const int kps = (ktiles + ks - 1) / ks;
-            if (ks > 1 && (items * ks > sms - sms / 8 || (ks - 1) * kps >= ktiles)) continue;
-            const double us = static_cast<double>((items * ks + sms - 1) / sms) * kps * us_kt + (ks > 1 ? 2.0 : 0.0);
+            if (ks > 1 && ((ks - 1) * kps >= ktiles || items > resident_clusters(ks))) continue;
+            const double us_sum = ks > 1 ? 1.0 + live * cols * (ks == 2 ? 0.015 : 0.006) : 0.0;
+            const double us = static_cast<double>((items * ks + sms - 1) / sms) * kps * us_kt + us_sum;
             if (us < best_us) {
                 best_us = us;
                 best = {cols, ks, kps};
@@ -511,7 +519,7 @@ int nvfp4_mma(const void* A, long long a_rows, const void* B, long long b_rows, 
     a.kt_per_split = (K + 255) / 256;
     // the sum of split tiles stores 4-column pieces; grouped calls have their tiles on the device
     if (!tile_expert && N % 8 == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0) {
-        const SplitPlan sp = split_plan(a.m_tiles, a.n_tiles, a.kt_per_split, sm_count());
+        const SplitPlan sp = split_plan(M, a.m_tiles, a.n_tiles, a.kt_per_split);
         a.tile_cols = sp.tile_cols;
         a.ksplit = sp.ksplit;
         a.kt_per_split = sp.kt_per_split;
@@ -525,21 +533,8 @@ int nvfp4_mma(const void* A, long long a_rows, const void* B, long long b_rows, 
     }
     const long long items = static_cast<long long>(a.m_tiles) * ((a.n_tiles + a.tile_cols - 1) / a.tile_cols);
     if (a.ksplit > 1) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(items * a.ksplit));
-        cfg.blockDim = dim3(kFThreads);
-        cfg.dynamicSmemBytes = kFSmem;
-        cfg.stream = s;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = static_cast<unsigned>(a.ksplit);
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 2;
-        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, nvfp4_mma_kernel, tmA, tmB, a));
+        LSG_CUDA_TRY(launch_clusters(nvfp4_mma_kernel, a.ksplit, dim3(static_cast<unsigned>(items * a.ksplit)), dim3(kFThreads), kFSmem, s,
+                                     true, tmA, tmB, a));
         return LSG_OK;
     }
     int grid = sm_count();

@@ -960,6 +960,10 @@ struct Plan {
 struct DenseCut {
     int nt, ksplit;
 };
+int resident_clusters(int ksplit) {   // of any type's kernel: all take an SM to themselves
+    static ClusterSlots seen;
+    return cluster_slots(tc_fused_kernel<LSG_GGUF_Q4_K>, ksplit, kFusedThreads, 227 * 1024, seen);
+}
 DenseCut dense_cut(int M, int N, int K) {
     static const int force = [] {
         const char* e = getenv("LSG_TC_FUSED_DENSE_NT");
@@ -990,14 +994,13 @@ DenseCut dense_cut(int M, int N, int K) {
     double best_us = 1e30;
     for (int h : {32, 64, 128, 256, 320, 384}) {
         const long long t = (M + h - 1) / h;
-        if (h < nt && h < 256) continue;   // shorter tiles than the rows only above 256
-        if (h > nt && h > 32) continue;
+        if (h != nt && (h < 256 || h > nt)) continue;   // shorter tiles than the rows only above 256
         const double kb_us = h <= 64 ? 0.40 : (h <= 128 ? 0.45 : (h <= 256 ? 0.53 : (h <= 320 ? 0.61 : 0.69)));
         for (int ks = 1; ks <= 8; ks *= 2) {
             const long long ctas = t * wtiles * ks;
             const int kps = (((kblocks + ks - 1) / ks) + 3) & ~3;
             // the parked tile has to fit the token stages, whole 256-value blocks per split, none empty
-            if (ks > 1 && (h > 256 || ctas > (ks == 2 ? sms : sms - sms / 8) || (ks - 1) * kps >= kblocks)) continue;
+            if (ks > 1 && (h > 256 || (ks - 1) * kps >= kblocks || t * wtiles > resident_clusters(ks))) continue;
             const double us = static_cast<double>((ctas + sms - 1) / sms) * kps * kb_us + (ks > 1 ? 3.0 + 0.01 * h : 0.0);
             if (us < best_us) {
                 best_us = us;
@@ -1045,21 +1048,8 @@ int launch_fused_t(const CUtensorMap& tmX, const FusedArgs& a, cudaStream_t s) {
     }
     const long long items = static_cast<long long>(a.t_tiles) * a.n_wtiles;
     if (a.ksplit > 1) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(items * a.ksplit));
-        cfg.blockDim = dim3(kFusedThreads);
-        cfg.dynamicSmemBytes = static_cast<size_t>(smem);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = static_cast<unsigned>(a.ksplit);
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 2;
-        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc_fused_kernel<T>, tmX, a));
+        LSG_CUDA_TRY(launch_clusters(tc_fused_kernel<T>, a.ksplit, dim3(static_cast<unsigned>(items * a.ksplit)), dim3(kFusedThreads), static_cast<size_t>(smem), s,
+                                     true, tmX, a));
         return LSG_OK;
     }
     int grid = sm_count();

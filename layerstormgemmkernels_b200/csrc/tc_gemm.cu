@@ -612,12 +612,13 @@ x_q8_1_roundtrip_f16_kernel(const __nv_bfloat16* __restrict__ x, __half* __restr
 // (about 4 us).  The sum stores 4-column pieces of one output matrix.
 int pick_ksplit(const TcArgs& a) {
     if (a.tile_expert || a.n_out > 0 || a.N % 8 != 0 || a.ldc != a.N || (reinterpret_cast<uintptr_t>(a.C) & 15)) return 1;
-    const int sms = sm_count(), items = a.m_tiles * a.n_tiles, kblocks = (a.K + BK - 1) / BK;
+    static ClusterSlots seen;
+    const int items = a.m_tiles * a.n_tiles, kblocks = (a.K + BK - 1) / BK;
     int best = 1;
     double best_us = kblocks * 0.5;
     for (int ks = 2; ks <= 8; ks *= 2) {
         const int kps = (kblocks + ks - 1) / ks;
-        if (static_cast<long long>(items) * ks > (ks == 2 ? sms : sms - sms / 8) || (ks - 1) * kps >= kblocks) break;
+        if ((ks - 1) * kps >= kblocks || items > cluster_slots(tc_gemm_f16_kernel, ks, kTcThreads, kTcSmem, seen)) break;
         const double us = kps * 0.5 + 4.0;
         if (us < best_us) {
             best = ks;
@@ -638,21 +639,8 @@ int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, TcArgs a, int max_
     a.ksplit = pick_ksplit(a);
     a.kb_per_split = ((a.K + BK - 1) / BK + a.ksplit - 1) / a.ksplit;
     if (a.ksplit > 1) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(max_items * a.ksplit));
-        cfg.blockDim = dim3(kTcThreads);
-        cfg.dynamicSmemBytes = kTcSmem;
-        cfg.stream = s;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = static_cast<unsigned>(a.ksplit);
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 2;
-        LSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc_gemm_f16_kernel, tmA, tmB, a));
+        LSG_CUDA_TRY(launch_clusters(tc_gemm_f16_kernel, a.ksplit, dim3(static_cast<unsigned>(max_items * a.ksplit)), dim3(kTcThreads), kTcSmem, s,
+                                     true, tmA, tmB, a));
         return LSG_OK;
     }
     int grid = sm_count();

@@ -154,6 +154,7 @@ def test_single_gemm_from_bf16(ops, M, N, K):
     (128, 264, 2048),     # last output tile of a pair is eight columns wide
     (129, 1024, 4096),    # a second row tile with one live row
     (300, 136, 1088),
+    (128, 4096, 1024),    # sixteen pairs: more than the clusters of eight that are resident
     (40, 100, 2048),      # N not a multiple of 8: never split
 ])
 def test_single_gemm_few_rows_split_k(ops, M, N, K, dt):
@@ -177,6 +178,27 @@ def test_single_gemm_few_rows_split_k(ops, M, N, K, dt):
     half_unit = 2.0 ** -8 if dt == "bf16" else 2.0 ** -11
     assert ((out.double() - ref).abs() <= half_unit * ref.abs() + 1e-5 * ref.abs().max()).all()
     assert torch.equal(out, ops.nvfp4_gemm(codes, wc, sfa, sfb, M, N, K, float(s2), dt))
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 4096, 4096), (512, 1024, 4096), (1, 4096, 14336)])
+def test_single_gemm_split_k_replays_from_a_graph(ops, M, N, K):
+    """Sizes with sixteen pairs of output tiles or thirty-two tiles, split over clusters, captured into
+    a CUDA graph: the eager call's bits on the inputs of the replay."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    w, ws = ops.bf16_to_nvfp4(torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16))
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    call = lambda: ops.nvfp4_gemm_from_bf16(x, w, ws, 1.0)  # noqa: E731
+    eager = call()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
+    x.copy_(torch.randn(M, K, generator=g, device="cuda"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, call()) and not torch.equal(out, eager)
 
 
 @pytest.mark.parametrize("N,K,s2", [(64, 256, 1.0), (130, 512, 0.0371), (1, 16, 3.5)])

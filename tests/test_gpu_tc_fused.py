@@ -106,6 +106,36 @@ def test_fused_q4k_cluster_split_k(ops, M, N, K):
     assert torch.equal(got.to(torch.bfloat16), ops.gguf_mmq(A, Wd, T["Q4_K"], N, K))
 
 
+@pytest.mark.parametrize("op,name,M,N,K", [
+    ("gguf_mmq", "Q4_K", 40, 264, 4352),        # fused, clusters of eight
+    ("gguf_mmq", "Q4_K", 300, 1024, 4096),      # .. of four: sixteen of eight are not resident at once
+    ("gguf_mmq", "Q6_K", 17, 4096, 4096),       # the same in the GEMM over expanded weights
+    ("gguf_mmq", "Q6_K", 12, 300, 18432),       # mat-vec in clusters of eight, two passes in a launch
+    ("gguf_gemm_bf16", "Q4_K", 100, 520, 4096),
+    ("gguf_gemm_bf16", "Q8_0", 33, 520, 4096),
+])
+def test_cluster_launches_replay_from_a_graph(ops, op, name, M, N, K):
+    """Launches of thread-block clusters captured into a CUDA graph: the eager call's bits, on the
+    inputs of the replay; the eager call against the oracle."""
+    A, W, Wd = make_case(name, M, N, K, seed=M)
+    call = lambda: getattr(ops, op)(A, Wd, T[name], N, K, out_dtype=torch.float32)  # noqa: E731
+    eager = call()
+    cols = np.r_[0:40, N - 40:N]
+    ref = (oracle.mmvq(T[name], oracle.quantize_q8_1(bits_of(A)), W[cols], K) if op == "gguf_mmq"
+           else oracle.dequant_gemm(T[name], bits_of(A), W[cols], K))
+    assert np.abs(eager.cpu().numpy()[:, cols] - ref).max() <= TOL_TC * np.abs(ref).max()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    other = torch.randn_like(A, dtype=torch.float32).to(torch.bfloat16)
+    for x in (A.clone(), other):
+        A.copy_(x)
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, call())
+
+
 @pytest.mark.parametrize("M", [2, 4, 8, 16, 40])
 @pytest.mark.parametrize("N,K", [(1024, 4096), (4096, 4096), (512, 14336)])
 def test_fused_q4k_decode_batches_split_k(ops, weight_path, M, N, K):
