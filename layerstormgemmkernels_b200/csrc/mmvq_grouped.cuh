@@ -133,9 +133,10 @@ __global__ void __launch_bounds__(512, 1) mmvq_grouped_kernel(const GroupedArgs 
             if (elect_one_lane()) {
                 if (unaligned) {
                     // Weights must be 16-byte aligned for bulk copies; fall back to byte
-                    // loads for such an expert rather than read before its buffer.
+                    // loads for such an expert rather than read before its buffer.  They go where
+                    // an aligned matrix would have them: the decoders' loads rely on it.
                     for (uintptr_t p = src_b; p < src_e; ++p)
-                        dst[(p - src_b) + (src_b & 15)] = *reinterpret_cast<const uint8_t*>(p);
+                        dst[(p - src_b) + ((src_b - w_base) & 15)] = *reinterpret_cast<const uint8_t*>(p);
                 } else if (ragged) {
                     for (uintptr_t p = cp_e; p < src_e; ++p)
                         dst[p - cp_b] = *reinterpret_cast<const uint8_t*>(p);
@@ -211,11 +212,9 @@ __global__ void __launch_bounds__(512, 1) mmvq_grouped_kernel(const GroupedArgs 
                 ok = false;
             }
             if (ok && g < nrows) {
-                const int e = a.seg[1 + 3 * sg];
-                const uintptr_t src_b = reinterpret_cast<uintptr_t>(a.B_ptrs[e]) +
-                                        static_cast<uintptr_t>(n0) * a.row_bytes;
+                // offset of the slab's first row from a 16-byte boundary of its (aligned) matrix
                 const uint32_t slab = smem_u32(ring + static_cast<size_t>(s) * a.stage_bytes) +
-                                      static_cast<uint32_t>(src_b & 15);
+                                      (static_cast<uint32_t>(n0) * static_cast<uint32_t>(a.row_bytes) & 15u);
                 uint32_t raddr[RW];
 #pragma unroll
                 for (int r = 0; r < RW; ++r)

@@ -256,7 +256,8 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
                 }
             }
         }
-        const float d0 = fp16_bits_to_float(lds16(r0 + 208)), d1 = fp16_bits_to_float(lds16(r1 + 208));
+        // rows keep the offset that their matrix has in memory, odd ones too: no 2-byte loads
+        const float d0 = fp16_bits_to_float(w[0].at(208)), d1 = fp16_bits_to_float(w[1].at(208));
         acc[0] += d0 * s[0];
         acc[2] += d1 * s[2];
         if (ODD) {

@@ -126,6 +126,24 @@ def test_grouped_matvec_edges(ops, name, N, K):
     check(out.cpu().numpy(), ref, TOL_F32)
 
 
+@pytest.mark.parametrize("name,K", [(n, 1280) for n in REF_TYPES + ["Q4_0"]] + [("Q6_K", 4352), ("Q8_0", 4352), ("Q4_K", 4352)])
+@pytest.mark.parametrize("off", [1, 2, 8])
+def test_grouped_matvec_weights_at_odd_addresses(ops, name, K, off):
+    """Expert matrices off a 16-byte boundary are moved byte by byte, the others in 16-byte pieces:
+    same bits as the aligned matrices, on both grouped mat-vec kernels."""
+    N = 100
+    A, offsets, ptrs, dev_w, host_w, offs = build_group(name, [2, 9, 1, 5], N, K, seed=off)
+    aligned = ops.gguf_grouped_gemm(A, offsets, ptrs, T[name], S_INT, N, K, F_MMVQ, out_dtype=torch.float32)
+    check(aligned.cpu().numpy(), oracle_grouped(name, A, host_w, offs, K), TOL_F32)
+    moved = [torch.zeros(w.numel() + 16, dtype=torch.uint8, device="cuda") for w in dev_w]
+    for m, w in zip(moved, dev_w):
+        m[off:off + w.numel()] = w.flatten()
+    p = ptrs.clone()
+    p[1], p[2] = moved[1].data_ptr() + off, moved[2].data_ptr() + off
+    out = ops.gguf_grouped_gemm(A, offsets, p, T[name], S_INT, N, K, F_MMVQ, out_dtype=torch.float32)
+    assert torch.equal(out, aligned)
+
+
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "Q4_0"])
 @pytest.mark.parametrize("N,K", [(40, 768), (33, 1024), (300, 2048)])
 def test_grouped_matvec_rows_do_not_depend_on_the_segment(ops, name, N, K):
