@@ -119,10 +119,55 @@ int rows_per_pass(int type, int M, int K, bool& eights) {
     return batch > 32 ? 32 : batch;
 }
 
+double eight_us(int type, int K, int n, const int* N) {
+    switch (type) {
+        case 0: return mmvq_eight_us_t0(K, n, N);
+        case 1: return mmvq_eight_us_t1(K, n, N);
+        case 2: return mmvq_eight_us_t2(K, n, N);
+        case 3: return mmvq_eight_us_t3(K, n, N);
+        case 4: return mmvq_eight_us_t4(K, n, N);
+        case 5: return mmvq_eight_us_t5(K, n, N);
+        case 6: return mmvq_eight_us_t6(K, n, N);
+        case 7: return mmvq_eight_us_t7(K, n, N);
+    }
+    return 0.0;
+}
+
+// Launches for the (matrix, pass) pairs of a call on the tensor-core kernel, which are spread over them
+// evenly: up to six pairs a launch, as many as the estimate likes.  Small matrices do not fill the
+// chip one by one; a long K in clusters of eight leaves 15 clusters, which four pairs cannot share
+// evenly (8192 x 28672 of Q8_0, four passes: 300 us one by one, 348 in one launch).
+int eight_launches(int type, int K, int n, const int* N, int passes) {
+    const int items = n * passes;
+    int best = items;
+    double best_us = 1e30;
+    for (int per = 1; per <= 1 + kMmvqMaxExtra && per <= items; ++per) {
+        const int launches = (items + per - 1) / per;
+        double us = 0.0, last_us = 0.0;
+        int last = 0;
+        for (int l = 0; l < launches && us < best_us; ++l) {
+            const int i0 = static_cast<int>(static_cast<long long>(items) * l / launches);
+            const int cnt = static_cast<int>(static_cast<long long>(items) * (l + 1) / launches) - i0;
+            if (n > 1 || cnt != last) {   // pairs of one matrix: launches of a size take the same time
+                int rows[1 + kMmvqMaxExtra];
+                for (int i = 0; i < cnt; ++i) rows[i] = N[(i0 + i) / passes];
+                last_us = eight_us(type, K, cnt, rows);
+                last = cnt;
+            }
+            us += last_us;
+        }
+        if (us < best_us) {
+            best_us = us;
+            best = launches;
+        }
+    }
+    return best;
+}
+
 // The same activations (or, with A_each / xq_each, activations of their own) against n <= 6 weight
 // matrices of one type and K.  Matrix j writes C[j], [M][N[j]] row-major; xq: Q8_1 blocks of all M
 // rows.  One launch per pass over the batch rows; on the tensor-core kernel the passes are further
-// matrices of the launch, up to six in all: one after the other, the passes of a call of 9 to 32 rows
+// matrices of the launch, up to six in all (eight_launches): one after the other, the passes of a call of 9 to 32 rows
 // took twice the dp4a kernel's time on small matrices, which do not fill the chip.
 int mmvq_q8_1_joined(int type, int M, int K, int n, const void* const* W, void* const* C, const int* N,
                      const void* xq, int out_f32, cudaStream_t stream, bool pdl, const void* A_bf16, int dep_mode = 0,
@@ -146,9 +191,9 @@ int mmvq_q8_1_joined(int type, int M, int K, int n, const void* const* W, void* 
     const size_t xq_row = static_cast<size_t>(K / 32) * kQ8_1Bytes;
     const size_t c_elem = out_f32 ? 4 : 2;
     // Items are (matrix, pass) pairs, a matrix's passes next to each other (they read the same weights
-    // at the same time); `per` of them share a launch.
+    // at the same time).
     const int passes = (M + batch - 1) / batch, items = n * passes;
-    const int launches = eights ? (items + kMmvqMaxExtra) / (1 + kMmvqMaxExtra) : passes;
+    const int launches = eights ? eight_launches(type, K, n, N, passes) : passes;
     for (int l = 0; l < launches; ++l) {
         const int i0 = static_cast<int>(static_cast<long long>(items) * l / launches);
         const int i1 = static_cast<int>(static_cast<long long>(items) * (l + 1) / launches);

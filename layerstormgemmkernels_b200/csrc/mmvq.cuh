@@ -125,7 +125,8 @@ MmvqTune mmvq_tuning();  // current process-wide geometry, clamped to valid rang
 #define LSG_DECLARE_MMVQ(id)                                         \
     int mmvq_launch_t##id(MmvqArgs a, const MmvqTune& tn, cudaStream_t stream, bool pdl); \
     int mmvq_max_rows_t##id(int K);                                                       \
-    bool mmvq_eight_rows_t##id(int M, int K);
+    bool mmvq_eight_rows_t##id(int M, int K);                                            \
+    double mmvq_eight_us_t##id(int K, int n, const int* N);
 LSG_DECLARE_MMVQ(0) LSG_DECLARE_MMVQ(1) LSG_DECLARE_MMVQ(2) LSG_DECLARE_MMVQ(3)
 LSG_DECLARE_MMVQ(4) LSG_DECLARE_MMVQ(5) LSG_DECLARE_MMVQ(6) LSG_DECLARE_MMVQ(7)
 

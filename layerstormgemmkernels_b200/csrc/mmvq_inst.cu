@@ -204,6 +204,20 @@ bool MMVQ_FN(eight_rows)(int M, int K) {
            mma_slots<T>(c.ksplit) > 0;
 }
 
+// About how long a launch of n matrices with N[j] rows takes the tensor-core mat-vec: 3 us, and 4 us
+// a round of the fullest cluster's sets (two 16 x 256 blocks per warp; 3.3 us for Q4_K to 4.7 for Q6_K).
+double MMVQ_FN(eight_us)(int K, int n, const int* N) {
+    MmaCut c = {};
+    if (!MmaDec<T>::kHas || !mma_cut_k(c, K, 8, kMmaSliceBlocks)) return 0.0;
+    int total = 0, ctas_of[1 + kMmvqMaxExtra];
+    for (int j = 0; j < n; ++j) total += N[j];
+    const int slots = mma_slots<T>(c.ksplit);
+    int grid = total < slots ? total : slots;
+    if (grid < n) grid = n;
+    const int groups = (share_ctas(grid, n, N, total, ctas_of) + 15) / 16, sets = kMmaWarps / c.wpg;
+    return 3.0 + 4.0 * ((groups + sets - 1) / sets);
+}
+
 int MMVQ_FN(launch)(MmvqArgs a, const MmvqTune& tn_in, cudaStream_t stream, bool pdl) {
     using F = Fmt<T>;
     a.row_bytes = (a.K / F::VALS) * F::BYTES;
