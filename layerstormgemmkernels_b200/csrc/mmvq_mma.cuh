@@ -758,15 +758,20 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_grouped_kernel(const 
     const MmaStream<D> stream(row_bytes, w.lane);
     const uint64_t policy = l2_policy_evict_first();
 
-    // The stream's cursor: row group pn of the range (pgi of segment psg), block psb of it.
+    // The stream's cursor: row group pn of the range (pgi of segment psg, whose matrix is at base),
+    // block psb of it.
     int pn = w.wi < g.nsb ? w.set : total, psg = sg0, pgi = first0 + w.set, psb = w.wi, pslot = 0;
+    uintptr_t base = 0;
+    auto locate = [&]() {
+        while (pgi >= gn) {
+            pgi -= gn;
+            ++psg;
+        }
+        base = reinterpret_cast<uintptr_t>(a.B_ptrs[a.seg[1 + 3 * psg]]);
+    };
+    if (pn < total) locate();
     auto prefetch = [&]() {
         if (pn < total) {
-            while (pgi >= gn) {
-                pgi -= gn;
-                ++psg;
-            }
-            const uintptr_t base = reinterpret_cast<uintptr_t>(a.B_ptrs[a.seg[1 + 3 * psg]]);
             // a matrix off a 16-byte boundary is moved byte by byte rather than read before its start
             const uintptr_t end = (base & 15) ? 0 : (base + static_cast<uintptr_t>(a.N) * row_bytes) & ~uintptr_t(15);
             stream.issue(w.slot(pslot), base + static_cast<uintptr_t>(pgi * 16) * row_bytes + static_cast<uint32_t>(psb * D::kBytes),
@@ -776,6 +781,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_grouped_kernel(const 
                 psb = w.wi;
                 pn += nsets;
                 pgi += nsets;
+                if (pgi >= gn && pn < total) locate();
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
