@@ -22,10 +22,10 @@
 //     (One bulk copy per row and stage, as first written, took the copy engine 80 to 110 cycles
 //     each: 66 MB of Q4_K in 20 us with the arithmetic left out.)
 //   * `wpg` warps share a row group, warp i taking blocks i, i + wpg, ..; their partial 16 x 8
-//     tiles are added in warp order through shared memory.  16 / wpg groups are in work at a time.
+//     tiles are added through shared memory, in a fixed order.  16 / wpg groups are in work at a time.
 //   * Long rows are split along K over the CTAs of a cluster (4096 values each): a CTA then
 //     quantizes and holds only its part of the activations, and the cluster has more rows.
-//     The CTAs add their sums in rank order through distributed shared memory, in as many pieces
+//     The CTAs add their sums in a fixed order through distributed shared memory, in as many pieces
 //     (`chunk` row groups) as the sums of the cluster's rows take beside the image and the rings.
 // Whether a call comes here depends on its type, K and batch rows alone, and how K is cut on the
 // type and K, so a result does not depend on the number of weight rows, on what shares the launch,
@@ -112,7 +112,7 @@ struct MmaWords {
 };
 
 // tile(): acc[i] += the products of one 256-value block: rows r0 (accumulators 0, 1) and r1 (2, 3)
-// with columns 2t and 2t + 1.
+// with columns 2t and 2t + 1 (types with a scale per 32 values: in four sets of accumulators, by turns).
 //   r0, r1  shared addresses of the block in rows g and g + 8
 //   xq      codes of this lane's column g: block j of the 256 values at xq + 256 j, lane offset in
 //   xs      scales of columns 2t, 2t + 1 (and what kKind says): block j at xs + j * kScaleBytes
@@ -130,7 +130,7 @@ template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
 
     template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
-                                                float (&acc)[4]) {
+                                                float (&acc)[16]) {
         constexpr int QS = FIVE ? 48 : 16;
         const uint4 h0 = lds128(r0), h1 = lds128(r1);
         uint32_t sc0[2], mn0[2], sc1[2], mn1[2];
@@ -141,9 +141,12 @@ template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
             f0 = lds64(r0 + 16 + 8 * t);
             f1 = lds64(r1 + 16 + 8 * t);
         }
-        float s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
+        const float d0 = fp16_bits_to_float(h0.x), e0 = fp16_bits_to_float(h0.x >> 16);
+        const float d1 = fp16_bits_to_float(h1.x), e1 = fp16_bits_to_float(h1.x >> 16);
+        float sum1[2][4] = {}, sum2[2][4] = {};   // of each half block: sums of four sub-blocks
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
+            float (&s1)[4] = sum1[p >> 1], (&s2)[4] = sum2[p >> 1];
             const uint2 q0 = lds64(r0 + QS + 32 * p + 8 * t), q1 = lds64(r1 + QS + 32 * p + 8 * t);
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
@@ -184,14 +187,9 @@ template <bool FIVE> struct MmaDecK45 {   // Q4_K, Q5_K
                 }
             }
         }
-        const float d0 = fp16_bits_to_float(h0.x), e0 = fp16_bits_to_float(h0.x >> 16);
-        const float d1 = fp16_bits_to_float(h1.x), e1 = fp16_bits_to_float(h1.x >> 16);
-        acc[0] += d0 * s1[0] - e0 * s2[0];
-        acc[2] += d1 * s1[2] - e1 * s2[2];
-        if (ODD) {
-            acc[1] += d0 * s1[1] - e0 * s2[1];
-            acc[3] += d1 * s1[3] - e1 * s2[3];
-        }
+#pragma unroll
+        for (int i = 0; i < 4; i += ODD ? 1 : 2)
+            acc[i] += (i < 2 ? d0 : d1) * (sum1[0][i] + sum1[1][i]) - (i < 2 ? e0 : e1) * (sum2[0][i] + sum2[1][i]);
     }
 };
 template <> struct MmaDec<LSG_GGUF_Q4_K> : MmaDecK45<false> {};
@@ -206,7 +204,7 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
 
     template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t xi,
-                                                float (&acc)[4]) {
+                                                float (&acc)[16]) {
         const MmaWords w[2] = {MmaWords(r0), MmaWords(r1)};
         uint32_t scw[2][4];
 #pragma unroll
@@ -214,9 +212,11 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
 #pragma unroll
             for (int i = 0; i < 4; ++i) scw[r][i] = w[r].at(192 + 4 * i) ^ 0x80808080u;
         const MmaWords v[2] = {MmaWords(r0 + 4 * t), MmaWords(r1 + 4 * t)};
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        // rows keep the offset that their matrix has in memory, odd ones too: no 2-byte loads
+        const float d0 = fp16_bits_to_float(w[0].at(208)), d1 = fp16_bits_to_float(w[1].at(208));
 #pragma unroll
         for (int ip = 0; ip < 2; ++ip) {
+            float s[4] = {0.f, 0.f, 0.f, 0.f};   // of half a block, as the dp4a kernel's units
             uint32_t la[2][2], lb[2][2], qh[2][2];   // [row][16-value half]
 #pragma unroll
             for (int r = 0; r < 2; ++r)
@@ -255,14 +255,8 @@ template <> struct MmaDec<LSG_GGUF_Q6_K> {
                         s[2 * r + 1] = fmaf(dx1, mma_scaled(c[0][2 * r + 1], sa, na) + mma_scaled(c[1][2 * r + 1], sb, nb), s[2 * r + 1]);
                 }
             }
-        }
-        // rows keep the offset that their matrix has in memory, odd ones too: no 2-byte loads
-        const float d0 = fp16_bits_to_float(w[0].at(208)), d1 = fp16_bits_to_float(w[1].at(208));
-        acc[0] += d0 * s[0];
-        acc[2] += d1 * s[2];
-        if (ODD) {
-            acc[1] += d0 * s[1];
-            acc[3] += d1 * s[3];
+#pragma unroll
+            for (int i = 0; i < 4; i += ODD ? 1 : 2) acc[i] += (i < 2 ? d0 : d1) * s[i];
         }
     }
 };
@@ -276,7 +270,7 @@ template <> struct MmaDec<LSG_GGUF_Q8_0> {   // eight 34-byte blocks
 
     template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
-                                                float (&acc)[4]) {
+                                                float (&acc)[16]) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             // rows start on 16-byte boundaries: every second block's codes are a half word off
@@ -300,11 +294,12 @@ template <> struct MmaDec<LSG_GGUF_Q8_0> {   // eight 34-byte blocks
             mma_s8s8_k32(c, w0[0], w1[0], w0[1], w1[1], xb.x, xb.y, kMmaBiasBits);
             const float d0 = fp16_bits_to_float(lds16(r0 + 34 * j)), d1 = fp16_bits_to_float(lds16(r1 + 34 * j));
             const float dx0 = __uint_as_float(xv.x), dx1 = __uint_as_float(xv.y);
-            acc[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, acc[0]);
-            acc[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, acc[2]);
+            float* const s = acc + 4 * (j & 3);
+            s[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, s[0]);
+            s[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, s[2]);
             if (ODD) {
-                acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
-                acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
+                s[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, s[1]);
+                s[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, s[3]);
             }
         }
     }
@@ -324,7 +319,7 @@ template <> struct MmaDec<LSG_GGUF_Q4_0> {   // eight 18-byte blocks; byte i: va
     }
     template <bool ODD>
     __device__ static __forceinline__ void tile(uint32_t r0, uint32_t r1, int t, uint32_t xq, uint32_t xs, uint32_t,
-                                                float (&acc)[4]) {
+                                                float (&acc)[16]) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             // rows start on 16-byte boundaries: every second block's codes are a half word off
@@ -338,11 +333,12 @@ template <> struct MmaDec<LSG_GGUF_Q4_0> {   // eight 18-byte blocks; byte i: va
                          sext4((w1 >> 4) & 0x0F0F0F0Fu), xb.x, xb.y, kMmaBiasBits);
             const float d0 = fp16_bits_to_float(lds16(r0 + 18 * j)), d1 = fp16_bits_to_float(lds16(r1 + 18 * j));
             const float dx0 = __uint_as_float(xv.x), dx1 = __uint_as_float(xv.y);
-            acc[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, acc[0]);
-            acc[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, acc[2]);
+            float* const s = acc + 4 * (j & 3);
+            s[0] = fmaf(d0 * dx0, __int_as_float(c[0]) - kMmaBias, s[0]);
+            s[2] = fmaf(d1 * dx0, __int_as_float(c[2]) - kMmaBias, s[2]);
             if (ODD) {
-                acc[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, acc[1]);
-                acc[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, acc[3]);
+                s[1] = fmaf(d0 * dx1, __int_as_float(c[1]) - kMmaBias, s[1]);
+                s[3] = fmaf(d1 * dx1, __int_as_float(c[3]) - kMmaBias, s[3]);
             }
         }
     }
@@ -562,7 +558,7 @@ struct MmaWarp {
     }
     __device__ __forceinline__ uint32_t slot(int i) const { return ring + static_cast<uint32_t>(i * 16 * D::kPitch); }
     // The block in slot i times the columns; lo: low bits of the address of its first row.
-    template <bool ODD> __device__ __forceinline__ void multiply(int i, int sb, uint32_t lo, uint32_t row_bytes, float (&acc)[4]) const {
+    template <bool ODD> __device__ __forceinline__ void multiply(int i, int sb, uint32_t lo, uint32_t row_bytes, float (&acc)[16]) const {
         const int gl = lane >> 2;
         uint32_t p0 = slot(i) + static_cast<uint32_t>(gl * D::kPitch), p1 = p0 + 8 * D::kPitch;
         if (MmaStream<D>::kShifted) {
@@ -574,29 +570,53 @@ struct MmaWarp {
     }
 };
 
-// The partial tiles of a row group's warps, added in warp order.  sink(row, column, value) takes
-// each sum of a batch row's column once (column: the batch row).  Tiles alternate between two buffers: the one being read is not
-// written before every warp of the group has passed the next barrier.
-template <bool ODD, class Sink>
-__device__ __forceinline__ void mma_add_tiles(const MmaCut& g, float* part, int set, int buf, int wi, int lane, const float (&acc)[4],
+// at(0) + .. + at(n - 1), n <= 8 a power of two: neighbours first, then neighbours of those.
+template <class At>
+__device__ __forceinline__ float mma_sum8(int n, At at) {
+    float p[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i] = i < n ? at(i) : 0.0f;
+    return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+}
+
+// The orders of the fp32 sums are chosen so that the error of a result against 64 bits is no larger
+// than the dp4a kernel's (2-norm, relative, K of 768 to 28672; dp4a / here): Q4_K and Q5_K 1.65e-7 to
+// 1.84e-7 / 1.64e-7 to 1.79e-7 (sums of four sub-blocks), Q6_K 7.5e-8 to 9.6e-8 / 6.2e-8 to 9.3e-8,
+// Q8_0 and Q4_0 6.4e-8 to 1.14e-7 / 6.1e-8 to 7.7e-8 (four accumulators per lane; what the additions
+// of the warps' tiles lose is carried along).
+//
+// The partial tiles of a row group's warps, added in a fixed order.  sink(row, column, value) takes
+// each sum of a batch row's column once (column: the batch row).  Tiles alternate between two buffers:
+// the one being read is not written before every warp of the group has passed the next barrier.
+template <class D, bool ODD, class Sink>
+__device__ __forceinline__ void mma_add_tiles(const MmaCut& g, float* part, int set, int buf, int wi, int lane, const float (&acc)[16],
                                               Sink sink) {
     float* all = part + (set * 2 + buf) * g.wpg * 128;
     float* mine = all + wi * 128;
     const int gl = lane >> 2, t = lane & 3;
+    const auto sum = [&](int i) { return (acc[i] + acc[4 + i]) + (acc[8 + i] + acc[12 + i]); };   // zeros where a type has one accumulator
     if (ODD) {
-        *reinterpret_cast<float2*>(mine + gl * 8 + 2 * t) = make_float2(acc[0], acc[1]);
-        *reinterpret_cast<float2*>(mine + (gl + 8) * 8 + 2 * t) = make_float2(acc[2], acc[3]);
+        *reinterpret_cast<float2*>(mine + gl * 8 + 2 * t) = make_float2(sum(0), sum(1));
+        *reinterpret_cast<float2*>(mine + (gl + 8) * 8 + 2 * t) = make_float2(sum(2), sum(3));
     } else {
-        mine[gl * 8 + t] = acc[0];
-        mine[(gl + 8) * 8 + t] = acc[2];
+        mine[gl * 8 + t] = sum(0);
+        mine[(gl + 8) * 8 + t] = sum(2);
     }
     if (g.wpg == 1) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(2 + set), "r"(g.wpg * 32) : "memory");
     for (int i = wi * 32 + lane; i < (ODD ? 128 : 64); i += g.wpg * 32) {
         const int col = i >> 4, r = i & 15;
-        float v = all[r * 8 + col];
-        for (int w = 1; w < g.wpg; ++w) v += all[w * 128 + r * 8 + col];
-        sink(r, col, v);
+        const float* p = all + r * 8 + col;
+        float v = p[0], low = 0.0f;
+        for (int w = 1; w < g.wpg; ++w) {
+            const float x = p[w * 128], t = v + x;
+            if (D::kKind == 0) {   // what the addition lost (exact)
+                const float b = t - v;
+                low += (v - (t - b)) + (x - b);
+            }
+            v = t;
+        }
+        sink(r, col, low == low ? v + low : v);   // an infinite sum loses NaN
     }
 }
 
@@ -686,7 +706,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
             const int c1 = min(groups, c0 + g.chunk);
             for (; gi < c1; gi += nsets, buf ^= 1) {
                 const int r0 = row_begin + gi * 16;
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                float acc[16] = {};
                 for (int sb = w.wi; sb < nsb; sb += g.wpg) {
                     prefetch();
                     mma_wait_block(w.depth);
@@ -696,7 +716,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
                     __syncwarp();   // every lane has read the slot before it is filled again
                     if (++slot == w.depth) slot = 0;
                 }
-                mma_add_tiles<ODD>(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int m, float v) {
+                mma_add_tiles<D, ODD>(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int m, float v) {
                     if (g.ksplit > 1) sums[((gi - c0) * 16 + r) * 8 + m] = v;
                     else if (m < Mm && r0 + r < row_end) store_out(Cm, a.out_f32, static_cast<size_t>(m) * ldcm + r0 + r, v);
                 });
@@ -709,8 +729,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_kernel(const MmaArgs 
                 for (int i = rank * kMmaThreads + tid; i < rows * Mm; i += g.ksplit * kMmaThreads) {
                     const int m = i / rows, r = i - m * rows;
                     const uint32_t at = base + static_cast<uint32_t>(r * 8 + m) * 4u;
-                    float v = mma_ld_cluster(at, 0);
-                    for (int k = 1; k < g.ksplit; ++k) v += mma_ld_cluster(at, k);
+                    const float v = mma_sum8(g.ksplit, [&](int k) { return mma_ld_cluster(at, k); });
                     store_out(Cm, a.out_f32, static_cast<size_t>(m) * ldcm + first + r, v);
                 }
                 __syncwarp();
@@ -803,7 +822,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_grouped_kernel(const 
             constexpr bool ODD = decltype(odd)::value;
             for (; next < done + last - first; next += nsets, buf ^= 1) {
                 const int r0 = (first + next - done) * 16;
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                float acc[16] = {};
                 for (int sb = w.wi; sb < g.nsb; sb += g.wpg) {
                     prefetch();
                     mma_wait_block(w.depth);
@@ -812,7 +831,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) mmvq_mma_grouped_kernel(const 
                     __syncwarp();
                     if (++slot == w.depth) slot = 0;
                 }
-                mma_add_tiles<ODD>(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int m, float v) {
+                mma_add_tiles<D, ODD>(g, part, w.set, buf, w.wi, w.lane, acc, [&](int r, int m, float v) {
                     if (m < mcount && r0 + r < a.N) store_out(a.D, a.out_f32, static_cast<size_t>(arow0 + m) * a.N + r0 + r, v);
                 });
             }
