@@ -183,7 +183,8 @@ LSG_API size_t lsg_gguf_mmvq_batch_workspace_bytes(const lsg_gguf_mmvq_params* p
  * the launch in front of it, 1 is the first launch of a batch whose later launches need not
  * wait (it waits for the work in front of the call and releases the next launch after that),
  * 2 does not wait for the launch in front of it; + 4 when a quantizer launch precedes the
- * mat-vec (activations above the in-kernel quantizer's limit).  Output arrays may be null. */
+ * mat-vec (activations above the in-kernel quantizer's limit).  An entry with more batch rows than
+ * one pass takes may be several launches and counts as one.  Output arrays may be null. */
 LSG_API int lsg_gguf_mmvq_batch_plan(const lsg_gguf_mmvq_params* p, int n, int* first, int* count, int* kind,
                                      int cap);
 LSG_API int lsg_gguf_mmvq_batch(const lsg_gguf_mmvq_params* p, int n, void* workspace,
@@ -350,7 +351,8 @@ LSG_API int lsg_gguf_grouped_gemm(const lsg_gguf_grouped_gemm_params* p, int tot
  * gguf_grouped_gemm (csrc/bindings_python.cu:552-611) builds the block; the reference fuses
  * activation and quantizer only on its NVFP4 path (launch_silu_mul_to_nvfp4_grouped).
  * Never synchronizes with the host.  Rows of experts without rows are untouched; all three
- * pointers of an expert that has rows must be valid.
+ * pointers of an expert that has rows must be valid (up to eight rows per expert on average, an
+ * expert that lacks one is skipped and its rows are untouched).
  * With `perm` set the permute (gather) of the MoE layer is folded into the call: A_base is
  * then the UNPERMUTED token matrix [num_tokens, H] and row i of the block is token
  * perm[i] / top_k (perm as lsg_moe_permutation writes it); the routed rows are never written
@@ -374,14 +376,15 @@ LSG_API size_t lsg_gguf_moe_ffn_workspace_bytes(int total_tokens, int H, int I, 
 LSG_API int lsg_gguf_moe_ffn(const lsg_gguf_moe_ffn_params* p, int total_tokens, void* workspace,
                              size_t workspace_bytes, void* stream);
 /* Average rows per expert (total_tokens / num_experts, rounded down) up to which
- * lsg_gguf_moe_ffn composes the block from the grouped mat-vec kernels, whose results are
- * bit-identical to the reference's; above it the tensor-core kernels run (equal within the
- * tolerance of a GEMM with fp32 accumulation in another order).  Default 8, the batch at which
- * the reference leaves its mat-vec kernels (gguf_grouped_int.cu:918-919), or the environment
- * variable LSG_MOE_MATVEC_ROWS; -1 sends every batch to the tensor cores, which is faster from
- * about two rows per expert (128 experts of 2048 x 768, 64 / 128 tokens top-8: 0.33 -> 0.27 ms
- * and 0.47 -> 0.27 ms per layer).  Returns the previous value.  Process-wide, not synchronized
- * with calls in flight on other threads. */
+ * lsg_gguf_moe_ffn composes the block from the grouped mat-vec kernels, whose integer sums are
+ * exactly the reference's; above it the tensor-core GEMMs run (equal within the tolerance of
+ * fp16 operands).  Default 8, the batch at which the reference leaves its mat-vec kernels
+ * (gguf_grouped_int.cu:918-919), or the environment variable LSG_MOE_MATVEC_ROWS; -1 sends every
+ * batch to the GEMMs.  Expert block of Q4_K, mat-vec / GEMM, us: 128 experts of 2048 x 768 at 4
+ * and 8 rows per expert 122 / 247 and 165 / 249, 32 of 2048 x 1536 79 / 145 and 105 / 145; with
+ * few wide experts (8 of 4096 x 14336, whose down projection has a K above the tensor-core
+ * mat-vec's 4096) 385 / 516 at 4 rows, but 728 / 516 at 8.  Returns the previous value.
+ * Process-wide, not synchronized with calls in flight on other threads. */
 LSG_API int lsg_gguf_moe_ffn_set_matvec_rows(int rows);
 
 /* Ascending list of the experts that have rows, padded with -1 to `cap` entries.
@@ -411,7 +414,9 @@ LSG_API int lsg_build_mmq_tile_map(const int32_t* expert_offsets, int num_expert
  * fp8_gemm.cu), launch_fp8_grouped_gemm (fp8_grouped_gemm.cu:52-151; no host synchronisation
  * here) and launch_weight_fp8_quant (csrc/smxx/quant/weight_fp8_quant.cu:51-150, bit-exact).
  * K must be a multiple of 16.  M <= 4 with 16-byte aligned operands takes a mat-vec kernel
- * that needs no workspace (the role of fp8_blockscaled_gemv.cu:54-145 for M = 1). */
+ * that needs no workspace (the role of fp8_blockscaled_gemv.cu:54-145 for M = 1).  Above that the
+ * workspace is asked for whatever the alignment, and used for operands off a 16-byte boundary
+ * only. */
 typedef struct lsg_fp8_gemm_params {
     int M, N, K;
     const void* A;         /* [M,K] e4m3 */

@@ -15,7 +15,8 @@
 // that size, 39 with the drain left out: the bytes that come out of L2 bound it first (48 KB per K
 // block of a 128 x 256 tile at about 42 B/clk and SM, against 512 cycles of tensor time), which is
 // why 256 columns are the tile (a narrower one moves more bytes per product), the drain second.
-// Sixteen drain warps with half the columns each: 57 us.
+// Sixteen drain warps with half the columns each: 57 us.  K is not split, so few rows leave most SMs
+// idle: 5 to 128 x 1024 x 14336 are 8 CTAs and 53 us (84 to 88 on the route this replaced).
 //   warps 0-7   drain and epilogue: warp w owns tensor-memory lanes 32 (w % 4).. (= token rows)
 //               and column half w / 4; output rows are stored as 16-byte pieces
 //   warp 8      TMA producer: one box of 128 tokens x 128 bytes, one of NC weight rows

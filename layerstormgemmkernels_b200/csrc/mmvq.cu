@@ -371,7 +371,7 @@ bool batch_overlap_enabled() {
 }
 
 // Entries [i, i + run) of a batch that can share one launch: same activations, type, K,
-// batch rows and output type, at most four, every N >= 1.
+// batch rows and output type, at most six, every N >= 1.
 int joinable_run(const lsg_gguf_mmvq_params* p, int i, int n, bool distinct_a = false) {
     int run = 1;
     if (p[i].M < 1 || p[i].N < 1) return 1;

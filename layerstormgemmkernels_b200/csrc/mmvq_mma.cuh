@@ -1,12 +1,14 @@
-// GGUF mat-vec for 5 to 8 batch rows on the integer tensor-core instruction (mma.sync s8).
+// GGUF mat-vec on the integer tensor-core instruction (mma.sync s8): dense calls from five batch rows
+// on, in passes of eight, and grouped calls, in segments of one to eight rows.
 //
 // With more batch rows the mat-vec of mmvq.cuh is bound by its dp4a arithmetic (eight rows of
 // Q6_K: a quarter of the copy bandwidth; 28672 x 4096 54.3 us there and 36.4 here, Q4_K 40.0 and
-// 25.2; the MoE layer of 64 tokens 307 and 145), so here a warp multiplies 16 weight rows by eight
+// 25.2; the MoE layer of 64 tokens 307 and 134), so here a warp multiplies 16 weight rows by eight
 // batch rows: one mma.m16n8k32 (k16 for Q6_K, whose scales cover 16 values) replaces 32 dp4a per
 // lane, and with the magic number 1.5 * 2^23 as the initial accumulator its integer result is
 // read as a float with one subtraction.  The sums of a scale group are the same exact integers
-// as before; the products with the scales and their fp32 sums keep the same terms.
+// as before; the products with the scales keep their terms, and their fp32 sums are made in an order
+// of their own (mma_add_tiles).
 //
 // mma.sync and not tcgen05: the sums have to be rescaled every 16 or 32 values of K, and an
 // accumulator in tensor memory would be drained as often.  At eight columns the instruction is

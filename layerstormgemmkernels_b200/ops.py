@@ -73,7 +73,7 @@ def gguf_mmvq(A, B_packed, type, N, K, out_dtype=torch.bfloat16):
 def gguf_mmvq_batch(A, weights, type, out_dtype=torch.bfloat16):
     """Several projections of the same activations: bf16 A[M,K] against each packed weight
     in `weights` (a sequence of (B_packed, N) with one GGUF type and K), through
-    lsg_gguf_mmvq_batch, which runs up to four of them per launch.  Returns the list of
+    lsg_gguf_mmvq_batch, which runs up to six of them per launch.  Returns the list of
     [M, N] results, equal bit for bit to separate gguf_mmvq calls."""
     _require(A.is_cuda and A.dtype == torch.bfloat16 and A.dim() == 2 and A.is_contiguous(),
              "gguf_mmvq_batch: A must be contiguous BF16 [M, K] on CUDA")
